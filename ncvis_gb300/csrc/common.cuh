@@ -44,9 +44,9 @@ inline void check_cuda(cudaError_t e, const char *what, const char *file, int li
 struct StreamBuffer {
     void *p = nullptr;
     cudaStream_t s;
-    StreamBuffer(size_t bytes, cudaStream_t st) : s(st) {
-        NCVIS_CUDA(cudaMallocAsync(&p, bytes > 0 ? bytes : 1, s));
-    }
+    explicit StreamBuffer(cudaStream_t st) : s(st) {}
+    StreamBuffer(size_t bytes, cudaStream_t st) : s(st) { alloc(bytes); }
+    void alloc(size_t bytes) { NCVIS_CUDA(cudaMallocAsync(&p, bytes > 0 ? bytes : 1, s)); }
     StreamBuffer(const StreamBuffer &) = delete;
     StreamBuffer &operator=(const StreamBuffer &) = delete;
     ~StreamBuffer() {

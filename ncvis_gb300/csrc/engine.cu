@@ -216,6 +216,75 @@ static BatchedTcWork plan_batched_tc(const std::vector<int64_t> &off, int ctas_m
     return w;
 }
 
+// The FP32 search of one problem: on the tensor cores over FP16 part rows where
+// the shape and the rows' norms allow it (split_scale), else K3 on the CUDA
+// cores.  The part rows, the further lists and the work list share one block
+// of memory.
+struct KnnF32Plan {
+    KnnPlan simt{};
+    KnnTcPlan tc{};
+    TcSweep sweep;
+    bool split = false;
+    size_t rows_bytes = 0, lists_bytes = 0, work_bytes = 0;
+    size_t cand_bytes(size_t N) const {
+        return sizeof(int32_t) * N * std::max(simt.C(), split ? tc.R : 0);
+    }
+    size_t block_bytes() const { return split ? rows_bytes + lists_bytes + work_bytes : 0; }
+};
+
+// From this many rows on the tensor cores are the faster of the two (a whole
+// stage call, K3 on the CUDA cores against them: 64 x 16 159 and 120 us, 1,000 x
+// 32 393 and 187, 10,000 x 64 2,180 and 540, 60,013 x 100 30,800 and 2,830); fewer
+// were not measured.
+constexpr size_t kSplitMinRows = 64;
+
+static KnnF32Plan plan_knn_fp32(size_t N, size_t D, int k, int rerank_factor, int dist) {
+    KnnF32Plan p;
+    p.simt = plan_knn_f32((int64_t)N, k, rerank_factor);
+    p.split = N >= kSplitMinRows && knn_split_supported((int64_t)N, (int)D, p.simt.R, dist);
+    if (!p.split) return p;
+    p.tc = plan_knn_split((int)D, p.simt.R, dist);
+    p.sweep = plan_sweep((int64_t)N, num_sms());
+    p.rows_bytes = align256(sizeof(__half) * (p.tc.fold ? 3 : 2) * N * p.tc.ldb);
+    p.lists_bytes = align256(sizeof(int32_t) * (size_t)p.sweep.split_rows *
+                             (p.sweep.lists - 1) * p.tc.R);
+    p.work_bytes = align256(sweep_work_bytes((int64_t)N, p.sweep));
+    return p;
+}
+
+// Where a search left its candidates: C per row, and the further lists.
+struct Candidates {
+    int C = 0;
+    TcLists lists;
+};
+
+// Runs the search into cand (plan.cand_bytes) with block (plan.block_bytes) as
+// scratch; norms: the words of launch_preprocess, on the host.
+static Candidates run_knn_fp32(const float *Xp, const float *sqn, size_t N, size_t D, int dist,
+                               const KnnF32Plan &plan, const uint32_t *norms, int32_t *cand,
+                               char *block, int *timeout_flag, cudaStream_t s) {
+    Candidates c;
+    const float scale = plan.split ? split_scale(norms, dist) : 0.f;
+    if (scale == 0.f) {
+        launch_knn_select_f32(Xp, sqn, (int64_t)N, (int)D, dist, plan.simt, cand, s);
+        c.C = plan.simt.C();
+        return c;
+    }
+    __half *rows = (__half *)block;
+    launch_split_rows(Xp, sqn, (int64_t)N, (int)D, scale, plan.tc, rows, (int64_t)N, s);
+    c.C = plan.tc.R;
+    c.lists.row0 = (int64_t)N - plan.sweep.split_rows;
+    c.lists.count = plan.sweep.lists - 1;
+    c.lists.extra = (int32_t *)(block + plan.rows_bytes);
+    if (plan.lists_bytes)
+        NCVIS_CUDA(cudaMemsetAsync(c.lists.extra, 0xff, plan.lists_bytes, s));
+    TcWork work = launch_sweep_work((int64_t)N, plan.sweep,
+                                    block + plan.rows_bytes + plan.lists_bytes, s);
+    work.lists = c.lists;
+    launch_knn_select_split(rows, (int64_t)N, plan.tc, cand, timeout_flag, s, work);
+    return c;
+}
+
 struct ncvis_engine {
     ncvis_params p{};
     std::vector<size_t> noise;
@@ -362,7 +431,8 @@ void ncvis_engine::fit(const float *X, size_t N, size_t D, float *Y, bool host) 
     const bool replay = (o.sgd_mode == NCVIS_SGD_REPLAY);
 
     cudaStream_t s = stream();
-    KnnPlan kp = plan_knn_f32((int64_t)N, k, o.rerank_factor);
+    KnnF32Plan fp;
+    if (!bf16) fp = plan_knn_fp32(N, D, k, o.rerank_factor, dist);
     KnnTcPlan tp = plan_knn_tc((int64_t)N, (int)D, k, o.rerank_factor, dist);
     tp.wait_cycles = o.wait_limit_cycles;
     tp.stall = o.inject_stall != 0;
@@ -370,7 +440,6 @@ void ncvis_engine::fit(const float *X, size_t N, size_t D, float *Y, bool host) 
         require(knn_tc_supported((int)D, tp.R),
                 "[ncvis] the BF16 tensor-core kNN supports D <= 128", kUnsupported);
     const bool fold = bf16 && tp.fold;
-    const int C = bf16 ? tp.R : kp.C();
     const int64_t nk = (int64_t)N * k;
     // The exact BF16 search with the rows ordered by k-means cell (warm start).
     const KnnOrderPlan op =
@@ -389,11 +458,9 @@ void ncvis_engine::fit(const float *X, size_t N, size_t D, float *Y, bool host) 
     const size_t o_Y = host ? L.take(sizeof(float) * N * d) : 0;
     const size_t o_Xp = L.take(sizeof(float) * N * D);
     const size_t o_sqn = L.take(sizeof(float) * N);
-    const size_t o_flag = L.take(sizeof(int) * 4);
+    const size_t o_flag = L.take(sizeof(int) * 8);
     const size_t o_Xb = bf16 ? L.take(sizeof(__nv_bfloat16) * N * tp.ldb) : 0;
     const size_t o_Xc = fold ? L.take(sizeof(__nv_bfloat16) * N * tp.ldb) : 0;
-    const size_t o_ci = L.take(sizeof(int32_t) * N * C);
-    const size_t o_cd = L.take(sizeof(float) * N * C);
     const size_t o_ki = L.take(sizeof(int32_t) * nk);
     const size_t o_kd = L.take(sizeof(float) * nk);
     const size_t o_rp = L.take(sizeof(int64_t) * (N + 1));
@@ -401,13 +468,37 @@ void ncvis_engine::fit(const float *X, size_t N, size_t D, float *Y, bool host) 
     const size_t o_vals = L.take(sizeof(float) * 2 * nk);
     const size_t o_src = L.take(sizeof(int32_t) * 2 * nk);
     const size_t o_Q = L.take(sizeof(float) * 4);
-    const size_t o_sym = L.take(symmetrize_workspace_bytes((int64_t)N, k));
     const size_t o_init = L.take(init_workspace_bytes((int64_t)N, d));
     const size_t o_sgd = L.take(sgd_workspace_bytes(chains));
     const size_t o_stream = replay ? L.take(sizeof(int32_t) * std::max<size_t>(o.replay_len, 1)) : 0;
     const size_t ord_bytes = knn_order_workspace_bytes((int64_t)N, (int)D, tp, op);
     const size_t o_ord = ord_bytes ? L.take(ord_bytes) : 0;
-    char *base = ensure_arena(L.total);
+    const TcSweep whole = whole_tiles((int64_t)N, num_sms());
+    const size_t o_work =
+        bf16 && !ivf && op.C <= 0 ? L.take(sweep_work_bytes((int64_t)N, whole)) : 0;
+    // Last: the candidates, and the symmetrization's workspace, which the FP32
+    // search's part rows and lists share (they are read for the last time by
+    // the rerank before it).  Where memory, or the caller's limit, has no room
+    // for those the search takes the CUDA cores.
+    const size_t o_ci = L.total;
+    auto cand_bytes = [&] {
+        return align256(bf16 ? sizeof(int32_t) * N * tp.R : fp.cand_bytes(N));
+    };
+    auto total_bytes = [&] {
+        return o_ci + cand_bytes() +
+               align256(std::max(symmetrize_workspace_bytes((int64_t)N, k), fp.block_bytes()));
+    };
+    if (fp.split && o.arena_limit && total_bytes() > o.arena_limit) fp.split = false;
+    char *base = nullptr;
+    try {
+        base = ensure_arena(total_bytes());
+    } catch (const Error &) {
+        if (!fp.split) throw;
+        cudaGetLastError();
+        fp.split = false;
+        base = ensure_arena(total_bytes());
+    }
+    const size_t o_sym = o_ci + cand_bytes();
 
     const float *dX = (host && !read_host) ? (float *)(base + o_X) : X;
     float *dY = host ? (float *)(base + o_Y) : Y;
@@ -417,7 +508,6 @@ void ncvis_engine::fit(const float *X, size_t N, size_t D, float *Y, bool host) 
     __nv_bfloat16 *Xb = bf16 ? (__nv_bfloat16 *)(base + o_Xb) : nullptr;
     __nv_bfloat16 *Xc = fold ? (__nv_bfloat16 *)(base + o_Xc) : nullptr;
     int32_t *cand_i = (int32_t *)(base + o_ci);
-    float *cand_d = (float *)(base + o_cd);
     int32_t *knn_i = (int32_t *)(base + o_ki);
     float *knn_d = (float *)(base + o_kd);
     int64_t *row_ptr = (int64_t *)(base + o_rp);
@@ -434,17 +524,18 @@ void ncvis_engine::fit(const float *X, size_t N, size_t D, float *Y, bool host) 
         NCVIS_CUDA(cudaMemcpyAsync((void *)dX, X, sizeof(float) * N * D, cudaMemcpyHostToDevice, s));
     NCVIS_CUDA(cudaEventRecord(ev.ev[1], s));
     nv.next("ncvis.preprocess");
-    NCVIS_CUDA(cudaMemsetAsync(flag, 0, sizeof(int) * 4, s));
-    launch_preprocess(dX, (int64_t)N, (int)D, dist, Xp, sqn, Xb, bf16 ? tp.ldb : 0, flag, s, Xc);
+    NCVIS_CUDA(cudaMemsetAsync(flag, 0, sizeof(int) * 8, s));
+    launch_preprocess(dX, (int64_t)N, (int)D, dist, Xp, sqn, Xb, bf16 ? tp.ldb : 0, flag, s, Xc,
+                      fp.split ? (uint32_t *)flag + 4 : nullptr);
     NCVIS_CUDA(cudaEventRecord(ev.ev[2], s));
-    {
-        int bad = 0;
-        NCVIS_CUDA(cudaMemcpyAsync(&bad, flag, sizeof(int), cudaMemcpyDeviceToHost, s));
-        NCVIS_CUDA(cudaStreamSynchronize(s));
-        require(bad == 0, "[ncvis] input contains non-finite values");
-    }
+    int h_flag[8];
+    NCVIS_CUDA(cudaMemcpyAsync(h_flag, flag, sizeof(h_flag), cudaMemcpyDeviceToHost, s));
+    NCVIS_CUDA(cudaStreamSynchronize(s));
+    require(h_flag[0] == 0, "[ncvis] input contains non-finite values");
     nv.next("ncvis.knn");
     const int32_t *cell_order = nullptr;  // rows in k-means cell order (ordered sweep only)
+    Candidates found;
+    found.C = tp.R;
     NCVIS_CUDA(cudaMemsetAsync(knn_i, 0xff, sizeof(int32_t) * nk, s));
     if (ivf)
         run_knn_ivf(Xp, Xb, Xc, (int64_t)N, (int)D, tp, dist,
@@ -454,16 +545,18 @@ void ncvis_engine::fit(const float *X, size_t N, size_t D, float *Y, bool host) 
         run_knn_tc_ordered(Xp, Xb, Xc, (int64_t)N, (int)D, tp, dist, op, (uint64_t)p.random_seed,
                            cand_i, flag + 2, s, base + o_ord, ord_bytes, ev.ev[9], &cell_order);
     else if (bf16)
-        launch_knn_select_tc(Xb, sqn, (int64_t)N, tp, dist, cand_i, cand_d, flag + 2, s, nullptr,
-                             Xc);
+        launch_knn_select_tc(Xb, sqn, (int64_t)N, tp, dist, cand_i, flag + 2, s,
+                             launch_sweep_work((int64_t)N, whole, base + o_work, s), Xc);
     else
-        launch_knn_select_f32(Xp, sqn, (int64_t)N, (int)D, dist, kp, cand_i, cand_d, s);
+        found = run_knn_fp32(Xp, sqn, N, D, dist, fp, (const uint32_t *)h_flag + 4, cand_i,
+                             base + o_sym, flag + 2, s);
     NCVIS_CUDA(cudaEventRecord(ev.ev[3], s));
     nv.next("ncvis.rerank");
-    launch_rerank(Xp, (int64_t)N, (int)D, dist, cand_i, C, k, knn_i, knn_d, s, cell_order);
+    launch_rerank(Xp, (int64_t)N, (int)D, dist, cand_i, found.C, k, knn_i, knn_d, s, cell_order,
+                  found.lists);
     NCVIS_CUDA(cudaEventRecord(ev.ev[4], s));
     nv.next("ncvis.symmetrize");
-    if (bf16) {
+    if (bf16 || fp.split) {
         int timeout = 0;
         NCVIS_CUDA(cudaMemcpyAsync(&timeout, flag + 2, sizeof(int), cudaMemcpyDeviceToHost, s));
         NCVIS_CUDA(cudaStreamSynchronize(s));
@@ -605,22 +698,26 @@ void ncvis_engine::fit_batched(const float *dX, size_t D, const int64_t *offsets
         tw = plan_batched_tc(h_off, num_sms());
         require(tw.pad[B] < (int64_t(1) << 31), "[ncvis] batched: too many rows");
     }
-    const int C = bf16 ? tp.R : kp.C();
+    // The FP32 search on the tensor cores (FP16 part rows) where it applies.
+    KnnTcPlan sp;
+    bool split = false;
+    if (!bf16 && total >= (int64_t)kSplitMinRows) {
+        tw = plan_batched_tc(h_off, num_sms());
+        split = knn_split_supported(tw.pad[B], (int)D, kp.R, dist);
+        if (split) sp = plan_knn_split((int)D, kp.R, dist);
+    }
     const int64_t max_chains = std::max<int64_t>(sgd_batched_resident_chains(d), (int64_t)B);
 
     Layout L;
     const size_t o_Xp = L.take(sizeof(float) * total * D);
     const size_t o_sqn = L.take(sizeof(float) * total);
-    const size_t o_flag = L.take(sizeof(int) * 4);
-    const size_t o_ci = L.take(sizeof(int32_t) * total * C);
-    const size_t o_cd = L.take(sizeof(float) * total * C);
+    const size_t o_flag = L.take(sizeof(int) * 8);
     const size_t o_ki = L.take(sizeof(int32_t) * nk);
     const size_t o_kd = L.take(sizeof(float) * nk);
     const size_t o_rp = L.take(sizeof(int64_t) * (total + 1));
     const size_t o_cols = L.take(sizeof(int32_t) * 2 * nk);
     const size_t o_vals = L.take(sizeof(float) * 2 * nk);
     const size_t o_src = L.take(sizeof(int32_t) * 2 * nk);
-    const size_t o_sym = L.take(symmetrize_workspace_bytes(total, k));
     const size_t o_init = L.take(init_batched_workspace_bytes(total, h_ti[B], (int)B, d));
     const size_t o_off = L.take(sizeof(int64_t) * (B + 1));
     const size_t o_tq = L.take(sizeof(int64_t) * (B + 1));
@@ -633,21 +730,46 @@ void ncvis_engine::fit_batched(const float *dX, size_t D, const int64_t *offsets
     const size_t o_cq = L.take(sizeof(float) * max_chains);
     const size_t o_Yt = L.take(sizeof(float) * total * d);
     const size_t o_Qt = L.take(sizeof(float) * B);
-    const int64_t total_pad = bf16 ? tw.pad[B] : 0;
+    const int64_t total_pad = bf16 || split ? tw.pad[B] : 0;
     const size_t o_Xb = bf16 ? L.take(sizeof(__nv_bfloat16) * total * tp.ldb) : 0;
     const size_t o_Xbp = bf16 ? L.take(sizeof(__nv_bfloat16) * total_pad * tp.ldb) : 0;
     const size_t o_Xc = fold ? L.take(sizeof(__nv_bfloat16) * total * tp.ldb) : 0;
     const size_t o_Xcp = fold ? L.take(sizeof(__nv_bfloat16) * total_pad * tp.ldb) : 0;
     const size_t o_sqp = bf16 ? L.take(sizeof(float) * total_pad) : 0;
-    const size_t o_pad = bf16 ? L.take(sizeof(int64_t) * (B + 1)) : 0;
-    const size_t o_wb = bf16 ? L.take(sizeof(int64_t) * (tw.ctas + 1)) : 0;
-    const size_t o_wi = bf16 ? L.take(sizeof(TcItem) * std::max<size_t>(tw.items.size(), 1)) : 0;
-    char *base = ensure_arena(L.total);
+    // The work list, the candidates and the symmetrization's workspace, which
+    // the FP32 search's part rows share, as in fit().
+    const size_t o_pad = L.total;
+    auto pad_bytes = [&] { return bf16 || split ? align256(sizeof(int64_t) * (B + 1)) : 0; };
+    auto wb_bytes = [&] { return bf16 || split ? align256(sizeof(int64_t) * (tw.ctas + 1)) : 0; };
+    auto wi_bytes = [&] {
+        return bf16 || split ? align256(sizeof(TcItem) * std::max<size_t>(tw.items.size(), 1)) : 0;
+    };
+    auto cand_bytes = [&] {
+        const int C = bf16 ? tp.R : std::max(kp.C(), split ? sp.R : 0);
+        return align256(sizeof(int32_t) * total * C);
+    };
+    auto total_bytes = [&] {
+        const size_t rows =
+            split ? sizeof(__half) * (sp.fold ? 3 : 2) * (size_t)total_pad * sp.ldb : 0;
+        return o_pad + pad_bytes() + wb_bytes() + wi_bytes() + cand_bytes() +
+               align256(std::max(symmetrize_workspace_bytes(total, k), rows));
+    };
+    if (split && o.arena_limit && total_bytes() > o.arena_limit) split = false;
+    char *base = nullptr;
+    try {
+        base = ensure_arena(total_bytes());
+    } catch (const Error &) {
+        if (!split) throw;
+        cudaGetLastError();
+        split = false;
+        base = ensure_arena(total_bytes());
+    }
+    const size_t o_wb = o_pad + pad_bytes(), o_wi = o_wb + wb_bytes();
+    const size_t o_ci = o_wi + wi_bytes(), o_sym = o_ci + cand_bytes();
     float *Xp = (float *)(base + o_Xp);
     float *sqn = (float *)(base + o_sqn);
     int *flag = (int *)(base + o_flag);
     int32_t *cand_i = (int32_t *)(base + o_ci);
-    float *cand_d = (float *)(base + o_cd);
     int32_t *knn_i = (int32_t *)(base + o_ki);
     float *knn_d = (float *)(base + o_kd);
     int64_t *row_ptr = (int64_t *)(base + o_rp);
@@ -672,24 +794,23 @@ void ncvis_engine::fit_batched(const float *dX, size_t D, const int64_t *offsets
     NCVIS_CUDA(cudaMemcpyAsync(d_seed, h_seed.data(), sizeof(uint64_t) * B, cudaMemcpyHostToDevice, s));
     NCVIS_CUDA(cudaEventRecord(ev.ev[1], s));
     nv.next("ncvis.batched.preprocess");
-    NCVIS_CUDA(cudaMemsetAsync(flag, 0, sizeof(int) * 4, s));
+    NCVIS_CUDA(cudaMemsetAsync(flag, 0, sizeof(int) * 8, s));
     __nv_bfloat16 *Xb = bf16 ? (__nv_bfloat16 *)(base + o_Xb) : nullptr;
     __nv_bfloat16 *Xc = fold ? (__nv_bfloat16 *)(base + o_Xc) : nullptr;
-    launch_preprocess(dX, total, (int)D, dist, Xp, sqn, Xb, bf16 ? tp.ldb : 0, flag, s, Xc);
+    launch_preprocess(dX, total, (int)D, dist, Xp, sqn, Xb, bf16 ? tp.ldb : 0, flag, s, Xc,
+                      split ? (uint32_t *)flag + 4 : nullptr);
     NCVIS_CUDA(cudaEventRecord(ev.ev[2], s));
-    {
-        int bad = 0;
-        NCVIS_CUDA(cudaMemcpyAsync(&bad, flag, sizeof(int), cudaMemcpyDeviceToHost, s));
-        NCVIS_CUDA(cudaStreamSynchronize(s));
-        require(bad == 0, "[ncvis] input contains non-finite values");
-    }
+    int h_flag[8];
+    NCVIS_CUDA(cudaMemcpyAsync(h_flag, flag, sizeof(h_flag), cudaMemcpyDeviceToHost, s));
+    NCVIS_CUDA(cudaStreamSynchronize(s));
+    require(h_flag[0] == 0, "[ncvis] input contains non-finite values");
+    const float scale = split ? split_scale((const uint32_t *)h_flag + 4, dist) : 0.f;
     nv.next("ncvis.batched.knn");
     NCVIS_CUDA(cudaMemsetAsync(knn_i, 0xff, sizeof(int32_t) * nk, s));
-    if (bf16) {
+    int C = kp.C();  // candidates per point
+    if (bf16 || scale != 0.f) {
         // Problems at 256-aligned rows of a padded copy; one tensor-core launch
         // over every problem's query tiles, each against its own rows.
-        __nv_bfloat16 *Xb_pad = (__nv_bfloat16 *)(base + o_Xbp);
-        float *sqn_pad = (float *)(base + o_sqp);
         int64_t *d_pad = (int64_t *)(base + o_pad), *d_wb = (int64_t *)(base + o_wb);
         TcItem *d_wi = (TcItem *)(base + o_wi);
         NCVIS_CUDA(cudaMemcpyAsync(d_pad, tw.pad.data(), sizeof(int64_t) * (B + 1),
@@ -698,20 +819,39 @@ void ncvis_engine::fit_batched(const float *dX, size_t D, const int64_t *offsets
                                    cudaMemcpyHostToDevice, s));
         NCVIS_CUDA(cudaMemcpyAsync(d_wi, tw.items.data(), sizeof(TcItem) * tw.items.size(),
                                    cudaMemcpyHostToDevice, s));
-        NCVIS_CUDA(cudaMemsetAsync(Xb_pad, 0, sizeof(__nv_bfloat16) * total_pad * tp.ldb, s));
-        NCVIS_CUDA(cudaMemsetAsync(sqn_pad, 0, sizeof(float) * total_pad, s));
-        NCVIS_LAUNCH(pad_rows, (unsigned)ceil_div(total * 32, 256), 256, 0, s, Xb, sqn, d_off,
-                     d_pad, (int)B, total, tp.ldb, Xb_pad, sqn_pad);
-        __nv_bfloat16 *Xc_pad = nullptr;
-        if (fold) {
-            Xc_pad = (__nv_bfloat16 *)(base + o_Xcp);
-            NCVIS_CUDA(cudaMemsetAsync(Xc_pad, 0, sizeof(__nv_bfloat16) * total_pad * tp.ldb, s));
-            NCVIS_LAUNCH(pad_rows, (unsigned)ceil_div(total * 32, 256), 256, 0, s, Xc, sqn, d_off,
-                         d_pad, (int)B, total, tp.ldb, Xc_pad, sqn_pad);
+        TcWork work;
+        work.ctas = tw.ctas;
+        work.begin = d_wb;
+        work.end = d_wb + 1;
+        work.items = d_wi;
+        if (bf16) {
+            C = tp.R;
+            __nv_bfloat16 *Xb_pad = (__nv_bfloat16 *)(base + o_Xbp);
+            float *sqn_pad = (float *)(base + o_sqp);
+            NCVIS_CUDA(cudaMemsetAsync(Xb_pad, 0, sizeof(__nv_bfloat16) * total_pad * tp.ldb, s));
+            NCVIS_CUDA(cudaMemsetAsync(sqn_pad, 0, sizeof(float) * total_pad, s));
+            NCVIS_LAUNCH(pad_rows, (unsigned)ceil_div(total * 32, 256), 256, 0, s, Xb, sqn, d_off,
+                         d_pad, (int)B, total, tp.ldb, Xb_pad, sqn_pad);
+            __nv_bfloat16 *Xc_pad = nullptr;
+            if (fold) {
+                Xc_pad = (__nv_bfloat16 *)(base + o_Xcp);
+                NCVIS_CUDA(
+                    cudaMemsetAsync(Xc_pad, 0, sizeof(__nv_bfloat16) * total_pad * tp.ldb, s));
+                NCVIS_LAUNCH(pad_rows, (unsigned)ceil_div(total * 32, 256), 256, 0, s, Xc, sqn,
+                             d_off, d_pad, (int)B, total, tp.ldb, Xc_pad, sqn_pad);
+            }
+            launch_knn_select_tc(Xb_pad, sqn_pad, total_pad, tp, dist, cand_i, flag + 2, s, work,
+                                 Xc_pad);
+        } else {
+            // The part rows go straight to their padded places; rows between
+            // problems are never read as outputs or candidates (the work
+            // items' ends mask them).
+            C = sp.R;
+            __half *rows = (__half *)(base + o_sym);
+            launch_split_rows(Xp, sqn, total, (int)D, scale, sp, rows, total_pad, s, d_off, d_pad,
+                              (int)B);
+            launch_knn_select_split(rows, total_pad, sp, cand_i, flag + 2, s, work);
         }
-        TcWork work{tw.ctas, d_wb, d_wi, nullptr};
-        launch_knn_select_tc(Xb_pad, sqn_pad, total_pad, tp, dist, cand_i, cand_d, flag + 2, s,
-                             &work, Xc_pad);
         int timeout = 0;
         NCVIS_CUDA(cudaMemcpyAsync(&timeout, flag + 2, sizeof(int), cudaMemcpyDeviceToHost, s));
         NCVIS_CUDA(cudaStreamSynchronize(s));
@@ -723,7 +863,7 @@ void ncvis_engine::fit_batched(const float *dX, size_t D, const int64_t *offsets
         seg.tile_prefix = d_tq;
         seg.B = (int)B;
         seg.n_tiles = h_tq[B];
-        launch_knn_select_f32(Xp, sqn, total, (int)D, dist, kp, cand_i, cand_d, s, seg);
+        launch_knn_select_f32(Xp, sqn, total, (int)D, dist, kp, cand_i, s, seg);
     }
     NCVIS_CUDA(cudaEventRecord(ev.ev[3], s));
     nv.next("ncvis.batched.rerank");
@@ -962,13 +1102,13 @@ void knn_device(const float *dX, size_t N, size_t D, int distance, size_t k, int
         const bool ivf = (mode == NCVIS_KNN_IVF);
         const bool bf16 = (mode == NCVIS_KNN_BF16_RERANK) || ivf;
         cudaStream_t s = (cudaStream_t)stream;
-        KnnPlan kp = plan_knn_f32((int64_t)N, (int)k, rerank_factor);
+        KnnF32Plan fp;
+        if (!bf16) fp = plan_knn_fp32(N, D, (int)k, rerank_factor, distance);
         KnnTcPlan tp = plan_knn_tc((int64_t)N, (int)D, (int)k, rerank_factor, distance);
         const bool fold = bf16 && tp.fold;
         if (bf16)
             require(knn_tc_supported((int)D, tp.R),
                     "knn: the BF16 tensor-core kNN supports D <= 128", kUnsupported);
-        const int C = bf16 ? tp.R : kp.C();
         const KnnOrderPlan op = (bf16 && !ivf) ? plan_knn_order((int64_t)N, (int)D, tp, distance,
                                                                 (precision & NCVIS_KNN_CALLER_ORDER)
                                                                     ? -1
@@ -978,51 +1118,71 @@ void knn_device(const float *dX, size_t N, size_t D, int distance, size_t k, int
         Layout L;
         const size_t o_Xp = L.take(sizeof(float) * N * D);
         const size_t o_sqn = L.take(sizeof(float) * N);
-        const size_t o_flag = L.take(sizeof(int) * 2);
-        const size_t o_ci = L.take(sizeof(int32_t) * N * C);
-        const size_t o_cd = L.take(sizeof(float) * N * C);
+        const size_t o_flag = L.take(sizeof(int) * 8);
         const size_t o_Xb = bf16 ? L.take(sizeof(__nv_bfloat16) * N * tp.ldb) : 0;
         const size_t o_Xc = fold ? L.take(sizeof(__nv_bfloat16) * N * tp.ldb) : 0;
         const size_t o_ord = ord_bytes ? L.take(ord_bytes) : 0;
-        StreamBuffer buf(L.total, s);
+        const TcSweep whole = whole_tiles((int64_t)N, num_sms());
+        const size_t o_work =
+            bf16 && !ivf && op.C <= 0 ? L.take(sweep_work_bytes((int64_t)N, whole)) : 0;
+        const size_t o_ci = L.total;
+        auto cand_bytes = [&] {
+            return align256(bf16 ? sizeof(int32_t) * N * tp.R : fp.cand_bytes(N));
+        };
+        StreamBuffer buf(s);
+        try {
+            buf.alloc(o_ci + cand_bytes() + fp.block_bytes());
+        } catch (const Error &) {
+            // No room for the part rows: the search on the CUDA cores needs less.
+            if (!fp.split) throw;
+            cudaGetLastError();
+            fp.split = false;
+            buf.alloc(o_ci + cand_bytes());
+        }
+        const size_t o_block = o_ci + cand_bytes();
         char *base = (char *)buf.p;
-        NCVIS_CUDA(cudaMemsetAsync(base + o_flag, 0, sizeof(int) * 2, s));
+        int *flag = (int *)(base + o_flag);
+        int32_t *cand = (int32_t *)(base + o_ci);
+        NCVIS_CUDA(cudaMemsetAsync(flag, 0, sizeof(int) * 8, s));
         __nv_bfloat16 *Xb = bf16 ? (__nv_bfloat16 *)(base + o_Xb) : nullptr;
         __nv_bfloat16 *Xc = fold ? (__nv_bfloat16 *)(base + o_Xc) : nullptr;
         launch_preprocess(dX, (int64_t)N, (int)D, distance, (float *)(base + o_Xp),
-                          (float *)(base + o_sqn), Xb, bf16 ? tp.ldb : 0, (int *)(base + o_flag),
-                          s, Xc);
-        int bad = 0;
-        NCVIS_CUDA(cudaMemcpyAsync(&bad, base + o_flag, sizeof(int), cudaMemcpyDeviceToHost, s));
+                          (float *)(base + o_sqn), Xb, bf16 ? tp.ldb : 0, flag, s, Xc,
+                          fp.split ? (uint32_t *)flag + 4 : nullptr);
+        int h_flag[8];
+        NCVIS_CUDA(cudaMemcpyAsync(h_flag, flag, sizeof(h_flag), cudaMemcpyDeviceToHost, s));
         NCVIS_CUDA(cudaStreamSynchronize(s));
-        require(!bad, "knn: input contains non-finite values");
+        require(!h_flag[0], "knn: input contains non-finite values");
         NCVIS_CUDA(cudaMemsetAsync(d_inds, 0xff, sizeof(int32_t) * N * k, s));
         const int32_t *cell_order = nullptr;
+        Candidates found;
+        found.C = tp.R;
         if (ivf) {
             run_knn_ivf((float *)(base + o_Xp), Xb, Xc, (int64_t)N, (int)D, tp, distance,
-                        plan_ivf((int64_t)N, lists, probe), 42, (int32_t *)(base + o_ci),
-                        (int *)(base + o_flag) + 1, s);
+                        plan_ivf((int64_t)N, lists, probe), 42, cand, flag + 2, s);
         } else if (op.C > 0) {
             run_knn_tc_ordered((float *)(base + o_Xp), Xb, Xc, (int64_t)N, (int)D, tp, distance,
-                               op, 42, (int32_t *)(base + o_ci), (int *)(base + o_flag) + 1, s,
-                               base + o_ord, ord_bytes, nullptr, &cell_order);
+                               op, 42, cand, flag + 2, s, base + o_ord, ord_bytes, nullptr,
+                               &cell_order);
         } else if (bf16) {
-            launch_knn_select_tc(Xb, (float *)(base + o_sqn), (int64_t)N, tp, distance,
-                                 (int32_t *)(base + o_ci), (float *)(base + o_cd),
-                                 (int *)(base + o_flag) + 1, s, nullptr, Xc);
+            launch_knn_select_tc(Xb, (float *)(base + o_sqn), (int64_t)N, tp, distance, cand,
+                                 flag + 2, s,
+                                 launch_sweep_work((int64_t)N, whole, base + o_work, s), Xc);
+        } else {
+            found = run_knn_fp32((float *)(base + o_Xp), (float *)(base + o_sqn), N, D, distance,
+                                 fp, (const uint32_t *)h_flag + 4, cand, base + o_block, flag + 2,
+                                 s);
+        }
+        launch_rerank((float *)(base + o_Xp), (int64_t)N, (int)D, distance, cand, found.C, (int)k,
+                      d_inds, d_dists, s, cell_order, found.lists);
+        // The tensor-core kernel without its own check of the timeout flag.
+        if ((bf16 && !ivf && op.C <= 0) || fp.split) {
             int timeout = 0;
-            NCVIS_CUDA(cudaMemcpyAsync(&timeout, (int *)(base + o_flag) + 1, sizeof(int),
-                                       cudaMemcpyDeviceToHost, s));
+            NCVIS_CUDA(cudaMemcpyAsync(&timeout, flag + 2, sizeof(int), cudaMemcpyDeviceToHost, s));
             NCVIS_CUDA(cudaStreamSynchronize(s));
             require(!timeout, "knn: the tensor-core kernel timed out waiting on a barrier",
                     kDeviceTimeout);
-        } else {
-            launch_knn_select_f32((float *)(base + o_Xp), (float *)(base + o_sqn), (int64_t)N,
-                                  (int)D, distance, kp, (int32_t *)(base + o_ci),
-                                  (float *)(base + o_cd), s);
         }
-        launch_rerank((float *)(base + o_Xp), (int64_t)N, (int)D, distance,
-                      (int32_t *)(base + o_ci), C, (int)k, d_inds, d_dists, s, cell_order);
     }
 }
 

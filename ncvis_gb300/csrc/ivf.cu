@@ -266,7 +266,13 @@ TcWork upload(const HostWork &w, const int32_t *map, DeviceArena &arena) {
     if (!w.items.empty())
         NCVIS_CUDA(cudaMemcpyAsync(items, w.items.data(), sizeof(TcItem) * w.items.size(),
                                    cudaMemcpyHostToDevice, arena.s));
-    return TcWork{w.ctas, begin, items, map};
+    TcWork work;
+    work.ctas = w.ctas;
+    work.begin = begin;
+    work.end = begin + 1;
+    work.items = items;
+    work.map = map;
+    return work;
 }
 
 void check_timeout(int *flag, cudaStream_t s) {

@@ -1,7 +1,8 @@
 // K3 + K4: exact kNN in FP32, the plain drop-in replacement for the
 // reference's HNSW build and query (src/ncvis.cpp:72-153).
 //
-// K3 (knn_select_f32): a tiled FP32 FFMA distance GEMM.  A block owns 64
+// K3 (knn_select_f32): a tiled FP32 FFMA distance GEMM, for the shapes the
+// tensor cores' FP32 search (knn_tc.cu, kParts = 2) does not take.  A block owns 64
 // query points and sweeps one candidate range in tiles of 128; each thread
 // accumulates a 4 x 8 patch of dot products.  Distances use the GEMM forms
 // |q|^2 + |c|^2 - 2<q,c> (squared L2) and 1 - <q,c> (inner-product spaces).
@@ -19,6 +20,7 @@
 // findKNN stores them.
 #include <algorithm>
 #include <cfloat>
+#include <type_traits>
 
 #include "common.cuh"
 #include "stages.cuh"
@@ -76,8 +78,7 @@ __device__ inline SelectSmem carve(char *base, int R) {
 __global__ void __launch_bounds__(NT) knn_select_f32(const float *__restrict__ Xp,
                                                      const float *__restrict__ sqnorm, int64_t N,
                                                      int D, int dist, int R, int splits,
-                                                     int32_t *__restrict__ cand_i,
-                                                     float *__restrict__ cand_d, Segments seg) {
+                                                     int32_t *__restrict__ cand_i, Segments seg) {
     extern __shared__ __align__(16) char smem_raw[];
     SelectSmem sm = carve(smem_raw, R);
     const int tid = threadIdx.x;
@@ -228,26 +229,34 @@ __global__ void __launch_bounds__(NT) knn_select_f32(const float *__restrict__ X
         if (gq >= N) continue;
         const bool have = p < sm.lst_n[q];
         cand_i[gq * C + (int64_t)split * R + p] = have ? sm.lst_i[p * BM + q] : -1;
-        cand_d[gq * C + (int64_t)split * R + p] = have ? sm.lst_d[p * BM + q] : FLT_MAX;
     }
 }
 
 // One warp per point.  The query row is spread over the lanes (coordinate
 // t in lane t % 32); each candidate row is read coalesced and its exact FP32
 // distance reduced across the warp (the same lane split for (i, j) and
-// (j, i), so d(i, j) == d(j, i)).  Candidates are then ranked; C <= 1024.
-template <int T>  // ceil(D / 32) coordinates per lane, T <= 4; T == 0: any D
+// (j, i), so d(i, j) == d(j, i)).  Candidates are then ranked; at most 1024.
+// Positions from lists.row0 on have lists.count more lists of C candidates.
+// T: ceil(D / 32) coordinates per lane, T <= 4; T == 0: any D.  kLists: some
+// rows have further lists (a form of its own, so that the other keeps 64
+// registers: with both in one the rerank of 1,024,000 rows took 3.5 ms, not 2.6).
+template <int T, bool kLists>
 __global__ void __launch_bounds__(128) rerank_rows(const float *__restrict__ Xp, int64_t N, int D,
                                                    int dist, const int32_t *__restrict__ cand_i,
-                                                   int C, int k, int32_t *__restrict__ inds,
+                                                   int C0, int k, int32_t *__restrict__ inds,
                                                    float *__restrict__ dists,
-                                                   const int32_t *__restrict__ order) {
+                                                   const int32_t *__restrict__ order,
+                                                   TcLists lists) {
     extern __shared__ __align__(16) char smem_raw[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t w = (int64_t)blockIdx.x * (blockDim.x >> 5) + warp;
-    float *sd = (float *)smem_raw + (size_t)warp * C * 2;
-    int *si = (int *)(sd + C);
+    const int most = kLists ? C0 * (1 + lists.count) : C0;
+    float *sd = (float *)smem_raw + (size_t)warp * most * 2;
+    int *si = (int *)(sd + most);
     if (w >= N) return;
+    const bool more = kLists && w >= lists.row0;
+    const int C = more ? most : C0;
+    const int32_t *extra = more ? lists.extra + (w - lists.row0) * lists.count * C0 : nullptr;
     // Rows in `order` (a permutation of [0, N)) when given: neighbouring points
     // then run together and share their candidates' rows in L2.
     const int64_t row = order ? (int64_t)order[w] : w;
@@ -270,7 +279,11 @@ __global__ void __launch_bounds__(128) rerank_rows(const float *__restrict__ Xp,
         float part[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            idx[u] = (c0 + u < C) ? cand_i[row * C + c0 + u] : -1;  // warp-uniform
+            const int c = c0 + u;  // warp-uniform
+            if constexpr (kLists)
+                idx[u] = c < C0 ? cand_i[row * C0 + c] : (c < C ? extra[c - C0] : -1);
+            else
+                idx[u] = c < C0 ? cand_i[row * C0 + c] : -1;
             part[u] = 0.f;
         }
         if (T > 0) {
@@ -359,7 +372,7 @@ KnnPlan plan_knn_f32(int64_t N, int k, int rerank_factor) {
 }
 
 void launch_knn_select_f32(const float *Xp, const float *sqnorm, int64_t N, int D, int dist,
-                           const KnnPlan &plan, int32_t *cand_i, float *cand_d, cudaStream_t s,
+                           const KnnPlan &plan, int32_t *cand_i, cudaStream_t s,
                            const Segments &seg) {
     const size_t smem = select_smem_bytes(plan.R);
     // Set on every launch: the attribute is per device, and a cached flag
@@ -369,29 +382,38 @@ void launch_knn_select_f32(const float *Xp, const float *sqnorm, int64_t N, int 
     const int64_t tiles = seg.B > 0 ? seg.n_tiles : (int64_t)ceil_div(N, BM);
     dim3 grid((unsigned)tiles, plan.splits);
     NCVIS_LAUNCH(knn_select_f32, grid, NT, smem, s, Xp, sqnorm, N, D, dist, plan.R, plan.splits,
-                 cand_i, cand_d, seg);
+                 cand_i, seg);
 }
 
 void launch_rerank(const float *Xp, int64_t N, int D, int dist, const int32_t *cand_i, int C,
-                   int k, int32_t *inds, float *dists, cudaStream_t s, const int32_t *order) {
-    require(C <= 1024, "rerank: too many candidates per point");
+                   int k, int32_t *inds, float *dists, cudaStream_t s, const int32_t *order,
+                   const TcLists &lists) {
+    const int most = C * (1 + lists.count);
+    require(most <= 1024, "rerank: too many candidates per point");
     const int warps = 4;
-    const size_t smem = (size_t)warps * C * 8;
+    const size_t smem = (size_t)warps * most * 8;
     const unsigned grid = ceil_div(N, warps);
     // The shared-memory attribute is set on every launch (per device; no
     // cached flag shared between host threads).
     auto go = [&](auto kernel) {
         NCVIS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         NCVIS_LAUNCH(kernel, grid, warps * 32, smem, s, Xp, N, D, dist, cand_i, C, k, inds, dists,
-                     order);
+                     order, lists);
     };
-    switch ((D + 31) / 32) {
-        case 1: go(rerank_rows<1>); break;
-        case 2: go(rerank_rows<2>); break;
-        case 3: go(rerank_rows<3>); break;
-        case 4: go(rerank_rows<4>); break;
-        default: go(rerank_rows<0>);
-    }
+    auto by_width = [&](auto more) {
+        constexpr bool kLists = decltype(more)::value;
+        switch ((D + 31) / 32) {
+            case 1: go(rerank_rows<1, kLists>); break;
+            case 2: go(rerank_rows<2, kLists>); break;
+            case 3: go(rerank_rows<3, kLists>); break;
+            case 4: go(rerank_rows<4, kLists>); break;
+            default: go(rerank_rows<0, kLists>);
+        }
+    };
+    if (lists.count > 0)
+        by_width(std::true_type());
+    else
+        by_width(std::false_type());
 }
 
 }  // namespace ncvis_gpu

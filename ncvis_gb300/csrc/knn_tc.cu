@@ -6,7 +6,8 @@
 // Work decomposition (one persistent CTA per SM, 11 warps):
 //   * a query tile is 256 preprocessed points (two M=128 halves), held in
 //     shared memory for the whole sweep (TMA, 128-byte swizzle, K-major);
-//   * candidate tiles of 128 points stream through a 3-stage TMA ring;
+//   * candidate tiles of 128 points stream through a TMA ring, a stage per part
+//     of a tile;
 //   * warp 0 issues TMA; warps 1 and 10 issue tcgen05.mma (M=128, N=128,
 //     K=16 steps), one query half each, into one of two double-buffered
 //     2x128-column FP32 accumulators (512 TMEM columns; warp 1 allocates);
@@ -19,17 +20,24 @@
 //     qualifying candidates go to a per-row queue in shared memory, which the
 //     warp inserts into the rows' register-resident sorted lists in lockstep
 //     rounds (R compare-exchanges each) when a queue passes half full;
-//   * a CTA takes query tiles round-robin over one problem, or items from its
-//     own work list: an item is a query tile's rows and one candidate range
-//     (masked at both ends), and may continue the previous item's tile, so
-//     one tile's lists are built over several ranges (batched problems: the
-//     tile's own problem; the inverted file: the tile's probed cells), with
-//     an optional map from sorted rows back to the caller's numbering;
+//   * a CTA takes items from its own work list: an item is a query tile's rows
+//     and one candidate range (masked at both ends), and may continue the
+//     previous item's tile, so one tile's lists are built over several ranges
+//     (batched problems: the tile's own problem; the inverted file: the tile's
+//     probed cells), with an optional map from sorted rows back to the caller's
+//     numbering; items of several CTAs may share a query tile, each writing a
+//     list of its own (sweep_items: the last wave of one problem's tiles);
 //   * squared L2 with D <= 126 folds the candidate norms into the product:
 //     candidates come from a second BF16 copy whose columns D, D + 1 hold
 //     -|c|^2 / 2 as a BF16 high and low part, the queries' copy 1, 1 there, so
 //     the accumulator holds <q, c> - |c|^2 / 2 and the scan is the
-//     inner-product one (otherwise the scan adds the FP32 norms per column).
+//     inner-product one (otherwise the scan adds the FP32 norms per column);
+//   * kParts = 2 is the FP32 search's form (launch_knn_select_split): every row
+//     is an FP16 high and low part (split_rows, preprocess.cu), a candidate
+//     tile is taken in two parts, and its product is the sum of three FP16
+//     products accumulated in FP32, the small ones first: q_hi c_lo, then
+//     q_lo c_hi and q_hi c_hi (rows of up to 32 columns q_lo c_lo as well, which
+//     is not below the others' rounding there).
 // Every mbarrier wait is bounded in time: on expiry the CTA sets *err,
 // stops, drains its MMAs and in-flight TMA copies, frees TMEM and returns.
 // The waits between roles use the plan's limit (default ~2 s); the drain
@@ -53,7 +61,6 @@ namespace {
 
 constexpr int kQueryTile = 256;   // queries per CTA tile (2 x M=128)
 constexpr int kCandTile = 128;    // candidates per tile (N=128)
-constexpr int kStages = 3;        // candidate-tile ring
 constexpr int kAtomBytes = 128 * 128;  // 128 rows x 128 bytes (64 bf16) per swizzle atom column
 constexpr int kMaxAtoms = 2;      // K <= 128
 constexpr int kThreads = 352;
@@ -61,13 +68,21 @@ constexpr int kEpiWarp0 = 2;
 constexpr int kEpiWarps = 8;
 constexpr int kMmaWarp1 = 10;  // issues the second query half's MMAs (warp 1 the first)
 constexpr int kEpiThreads = kEpiWarps * 32;
-constexpr int kQueue = 32;  // per-row insertion queue slots (shared memory)
 constexpr uint32_t kTmemCols = 512;
+constexpr int kLowLowSteps = 2;  // K steps up to which the low parts' product is taken too
 constexpr long long kWaitCycles = 4000000000LL;  // ~2 s at 2 GHz
 
+// Shared memory by the number of parts a row is held in: the query tile takes
+// 64 KB a part, so the two-part form has a ring of 2 stages and 16 queue slots
+// per row where the one-part form has 3 and 32 (both 224 KB in all).  Stages of
+// 64 columns (half a part, twice as many) made the BF16 sweep of 1,024,000 x 100
+// 18% slower: the MMA warps then wait within a tile too.
+template <int kParts>
 struct SharedStorage {
+    static constexpr int kStages = kParts == 1 ? 3 : 2;  // candidate ring (32 KB each)
+    static constexpr int kQueue = kParts == 1 ? 32 : 16;  // per-row insertion queue slots
     // 1024-byte aligned tiles first (128B swizzle atoms repeat every 1024 B).
-    uint8_t a[2][kMaxAtoms][kAtomBytes];
+    uint8_t a[2][kParts][kMaxAtoms][kAtomBytes];
     uint8_t b[kStages][kMaxAtoms][kAtomBytes];
     float queue_v[kQueue][kEpiThreads];    // queued candidate scores, [slot][thread]
     int32_t queue_i[kQueue][kEpiThreads];  // and their candidate indices
@@ -113,13 +128,13 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
 
 // Bounded wait (`limit` SM cycles) for the phase of `parity`; false if it
 // expired or the CTA aborted.
-__device__ __forceinline__ bool mbar_wait(SharedStorage &s, uint64_t *bar, uint32_t parity,
+__device__ __forceinline__ bool mbar_wait(volatile int &abort, uint64_t *bar, uint32_t parity,
                                           int *err, int code, long long limit) {
     const long long t0 = clock64();
     while (!mbar_try_wait(bar, parity)) {
-        if (s.abort) return false;
+        if (abort) return false;
         if (clock64() - t0 > limit) {
-            s.abort = 1;
+            abort = 1;
             atomicExch(err, code);
             return false;
         }
@@ -147,11 +162,15 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr) {
     return d;
 }
 
-// Instruction descriptor, kind::f16: D f32, A and B bf16, both K-major, M=128, N=128.
-constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kCandTile >> 3) << 17) |
-                            ((uint32_t)(128 >> 4) << 24);
+// Instruction descriptor, kind::f16: D f32, A and B both bf16 (type 1) or both
+// f16 (type 0), both K-major, M=128, N=128.
+constexpr uint32_t idesc(uint32_t type) {
+    return (1u << 4) | (type << 7) | (type << 10) | ((uint32_t)(kCandTile >> 3) << 17) |
+           ((uint32_t)(128 >> 4) << 24);
+}
 
-__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t acc) {
+template <uint32_t kIdesc>
+__device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t acc) {
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %3, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %4, p;\n\t}" ::"r"(tmem_d),
@@ -277,62 +296,94 @@ __device__ __forceinline__ void flush_queue(float (&ls)[R], int32_t (&li)[R], fl
     __syncwarp();
 }
 
-// One item of work: the query tile of 256 rows from row0 (rows at or past
-// qend are not outputs) against candidate rows [lo, hi); `cont`: the item
+// One item of work (TcItem): the query tile of 256 rows from row0 (rows at or
+// past qend are not outputs) against candidate rows [lo, hi); `cont`: the item
 // extends the previous item's query tile (no reload, lists carry over);
 // `more`: a later item extends this one (lists written after the last).
-// Without a work list a CTA takes the query tiles blockIdx.x,
-// blockIdx.x + gridDim.x, ... of one problem of N rows, each against all N.
 struct QueryTile {
-    int32_t row0, qend, lo, hi, out_off;  // N < 2^31
+    int32_t row0, qend, lo, hi;  // N < 2^31
     bool cont, more;
 };
 
-__device__ __forceinline__ int64_t work_items(const int64_t *__restrict__ work_begin,
-                                              int64_t n_qt) {
-    if (work_begin) return work_begin[blockIdx.x + 1] - work_begin[blockIdx.x];
-    return blockIdx.x < n_qt ? (n_qt - 1 - blockIdx.x) / gridDim.x + 1 : 0;
-}
-
-__device__ __forceinline__ QueryTile work_item(const int64_t *__restrict__ work_begin,
-                                               const TcItem *__restrict__ work, int64_t it,
-                                               int64_t N) {
+__device__ __forceinline__ QueryTile work_item(const TcItem *__restrict__ work, int64_t it) {
+    const TcItem w = work[it];
     QueryTile q;
-    if (work_begin) {
-        const TcItem w = work[work_begin[blockIdx.x] + it];
-        q.row0 = w.row0;
-        q.qend = w.qend;
-        q.lo = w.lo;
-        q.hi = w.hi;
-        q.out_off = w.out_off;
-        q.cont = (w.flags & kTcContinue) != 0;
-        q.more = (w.flags & kTcMore) != 0;
-    } else {
-        q.row0 = (int32_t)(((int64_t)blockIdx.x + it * gridDim.x) * kQueryTile);
-        q.qend = (int32_t)N;
-        q.lo = 0;
-        q.hi = (int32_t)N;
-        q.out_off = 0;
-        q.cont = q.more = false;
-    }
+    q.row0 = w.row0;
+    q.qend = w.qend;
+    q.lo = w.lo;
+    q.hi = w.hi;
+    q.cont = (w.flags & kTcContinue) != 0;
+    q.more = (w.flags & kTcMore) != 0;
     return q;
 }
 
-template <int R, bool kIP>
+// The work list of one problem of N rows spread as `w` says: CTA b takes the
+// whole query tiles b, b + ctas, ... below full_qt, then its run of the other
+// tiles' (query tile, candidate tile) pairs, an item per query tile it meets.
+__global__ void sweep_items(int64_t N, TcSweep w, int stride, int64_t *__restrict__ begin,
+                            int64_t *__restrict__ end, TcItem *__restrict__ items) {
+    const int64_t b = blockIdx.x, G = w.rest_ctas;
+    const int64_t n_qt = (N + kQueryTile - 1) / kQueryTile, n_ct = (N + kCandTile - 1) / kCandTile;
+    const int64_t rest = (n_qt - w.full_qt) * n_ct;
+    const int64_t r0 = b < G ? rest * b / G : 0, r1 = b < G ? rest * (b + 1) / G : 0;
+    const int64_t whole = b < w.full_qt ? (w.full_qt - 1 - b) / w.ctas + 1 : 0;
+    const int64_t n = whole + (r1 > r0 ? (r1 - 1) / n_ct - r0 / n_ct + 1 : 0);
+    TcItem *mine = items + b * stride;
+    for (int64_t it = threadIdx.x; it < n; it += blockDim.x) {
+        TcItem q{};
+        q.qend = q.hi = (int32_t)N;
+        if (it < whole) {
+            q.row0 = (int32_t)((b + it * w.ctas) * kQueryTile);
+        } else {
+            const int64_t t = r0 / n_ct + (it - whole);  // query tile among the rest
+            const int64_t u0 = max(r0, t * n_ct), u1 = min(r1, (t + 1) * n_ct);
+            q.row0 = (int32_t)((w.full_qt + t) * kQueryTile);
+            q.lo = (int32_t)((u0 - t * n_ct) * kCandTile);
+            q.hi = (int32_t)min(N, (u1 - t * n_ct) * kCandTile);
+            // The tile's first pair is in the run of the last CTA that begins
+            // at or before it; the CTAs after it write the next lists.
+            q.slot = (int32_t)(b - ((t * n_ct + 1) * G - 1) / rest);
+        }
+        mine[it] = q;
+    }
+    if (threadIdx.x == 0) {
+        begin[b] = b * stride;
+        end[b] = b * stride + n;
+    }
+}
+
+// Items of one CTA at most: its whole tiles and the query tiles its run meets.
+int sweep_stride(int64_t N, const TcSweep &w) {
+    const int64_t n_qt = (N + kQueryTile - 1) / kQueryTile, n_ct = (N + kCandTile - 1) / kCandTile;
+    const int64_t run = ((n_qt - w.full_qt) * n_ct + w.rest_ctas - 1) / w.rest_ctas;
+    return (int)((w.full_qt + w.ctas - 1) / w.ctas + (run + n_ct - 1) / n_ct + 1);
+}
+
+// Rows of the operands' parts in their tensor maps: part p of row r is row
+// part[p] + r (part 0 the high or only one, part 1 the low one).
+struct TcParts {
+    int32_t q[2], c[2];
+};
+
+template <int R, bool kIP, int kParts>
 __global__ void __launch_bounds__(kThreads, 1)
     knn_select_tc(const __grid_constant__ CUtensorMap tmap,
-                  const __grid_constant__ CUtensorMap tmap_c, const float *__restrict__ sqnorm,
-                  int64_t N, int ksteps, int katoms, const int64_t *__restrict__ work_begin,
+                  const __grid_constant__ CUtensorMap tmap_c, const TcParts parts,
+                  const float *__restrict__ sqnorm, int ksteps, int katoms,
+                  const int64_t *__restrict__ work_begin, const int64_t *__restrict__ work_end,
                   const TcItem *__restrict__ work, const int32_t *__restrict__ row_map,
-                  int32_t *__restrict__ cand_i, int *__restrict__ err, long long wait_limit,
-                  int stall) {
+                  int32_t *__restrict__ cand_i, int32_t *__restrict__ extra, int64_t extra_row0,
+                  int extra_lists, int *__restrict__ err, long long wait_limit, int stall) {
+    using Shared = SharedStorage<kParts>;
+    constexpr int kStages = Shared::kStages;
+    constexpr int kQueue = Shared::kQueue;
     extern __shared__ uint8_t smem_raw[];
-    SharedStorage &s = *reinterpret_cast<SharedStorage *>(
-        (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    Shared &s = *reinterpret_cast<Shared *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
+                                            ~(uintptr_t)1023);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t n_qt = (N + kQueryTile - 1) / kQueryTile;
-    const int64_t n_items = work_items(work_begin, n_qt);
-    const uint32_t a_bytes = 2u * katoms * kAtomBytes;
+    const int64_t n_items = work_end[blockIdx.x] - work_begin[blockIdx.x];
+    work += work_begin[blockIdx.x];
+    const uint32_t a_bytes = 2u * kParts * katoms * kAtomBytes;
     const uint32_t b_bytes = (uint32_t)katoms * kAtomBytes;
 
     if (threadIdx.x == 0) {
@@ -376,29 +427,37 @@ __global__ void __launch_bounds__(kThreads, 1)
         for (int i = 0; i < kStages; ++i) issued[i] = false, issued_parity[i] = 0;
         bool a_issued = false;
         uint32_t a_parity = 0;
-        if (stall) mbar_wait(s, &s.never, 0, err, 7, wait_limit);
+        if (stall) mbar_wait(s.abort, &s.never, 0, err, 7, wait_limit);
         for (int64_t it = 0; it < n_items && !s.abort; ++it) {
-            const QueryTile q = work_item(work_begin, work, it, N);
+            const QueryTile q = work_item(work, it);
             if (!q.cont) {
-                if (!mbar_wait(s, &s.a_empty, a_phase ^ 1, err, 1, wait_limit)) break;
+                if (!mbar_wait(s.abort, &s.a_empty, a_phase ^ 1, err, 1, wait_limit)) break;
                 mbar_expect_tx(&s.a_full, a_bytes);
                 for (int h = 0; h < 2; ++h)
-                    for (int at = 0; at < katoms; ++at)
-                        tma_load_2d(s.a[h][at], &tmap, &s.a_full, at * 64,
-                                    (int)(q.row0 + h * 128));
+                    for (int p = 0; p < kParts; ++p)
+                        for (int at = 0; at < katoms; ++at)
+                            tma_load_2d(s.a[h][p][at], &tmap, &s.a_full, at * 64,
+                                        (int)(parts.q[p] + q.row0 + h * 128));
                 a_issued = true;
                 a_parity = a_phase;
                 a_phase ^= 1;
             }
-            for (int64_t ct = q.lo / kCandTile; ct * kCandTile < q.hi; ++ct) {
-                if (!mbar_wait(s, &s.empty[stage], phase ^ 1, err, 2, wait_limit)) break;
-                mbar_expect_tx(&s.full[stage], b_bytes);
-                for (int at = 0; at < katoms; ++at)
-                    tma_load_2d(s.b[stage][at], &tmap_c, &s.full[stage], at * 64,
-                                (int)(ct * kCandTile));
-                issued[stage] = true;
-                issued_parity[stage] = phase;
-                if (++stage == kStages) stage = 0, phase ^= 1;
+            bool ok = true;
+            for (int64_t ct = q.lo / kCandTile; ok && ct * kCandTile < q.hi; ++ct) {
+                // The low part of a tile first, then the high one.
+                for (int p = kParts - 1; p >= 0; --p) {
+                    if (!mbar_wait(s.abort, &s.empty[stage], phase ^ 1, err, 2, wait_limit)) {
+                        ok = false;
+                        break;
+                    }
+                    mbar_expect_tx(&s.full[stage], b_bytes);
+                    for (int at = 0; at < katoms; ++at)
+                        tma_load_2d(s.b[stage][at], &tmap_c, &s.full[stage], at * 64,
+                                    (int)(parts.c[p] + ct * kCandTile));
+                    issued[stage] = true;
+                    issued_parity[stage] = phase;
+                    if (++stage == kStages) stage = 0, phase ^= 1;
+                }
             }
         }
         // Copies still in flight must land before the CTA's shared memory goes away.
@@ -419,29 +478,41 @@ __global__ void __launch_bounds__(kThreads, 1)
         uint32_t phase = 0, a_phase = 0, acc_phase = 0;
         int acc = 0;
         for (int64_t it = 0; it < n_items && !s.abort; ++it) {
-            const QueryTile q = work_item(work_begin, work, it, N);
+            const QueryTile q = work_item(work, it);
             if (!q.cont) {
-                if (!mbar_wait(s, &s.a_full, a_phase, err, 3, wait_limit)) break;
+                if (!mbar_wait(s.abort, &s.a_full, a_phase, err, 3, wait_limit)) break;
                 a_phase ^= 1;
             }
             tmem_fence_after();
-            for (int64_t ct = q.lo / kCandTile; ct * kCandTile < q.hi; ++ct) {
-                if (!mbar_wait(s, &s.acc_empty[acc][h], acc_phase ^ 1, err, 4, wait_limit)) break;
-                if (!mbar_wait(s, &s.full[stage], phase, err, 5, wait_limit)) break;
-                tmem_fence_after();
-                {
-                    const uint32_t d_tmem = tmem + (uint32_t)(acc * 256 + h * 128);
-                    for (int ks = 0; ks < ksteps; ++ks) {
-                        const int at = ks >> 2;
-                        const uint32_t off = (uint32_t)(ks & 3) * 32;
-                        const uint64_t ad = smem_desc(smem_u32(s.a[h][at]) + off);
-                        const uint64_t bd = smem_desc(smem_u32(s.b[stage][at]) + off);
-                        umma_bf16(d_tmem, ad, bd, ks > 0 ? 1u : 0u);
+            bool ok = true;
+            for (int64_t ct = q.lo / kCandTile; ok && ct * kCandTile < q.hi; ++ct) {
+                if (!mbar_wait(s.abort, &s.acc_empty[acc][h], acc_phase ^ 1, err, 4, wait_limit))
+                    break;
+                const uint32_t d_tmem = tmem + (uint32_t)(acc * 256 + h * 128);
+                uint32_t accumulate = 0u;
+                for (int p = kParts - 1; p >= 0; --p) {
+                    if (!mbar_wait(s.abort, &s.full[stage], phase, err, 5, wait_limit)) {
+                        ok = false;
+                        break;
                     }
+                    tmem_fence_after();
+                    auto product = [&](int qp) {
+                        for (int ks = 0; ks < ksteps; ++ks) {
+                            const int at = ks >> 2;
+                            const uint32_t off = (uint32_t)(ks & 3) * 32;
+                            const uint64_t ad = smem_desc(smem_u32(s.a[h][qp][at]) + off);
+                            const uint64_t bd = smem_desc(smem_u32(s.b[stage][at]) + off);
+                            umma_f16<idesc(kParts == 1 ? 1u : 0u)>(d_tmem, ad, bd, accumulate);
+                            accumulate = 1u;
+                        }
+                    };
+                    if (kParts == 2 && (p == 0 || ksteps <= kLowLowSteps)) product(kParts - 1);
+                    product(0);
+                    umma_commit(&s.empty[stage]);
+                    if (++stage == kStages) stage = 0, phase ^= 1;
                 }
-                umma_commit(&s.empty[stage]);
+                if (!ok) break;
                 umma_commit(&s.acc_full[acc][h]);
-                if (++stage == kStages) stage = 0, phase ^= 1;
                 acc ^= 1;
                 if (acc == 0) acc_phase ^= 1;
             }
@@ -461,6 +532,9 @@ __global__ void __launch_bounds__(kThreads, 1)
         // Accumulator columns per tcgen05.ld: 32 with 32-entry lists; 64-entry
         // lists leave registers for 16.
         constexpr int kC = R <= 32 ? 32 : 16;
+        // Columns queued between two looks at the queue: half the queue, so
+        // that one that is at most half full takes them.
+        constexpr int kAppend = kQueue / 2;
         uint32_t acc_phase = 0;
         int acc = 0;
         float ls[R];
@@ -470,9 +544,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         for (int64_t it = 0; it < n_items; ++it) {
             // Lanes read the abort flag at different times: the warp stops as one.
             if (__any_sync(0xffffffffu, s.abort != 0)) break;
-            const QueryTile q = work_item(work_begin, work, it, N);
-            const int64_t grow = q.row0 + row_in_tile;
-            const bool live = grow < q.qend;
+            const QueryTile q = work_item(work, it);
+            const bool live = q.row0 + row_in_tile < q.qend;
             if (!q.cont) {
 #pragma unroll
                 for (int t = 0; t < R; ++t) {
@@ -484,7 +557,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             }
             bool ok = true;
             for (int64_t ct = q.lo / kCandTile; ct * kCandTile < q.hi; ++ct) {
-                const bool got = mbar_wait(s, &s.acc_full[acc][h], acc_phase, err, 6, wait_limit);
+                const bool got = mbar_wait(s.abort, &s.acc_full[acc][h], acc_phase, err, 6, wait_limit);
                 if (!__all_sync(0xffffffffu, got)) {
                     ok = false;
                     break;
@@ -553,17 +626,17 @@ __global__ void __launch_bounds__(kThreads, 1)
                     const float best = tree_reduce<false, kG>(gb);
                     const bool hit = live && best < worst;
                     if (!__any_sync(0xffffffffu, hit)) continue;
-                    // Qualifying candidates are queued 16 columns at a time,
+                    // Qualifying candidates are queued kAppend columns at a time,
                     // looking only into the 8-column groups whose best beats
                     // the row's worst; a queue past half full is flushed into
                     // the lists first.
 #pragma unroll
-                    for (int half = 0; half < kC / 16; ++half) {
-                        if (__any_sync(0xffffffffu, qlen > kQueue - 16))
+                    for (int part = 0; part < kC / kAppend; ++part) {
+                        if (__any_sync(0xffffffffu, qlen > kQueue - kAppend))
                             flush_queue<R>(ls, li, worst, qlen, s.queue_v, s.queue_i, etid);
                         if (hit) {
 #pragma unroll
-                            for (int g = 2 * half; g < 2 * half + 2; ++g) {
+                            for (int g = part * kAppend / 8; g < (part + 1) * kAppend / 8; ++g) {
                                 if (gb[g] < worst) {
 #pragma unroll
                                     for (int j = 8 * g; j < 8 * g + 8; ++j) {
@@ -585,19 +658,28 @@ __global__ void __launch_bounds__(kThreads, 1)
                 // is released, so that the MMAs of the next tiles go on meanwhile;
                 // a flush inside the tile happens only when one tile overfills a
                 // queue (early in the sweep).
-                if (__any_sync(0xffffffffu, qlen > kQueue - 16))
+                if (__any_sync(0xffffffffu, qlen > kQueue - kAppend))
                     flush_queue<R>(ls, li, worst, qlen, s.queue_v, s.queue_i, etid);
             }
             if (!ok) break;
             if (q.more) continue;  // the next item extends this query tile
             flush_queue<R>(ls, li, worst, qlen, s.queue_v, s.queue_i, etid);
-            if (live) {
-                const int64_t orow = row_map ? (int64_t)row_map[grow] : grow + q.out_off;
+            // The item read again: where its lists go is not held in registers
+            // over the sweep (the barrier keeps the two reads apart).
+            int64_t again = it;
+            asm volatile("" : "+l"(again));
+            const TcItem o = work[again];
+            const int64_t grow = o.row0 + row_in_tile;
+            if (grow < o.qend) {
+                const int64_t orow = row_map ? (int64_t)row_map[grow] : grow + o.out_off;
+                int32_t *out =
+                    o.slot == 0
+                        ? cand_i + orow * R
+                        : extra + ((grow - extra_row0) * extra_lists + (o.slot - 1)) * R;
 #pragma unroll
                 for (int t = 0; t < R; ++t)
-                    cand_i[orow * R + t] =
-                        li[t] < 0 ? -1
-                                  : (row_map ? row_map[li[t]] : (int32_t)(li[t] + q.out_off));
+                    out[t] = li[t] < 0 ? -1
+                                       : (row_map ? row_map[li[t]] : (int32_t)(li[t] + o.out_off));
             }
         }
     }
@@ -636,9 +718,77 @@ KnnTcPlan plan_knn_tc(int64_t N, int D, int k, int rerank_factor, int dist) {
     // Squared L2 folds -|c|^2 / 2 into two extra K columns when they fit (D <= 126).
     p.fold = (dist == kSquaredL2) && D + 2 <= 64 * kMaxAtoms;
     p.ldb = (D + (p.fold ? 2 : 0) + 7) / 8 * 8;
-    p.Npad = N;
     (void)N;
     return p;
+}
+
+KnnTcPlan plan_knn_split(int D, int R, int dist) {
+    KnnTcPlan p;
+    p.parts = 2;
+    p.R = R <= 32 ? 32 : 64;
+    // Squared L2 folds -|c|^2 / 2 into three extra columns.
+    p.fold = dist == kSquaredL2;
+    p.ldb = (D + (p.fold ? 3 : 0) + 7) / 8 * 8;
+    return p;
+}
+
+// Scores against 64 bits (rms over 500 queries' 32 best of 20,000, the three
+// products against K3's FP32 sums): 0.46 to 0.94 times K3's error for 8 to 126
+// columns, raw and unit rows, products and squared L2; 1.04 times at 4 columns
+// and 1.4 at 2 (the parts' own rounding), which therefore stay on the CUDA cores.
+constexpr int kSplitMinCols = 8;
+
+bool knn_split_supported(int64_t N, int D, int R, int dist) {
+    return N < (int64_t(1) << 30) && R <= 64 && D >= kSplitMinCols &&
+           D + (dist == kSquaredL2 ? 3 : 0) <= 64 * kMaxAtoms;
+}
+
+TcSweep plan_sweep(int64_t N, int ctas) {
+    TcSweep w;
+    const int64_t n_qt = (N + kQueryTile - 1) / kQueryTile, n_ct = (N + kCandTile - 1) / kCandTile;
+    w.full_qt = n_qt / ctas * ctas;
+    const int64_t left = n_qt - w.full_qt;
+    w.ctas = ctas;
+    if (left == 0) return w;
+    if (10 * left > 9 * ctas) {  // the last wave is nearly full
+        return whole_tiles(N, ctas);
+    }
+    // Runs of at least two candidate tiles and a sixth of a sweep: shorter ones
+    // give the rows more candidates to re-rank than they save.
+    const int64_t rest = left * n_ct;
+    w.rest_ctas = (int)std::max<int64_t>(1, std::min<int64_t>({ctas, rest / 2, 6 * left}));
+    if (w.full_qt == 0) w.ctas = w.rest_ctas;
+    const int64_t G = w.rest_ctas;
+    for (int64_t t = 0; t < left; ++t) {
+        const int64_t first = ((t * n_ct + 1) * G - 1) / rest, last = ((t + 1) * n_ct * G - 1) / rest;
+        w.lists = std::max<int>(w.lists, (int)(last - first + 1));
+    }
+    w.split_rows = N - w.full_qt * kQueryTile;
+    return w;
+}
+
+TcSweep whole_tiles(int64_t N, int ctas) {
+    TcSweep w;
+    w.full_qt = (N + kQueryTile - 1) / kQueryTile;
+    w.ctas = (int)std::min<int64_t>(w.full_qt, ctas);
+    return w;
+}
+
+size_t sweep_work_bytes(int64_t N, const TcSweep &w) {
+    return 16 * (((size_t)w.ctas + 1) / 2 * 2) + sizeof(TcItem) * (size_t)w.ctas * sweep_stride(N, w);
+}
+
+TcWork launch_sweep_work(int64_t N, const TcSweep &w, void *workspace, cudaStream_t s) {
+    TcWork work;
+    work.ctas = w.ctas;
+    int64_t *begin = (int64_t *)workspace, *end = begin + (w.ctas + 1) / 2 * 2;
+    TcItem *items = (TcItem *)(end + (w.ctas + 1) / 2 * 2);
+    NCVIS_LAUNCH(sweep_items, (unsigned)w.ctas, 32, 0, s, N, w, sweep_stride(N, w), begin, end,
+                 items);
+    work.begin = begin;
+    work.end = end;
+    work.items = items;
+    return work;
 }
 
 bool knn_tc_supported(int D, int R) { return D >= 1 && D <= 64 * kMaxAtoms && (R == 32 || R == 64); }
@@ -646,12 +796,15 @@ bool knn_tc_supported(int D, int R) { return D >= 1 && D <= 64 * kMaxAtoms && (R
 
 namespace {
 
-void encode_rows(const __nv_bfloat16 *base, int64_t rows, int ldb, CUtensorMap &map) {
+void encode_rows(const void *base, int64_t rows, int ldb, bool half, CUtensorMap &map) {
     cuuint64_t dims[2] = {(cuuint64_t)ldb, (cuuint64_t)rows};
     cuuint64_t strides[1] = {(cuuint64_t)ldb * 2};
     cuuint32_t box[2] = {64, 128};
     cuuint32_t estr[2] = {1, 1};
-    CUresult r = tensor_map_encoder()(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (void *)base,
+    CUresult r = tensor_map_encoder()(&map,
+                                      half ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
+                                           : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16,
+                                      2, (void *)base,
                                       dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                                       CU_TENSOR_MAP_SWIZZLE_128B,
                                       CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -660,32 +813,31 @@ void encode_rows(const __nv_bfloat16 *base, int64_t rows, int ldb, CUtensorMap &
             "knn: cuTensorMapEncodeTiled failed (" + std::to_string((int)r) + ")", kCudaError);
 }
 
-void launch_select(const CUtensorMap &map, const CUtensorMap &map_c, const float *sqnorm,
-                   int64_t N, const KnnTcPlan &plan, bool ip, int32_t *cand_i, int *timeout_flag,
-                   cudaStream_t s, const TcWork *work) {
+void launch_select(const CUtensorMap &map, const CUtensorMap &map_c, const TcParts &parts,
+                   const float *sqnorm, const KnnTcPlan &plan, bool ip, int32_t *cand_i,
+                   int *timeout_flag, cudaStream_t s, const TcWork &work) {
     const int ksteps = (plan.ldb + 15) / 16;
     const int katoms = (ksteps * 16 + 63) / 64;
-    const size_t smem = sizeof(SharedStorage) + 1024;
-    const int64_t n_qt = (N + kQueryTile - 1) / kQueryTile;
-    const unsigned grid =
-        work ? (unsigned)work->ctas : (unsigned)std::min<int64_t>(n_qt, num_sms());
-    const int64_t *work_begin = work ? work->begin : nullptr;
-    const TcItem *items = work ? work->items : nullptr;
-    const int32_t *row_map = work ? work->map : nullptr;
+    const unsigned grid = (unsigned)work.ctas;
     if (grid == 0) return;
-    auto go = [&](auto kernel) {
+    auto go = [&](auto kernel, size_t shared) {
+        const size_t smem = shared + 1024;
         NCVIS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         (int)smem));
-        NCVIS_LAUNCH(kernel, grid, kThreads, smem, s, map, map_c, sqnorm, N, ksteps, katoms,
-                     work_begin, items, row_map, cand_i, timeout_flag,
+        NCVIS_LAUNCH(kernel, grid, kThreads, smem, s, map, map_c, parts, sqnorm, ksteps, katoms,
+                     work.begin, work.end, work.items, work.map, cand_i, work.lists.extra,
+                     work.lists.row0, work.lists.count, timeout_flag,
                      plan.wait_cycles > 0 ? plan.wait_cycles : kWaitCycles, plan.stall ? 1 : 0);
     };
-    if (plan.R == 8)
-        ip ? go(knn_select_tc<8, true>) : go(knn_select_tc<8, false>);
+    constexpr size_t one = sizeof(SharedStorage<1>), two = sizeof(SharedStorage<2>);
+    if (plan.parts == 2)
+        plan.R == 32 ? go(knn_select_tc<32, true, 2>, two) : go(knn_select_tc<64, true, 2>, two);
+    else if (plan.R == 8)
+        ip ? go(knn_select_tc<8, true, 1>, one) : go(knn_select_tc<8, false, 1>, one);
     else if (plan.R == 32)
-        ip ? go(knn_select_tc<32, true>) : go(knn_select_tc<32, false>);
+        ip ? go(knn_select_tc<32, true, 1>, one) : go(knn_select_tc<32, false, 1>, one);
     else
-        ip ? go(knn_select_tc<64, true>) : go(knn_select_tc<64, false>);
+        ip ? go(knn_select_tc<64, true, 1>, one) : go(knn_select_tc<64, false, 1>, one);
 }
 
 void check_plan(const KnnTcPlan &plan) {
@@ -699,9 +851,8 @@ void check_plan(const KnnTcPlan &plan) {
 }  // namespace
 
 void launch_knn_select_tc(const __nv_bfloat16 *Xb, const float *sqnorm, int64_t N,
-                          const KnnTcPlan &plan, int dist, int32_t *cand_i, float * /*cand_d*/,
-                          int *timeout_flag, cudaStream_t s, const TcWork *work,
-                          const __nv_bfloat16 *Xc) {
+                          const KnnTcPlan &plan, int dist, int32_t *cand_i, int *timeout_flag,
+                          cudaStream_t s, const TcWork &work, const __nv_bfloat16 *Xc) {
     require(N < (int64_t(1) << 31), "knn: N must be below 2^31");
     check_plan(plan);
     require(((uintptr_t)Xb & 15) == 0, "knn: BF16 rows must be 16-byte aligned");
@@ -710,11 +861,27 @@ void launch_knn_select_tc(const __nv_bfloat16 *Xb, const float *sqnorm, int64_t 
             "knn: the folded squared-L2 mode needs a 16-byte aligned candidate copy");
     // Queries come from Xb, candidates from Xc in the folded mode (else Xb).
     CUtensorMap map, map_c;
-    encode_rows(Xb, N, plan.ldb, map);
-    encode_rows(plan.fold ? Xc : Xb, N, plan.ldb, map_c);
+    encode_rows(Xb, N, plan.ldb, false, map);
+    encode_rows(plan.fold ? Xc : Xb, N, plan.ldb, false, map_c);
     // The folded squared-L2 product <q, c> - |c|^2 / 2 ranks like an inner product.
     const bool ip = dist != kSquaredL2 || plan.fold;
-    launch_select(map, map_c, sqnorm, N, plan, ip, cand_i, timeout_flag, s, work);
+    launch_select(map, map_c, TcParts{}, sqnorm, plan, ip, cand_i, timeout_flag, s, work);
+}
+
+void launch_knn_select_split(const __half *rows, int64_t N, const KnnTcPlan &plan,
+                             int32_t *cand_i, int *timeout_flag, cudaStream_t s,
+                             const TcWork &work) {
+    require(plan.parts == 2 && N < (int64_t(1) << 30), "knn: N must be below 2^30");
+    check_plan(plan);
+    require(((uintptr_t)rows & 15) == 0, "knn: FP16 rows must be 16-byte aligned");
+    // Blocks of N rows: the high parts, the low parts and, folded, the
+    // candidates' high parts; the candidates' map starts at the low parts then.
+    const int32_t n = (int32_t)N;
+    CUtensorMap map, map_c;
+    encode_rows(rows, 2 * N, plan.ldb, true, map);
+    encode_rows(plan.fold ? rows + (size_t)N * plan.ldb : rows, 2 * N, plan.ldb, true, map_c);
+    const TcParts parts = plan.fold ? TcParts{{0, n}, {n, 0}} : TcParts{{0, n}, {0, n}};
+    launch_select(map, map_c, parts, nullptr, plan, true, cand_i, timeout_flag, s, work);
 }
 
 void launch_knn_select_tc_pair(const __nv_bfloat16 *Q, int64_t nq, const __nv_bfloat16 *Cm,
@@ -727,9 +894,9 @@ void launch_knn_select_tc_pair(const __nv_bfloat16 *Q, int64_t nq, const __nv_bf
     require(ip || (c_sqnorm && ((uintptr_t)c_sqnorm & 15) == 0),
             "knn: squared L2 without folded norms needs 16-byte aligned candidate norms");
     CUtensorMap map, map_c;
-    encode_rows(Q, nq, plan.ldb, map);
-    encode_rows(Cm, nc, plan.ldb, map_c);
-    launch_select(map, map_c, c_sqnorm, nq, plan, ip, cand_i, timeout_flag, s, &work);
+    encode_rows(Q, nq, plan.ldb, false, map);
+    encode_rows(Cm, nc, plan.ldb, false, map_c);
+    launch_select(map, map_c, TcParts{}, c_sqnorm, plan, ip, cand_i, timeout_flag, s, work);
 }
 
 }  // namespace ncvis_gpu

@@ -4,6 +4,9 @@
 // copy.  One warp per row; the squared norm of the result (for the
 // |x|^2 + |y|^2 - 2<x,y> form of squared L2) and the zero-padded BF16
 // copies for the tensor-core kNN are produced in the same pass.
+#include <cmath>
+#include <cstring>
+
 #include "common.cuh"
 #include "stages.cuh"
 
@@ -22,7 +25,8 @@ __global__ void __launch_bounds__(256) preprocess_rows(const float *__restrict__
                                                        float *__restrict__ sqnorm,
                                                        __nv_bfloat16 *__restrict__ Xb,
                                                        __nv_bfloat16 *__restrict__ Xc, int ldb,
-                                                       int *__restrict__ bad_flag) {
+                                                       int *__restrict__ bad_flag,
+                                                       uint32_t *__restrict__ norms) {
     const int lane = threadIdx.x & 31;
     const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (row >= N) return;
@@ -67,6 +71,13 @@ __global__ void __launch_bounds__(256) preprocess_rows(const float *__restrict__
     sq_out = warp_sum(sq_out);
     if (lane == 0) {
         sqnorm[row] = sq_out;
+        if (norms) {
+            // Most rows find both words past their norm already: a read, no atomic.
+            const uint32_t bits = __float_as_uint(sq_out);
+            if (bits > __ldcg(norms)) atomicMax(norms, bits);
+            if (bits != 0u && bits <= kInfBits && kInfBits - bits > __ldcg(norms + 1))
+                atomicMax(norms + 1, kInfBits - bits);
+        }
         if (Xc) {
             const float h = -0.5f * sq_out;
             const __nv_bfloat16 hi = __float2bfloat16_rn(h);
@@ -80,14 +91,103 @@ __global__ void __launch_bounds__(256) preprocess_rows(const float *__restrict__
     if (!__all_sync(0xffffffffu, finite) && lane == 0) atomicOr(bad_flag, 1);
 }
 
+// FP16 parts of s * x for the FP32 search on the tensor cores: 8 columns of one
+// row per thread, 16-byte stores.  hi is s x rounded to 11 bits; s x - hi is
+// exact in FP32 and its 11 bits are lo, so hi + lo holds s x to at most one unit
+// in FP32's last place.  The tensor cores' FP32 accumulator truncates: a product
+// loses about 0.6 units in its 24th place per 16 columns (measured: 0.36 on unit
+// rows to 0.85 on rows far from the origin), which lo makes up for on both sides
+// (`lift` = half of that, relative).  Squared L2 (fold): w = -|s c|^2 / 2 goes into three
+// columns, w = 2^14 a + 2^3 b + 2^-8 c with a, b, c in FP16, each part's
+// remainder exact; the powers keep all three within FP16's normal range for
+// norms from 2^1 to 2^14.
+__global__ void __launch_bounds__(256) split_rows(
+    const float *__restrict__ Xp, const float *__restrict__ sqnorm, int64_t N, int D, int ldb,
+    float scale, float lift, bool fold, __half *__restrict__ hi, __half *__restrict__ lo,
+    __half *__restrict__ cand, const int64_t *__restrict__ off, const int64_t *__restrict__ pad,
+    int B) {
+    const int per = ldb >> 3;
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= N * per) return;
+    const int64_t row = t / per;
+    const int c0 = (int)(t - row * per) * 8;
+    int64_t to = row;
+    if (off) {
+        const int p = segment_of(off, B, row);
+        to = pad[p] + (row - off[p]);
+    }
+    const float *x = Xp + row * D;
+    float v[8];
+    if ((D & 3) == 0 && c0 + 8 <= D) {
+        const float4 a = __ldg(reinterpret_cast<const float4 *>(x + c0));
+        const float4 b = __ldg(reinterpret_cast<const float4 *>(x + c0 + 4));
+        v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w;
+        v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+    } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = c0 + j < D ? __ldg(x + c0 + j) : 0.f;
+    }
+    __align__(16) __half h[8], l[8], c[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const float y = v[j] * scale;
+        h[j] = __float2half_rn(y);
+        l[j] = __float2half_rn(fmaf(y, lift, y - __half2float(h[j])));
+        c[j] = h[j];
+    }
+    if (fold && c0 + 8 > D) {
+        const float w = -0.5f * sqnorm[row] * scale * scale;
+        const __half a = __float2half_rn(w * 0x1p-14f);
+        const float r1 = w - __half2float(a) * 0x1p14f;
+        const __half b = __float2half_rn(r1 * 0x1p-3f);
+        const float r2 = r1 - __half2float(b) * 0x1p3f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            if (c0 + j == D) c[j] = a, h[j] = __float2half_rn(0x1p14f);
+            if (c0 + j == D + 1) c[j] = b, h[j] = __float2half_rn(0x1p3f);
+            if (c0 + j == D + 2) c[j] = __float2half_rn(r2 * 0x1p8f), h[j] = __float2half_rn(0x1p-8f);
+        }
+    }
+    const int64_t o = to * ldb + c0;
+    *reinterpret_cast<uint4 *>(hi + o) = *reinterpret_cast<const uint4 *>(h);
+    *reinterpret_cast<uint4 *>(lo + o) = *reinterpret_cast<const uint4 *>(l);
+    if (fold) *reinterpret_cast<uint4 *>(cand + o) = *reinterpret_cast<const uint4 *>(c);
+}
+
 }  // namespace
+
+float split_scale(const uint32_t norms[2], int dist) {
+    // Unit rows (and rows of zeros).
+    if (dist == kCosine || dist == kCorrelation) return 0x1p14f;
+    if (norms[0] == 0u) return 1.f;
+    if (norms[0] >= kInfBits) return 0.f;
+    const uint32_t low_bits = kInfBits - norms[1];
+    float top, low;
+    std::memcpy(&top, &norms[0], 4);
+    std::memcpy(&low, &low_bits, 4);
+    // Squared norms must keep their own precision in FP32.
+    if (low < 0x1p-100f || top > 0x1p100f) return 0.f;
+    const int e = std::ilogb(std::sqrt(top)) + 1;  // norms < 2^e (1 + rounding)
+    const float scale = std::ldexp(1.f, 14 - e);
+    return std::sqrt(low) * scale >= 2.f ? scale : 0.f;
+}
+
+void launch_split_rows(const float *Xp, const float *sqnorm, int64_t N, int D, float scale,
+                       const KnnTcPlan &plan, __half *rows, int64_t rows_per_part, cudaStream_t s,
+                       const int64_t *off, const int64_t *pad, int B) {
+    const size_t part = (size_t)rows_per_part * plan.ldb;
+    const float lift = 0.5f * 0.6f * (float)D / 16.f * 0x1p-24f;
+    NCVIS_LAUNCH(split_rows, ceil_div((size_t)N * (plan.ldb / 8), 256), 256, 0, s, Xp, sqnorm, N, D,
+                 plan.ldb, scale, lift, plan.fold, rows, rows + part,
+                 plan.fold ? rows + 2 * part : nullptr, off, pad, B);
+}
 
 void launch_preprocess(const float *X, int64_t N, int D, int dist, float *Xp, float *sqnorm,
                        __nv_bfloat16 *Xb, int ldb, int *bad_flag, cudaStream_t s,
-                       __nv_bfloat16 *Xc) {
+                       __nv_bfloat16 *Xc, uint32_t *norms) {
     const int warps_per_block = 8;
     NCVIS_LAUNCH(preprocess_rows, ceil_div(N, warps_per_block), 32 * warps_per_block, 0, s, X, N,
-                 D, dist, Xp, sqnorm, Xb, Xc, ldb, bad_flag);
+                 D, dist, Xp, sqnorm, Xb, Xc, ldb, bad_flag, norms);
 }
 
 }  // namespace ncvis_gpu

@@ -3,6 +3,7 @@
 #pragma once
 
 #include <cuda_bf16.h>
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
 #include <cstddef>
@@ -18,9 +19,12 @@ enum Distance { kSquaredL2 = 0, kInnerProduct = 1, kCosine = 2, kCorrelation = 3
 // is set to 1 if any input is not finite.
 // Xc (optional, squared L2 on the tensor cores): candidate copy whose columns
 // D, D + 1 hold -|x|^2 / 2 as BF16 high + low parts; Xb then holds 1, 1 there.
+// norms (optional, two device words that start at 0): the bits of the largest
+// |xp|^2, and kInfBits minus the bits of the smallest that is not 0.
+constexpr uint32_t kInfBits = 0x7f800000u;
 void launch_preprocess(const float *X, int64_t N, int D, int dist, float *Xp, float *sqnorm,
                        __nv_bfloat16 *Xb, int ldb, int *bad_flag, cudaStream_t s,
-                       __nv_bfloat16 *Xc = nullptr);
+                       __nv_bfloat16 *Xc = nullptr, uint32_t *norms = nullptr);
 
 // Independent problems packed in one point array: problem p owns rows
 // [offsets[p], offsets[p+1]) (device arrays).  B == 0: one problem, all rows.
@@ -38,25 +42,35 @@ struct KnnPlan {
     int C() const { return R * splits; }
 };
 KnnPlan plan_knn_f32(int64_t N, int k, int rerank_factor);
-// cand_i/cand_d: [N, plan.C()]; -1 marks an empty slot.
+// cand_i: [N, plan.C()]; -1 marks an empty slot.
 void launch_knn_select_f32(const float *Xp, const float *sqnorm, int64_t N, int D, int dist,
-                           const KnnPlan &plan, int32_t *cand_i, float *cand_d, cudaStream_t s,
+                           const KnnPlan &plan, int32_t *cand_i, cudaStream_t s,
                            const Segments &seg = Segments());
 int knn_f32_query_tile();
+// Lists beyond a row's first one, where several items of a tensor-core launch
+// share a query tile: rows (in the launch's numbering) from row0 on have
+// `count` more lists at extra[(row - row0) * count * R], R candidates each; -1
+// marks an empty slot.
+struct TcLists {
+    int32_t *extra = nullptr;
+    int64_t row0 = 0;
+    int count = 0;
+};
 // Exact distances of the candidates, top k+1 by (distance, index), smallest
 // dropped, k written in descending order: inds/dists [N, k].  `order` (a
 // permutation of the rows, or nullptr) is the order the rows are processed
-// in; the result does not depend on it.
+// in; the result does not depend on it.  `lists`: further lists of C
+// candidates of the rows from lists.row0 on (in that order).
 void launch_rerank(const float *Xp, int64_t N, int D, int dist, const int32_t *cand_i, int C,
                    int k, int32_t *inds, float *dists, cudaStream_t s,
-                   const int32_t *order = nullptr);
+                   const int32_t *order = nullptr, const TcLists &lists = TcLists());
 
 // ---- K2 BF16 tensor-core candidate selection ---------------------------------
 struct KnnTcPlan {
     int R;       // candidates kept per point (multiple of 4 is not required)
-    int ldb;     // padded row length of Xb (bf16 elements)
+    int ldb;     // padded row length of Xb (16-bit elements)
     bool fold;   // squared L2 with the norms folded into the product (needs Xc)
-    int64_t Npad;
+    int parts = 1;  // 1: BF16 rows; 2: FP16 high and low parts (the FP32 search)
     // Diagnostics: limit of the kernel's waits between its roles in SM cycles
     // (<= 0: about 2 s), and a stall on a barrier nothing completes (the
     // timeout path's test).
@@ -76,19 +90,53 @@ constexpr int kTcContinue = 1;
 constexpr int kTcMore = 2;
 struct alignas(16) TcItem {
     int32_t row0, qend, lo, hi;
-    int32_t out_off, flags, pad0, pad1;
+    int32_t out_off, flags;
+    int32_t slot;  // which of the query tile's lists the item writes (TcLists)
+    int32_t pad;
 };
-// Work of one launch (device arrays): CTA b takes items[begin[b] .. begin[b+1]).
+// Work of one launch (device arrays): CTA b takes items[begin[b] .. end[b]).
 struct TcWork {
-    int ctas;
-    const int64_t *begin;
-    const TcItem *items;
-    const int32_t *map;  // optional row map (sorted row -> output row), or null
+    int ctas = 0;
+    const int64_t *begin = nullptr, *end = nullptr;
+    const TcItem *items = nullptr;
+    const int32_t *map = nullptr;  // optional row map (sorted row -> output row)
+    TcLists lists;
 };
+// How the query tiles of one problem of N rows are spread over at most `ctas`
+// CTAs: the first full_qt whole and round-robin, the rest in equal runs of
+// candidate tiles over the first rest_ctas, so that the last wave fills the
+// GPU; rows of the last `split_rows` have up to `lists` lists.
+struct TcSweep {
+    int64_t full_qt = 0, split_rows = 0;
+    int ctas = 0, rest_ctas = 1, lists = 1;
+};
+TcSweep plan_sweep(int64_t N, int ctas);
+TcSweep whole_tiles(int64_t N, int ctas);  // every query tile whole
+// Its work list, written by a kernel into `workspace` (16-byte aligned).
+size_t sweep_work_bytes(int64_t N, const TcSweep &w);
+TcWork launch_sweep_work(int64_t N, const TcSweep &w, void *workspace, cudaStream_t s);
 void launch_knn_select_tc(const __nv_bfloat16 *Xb, const float *sqnorm, int64_t N,
-                          const KnnTcPlan &plan, int dist, int32_t *cand_i, float *cand_d,
-                          int *timeout_flag, cudaStream_t s, const TcWork *work = nullptr,
-                          const __nv_bfloat16 *Xc = nullptr);
+                          const KnnTcPlan &plan, int dist, int32_t *cand_i, int *timeout_flag,
+                          cudaStream_t s, const TcWork &work, const __nv_bfloat16 *Xc = nullptr);
+
+// ---- FP32 candidate selection on the tensor cores -----------------------------
+// Rows as FP16 high and low parts of s * x, s a power of two: rows[0, N) the
+// high parts, [N, 2N) the low parts and, for squared L2 (plan.fold),
+// [2N, 3N) the high parts of the candidates, whose columns D .. D + 2 hold
+// -|c|^2 / 2 in three parts (ldb elements a row); rows_per_part may exceed N.
+// split_scale: the s for the rows' norms (the words of launch_preprocess), 0
+// where no s serves them all: hi + lo holds s x to one unit in FP32's last
+// place only while |s x| >= 2^-3, so every row's norm must stay within 2^13 of
+// the largest (and that be finite).
+float split_scale(const uint32_t norms[2], int dist);
+KnnTcPlan plan_knn_split(int D, int R, int dist);
+bool knn_split_supported(int64_t N, int D, int R, int dist);
+void launch_split_rows(const float *Xp, const float *sqnorm, int64_t N, int D, float scale,
+                       const KnnTcPlan &plan, __half *rows, int64_t rows_per_part, cudaStream_t s,
+                       const int64_t *off = nullptr, const int64_t *pad = nullptr, int B = 0);
+void launch_knn_select_split(const __half *rows, int64_t N, const KnnTcPlan &plan,
+                             int32_t *cand_i, int *timeout_flag, cudaStream_t s,
+                             const TcWork &work);
 // Approximate candidate selection (inverted file): C cells from k-means on
 // the BF16 rows, each cell searched against its `probe` nearest cells.
 struct IvfPlan {
