@@ -258,21 +258,20 @@ __device__ __forceinline__ float tree_reduce(const float (&a)[n]) {
 }
 
 // Insert (v, vi) into the ascending list (ls, li) of R entries, dropping the
-// largest: one compare-exchange per slot, indices follow their scores.
+// largest.  Every slot's new entry comes from the old ones alone (its own, its
+// left neighbour's or the new value, by two compares), so the R slots are
+// independent: passing the displaced entry on from slot to slot instead is a
+// chain of R dependent compares, which cost the sweeps 6% (131,072 x 100) to 30%
+// (65,536 x 50 with 64 entries).
 template <int R>
 __device__ __forceinline__ void list_push(float (&ls)[R], int32_t (&li)[R], float v, int32_t vi) {
 #pragma unroll
-    for (int t = 0; t < R; ++t) {
-        const bool lt = v < ls[t];
-        const float a = lt ? v : ls[t];
-        const int32_t ai = lt ? vi : li[t];
-        const float b = lt ? ls[t] : v;
-        const int32_t bi = lt ? li[t] : vi;
-        ls[t] = a;
-        li[t] = ai;
-        v = b;
-        vi = bi;
+    for (int t = R - 1; t > 0; --t) {
+        const bool here = v < ls[t], left = v < ls[t - 1];
+        li[t] = here ? (left ? li[t - 1] : vi) : li[t];
+        ls[t] = fminf(fmaxf(ls[t - 1], v), ls[t]);
     }
+    if (v < ls[0]) ls[0] = v, li[0] = vi;
 }
 
 // Every queued candidate of the warp's rows goes into its row's list, in
