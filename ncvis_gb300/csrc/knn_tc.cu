@@ -625,25 +625,36 @@ __global__ void __launch_bounds__(kThreads, 1)
                     const float best = tree_reduce<false, kG>(gb);
                     const bool hit = live && best < worst;
                     if (!__any_sync(0xffffffffu, hit)) continue;
-                    // Qualifying candidates are queued kAppend columns at a time,
-                    // looking only into the 8-column groups whose best beats
-                    // the row's worst; a queue past half full is flushed into
-                    // the lists first.
-#pragma unroll
-                    for (int part = 0; part < kC / kAppend; ++part) {
-                        if (__any_sync(0xffffffffu, qlen > kQueue - kAppend))
-                            flush_queue<R>(ls, li, worst, qlen, s.queue_v, s.queue_i, etid);
+                    if constexpr (R == 1) {
+                        // The best alone: its column is looked for when it wins.
                         if (hit) {
+                            const float raw = kIP ? -best : best;
 #pragma unroll
-                            for (int g = part * kAppend / 8; g < (part + 1) * kAppend / 8; ++g) {
-                                if (gb[g] < worst) {
+                            for (int j = kC - 1; j >= 0; --j)
+                                if (v[j] == raw) li[0] = (int32_t)(cb + j);
+                            ls[0] = worst = best;
+                        }
+                    } else {
+                        // Qualifying candidates are queued kAppend columns at a time,
+                        // looking only into the 8-column groups whose best beats
+                        // the row's worst; a queue past half full is flushed into
+                        // the lists first.
 #pragma unroll
-                                    for (int j = 8 * g; j < 8 * g + 8; ++j) {
-                                        const float x = kIP ? -v[j] : v[j];
-                                        if (x < worst) {
-                                            s.queue_v[qlen][etid] = x;
-                                            s.queue_i[qlen][etid] = (int32_t)(cb + j);
-                                            ++qlen;
+                        for (int part = 0; part < kC / kAppend; ++part) {
+                            if (__any_sync(0xffffffffu, qlen > kQueue - kAppend))
+                                flush_queue<R>(ls, li, worst, qlen, s.queue_v, s.queue_i, etid);
+                            if (hit) {
+#pragma unroll
+                                for (int g = part * kAppend / 8; g < (part + 1) * kAppend / 8; ++g) {
+                                    if (gb[g] < worst) {
+#pragma unroll
+                                        for (int j = 8 * g; j < 8 * g + 8; ++j) {
+                                            const float x = kIP ? -v[j] : v[j];
+                                            if (x < worst) {
+                                                s.queue_v[qlen][etid] = x;
+                                                s.queue_i[qlen][etid] = (int32_t)(cb + j);
+                                                ++qlen;
+                                            }
                                         }
                                     }
                                 }
@@ -831,8 +842,8 @@ void launch_select(const CUtensorMap &map, const CUtensorMap &map_c, const TcPar
     constexpr size_t one = sizeof(SharedStorage<1>), two = sizeof(SharedStorage<2>);
     if (plan.parts == 2)
         plan.R == 32 ? go(knn_select_tc<32, true, 2>, two) : go(knn_select_tc<64, true, 2>, two);
-    else if (plan.R == 8)
-        ip ? go(knn_select_tc<8, true, 1>, one) : go(knn_select_tc<8, false, 1>, one);
+    else if (plan.R == 1)
+        go(knn_select_tc<1, true, 1>, one);
     else if (plan.R == 32)
         ip ? go(knn_select_tc<32, true, 1>, one) : go(knn_select_tc<32, false, 1>, one);
     else
@@ -843,8 +854,8 @@ void check_plan(const KnnTcPlan &plan) {
     const int ksteps = (plan.ldb + 15) / 16;
     const int katoms = (ksteps * 16 + 63) / 64;
     require(katoms <= kMaxAtoms, "knn: the tensor-core path supports D <= 128", kUnsupported);
-    require(plan.R == 8 || plan.R == 32 || plan.R == 64,
-            "knn: the tensor-core kernel keeps 8, 32 or 64 candidates");
+    require(plan.R == 1 || plan.R == 32 || plan.R == 64,
+            "knn: the tensor-core kernel keeps 1, 32 or 64 candidates");
 }
 
 }  // namespace
