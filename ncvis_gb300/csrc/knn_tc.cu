@@ -17,9 +17,10 @@
 //     32-column chunks, turn dot products into ranking scores (-<q,c> for the
 //     inner-product spaces, |c|^2 - 2<q,c> for squared L2), reduce each chunk
 //     with 3-input min/max trees and compare its best with the row's worst;
-//     qualifying candidates go to a per-row queue in shared memory, which the
-//     warp inserts into the rows' register-resident sorted lists in lockstep
-//     rounds (R compare-exchanges each) when a queue passes half full;
+//     a group of 4 columns that holds a qualifying candidate goes whole to a
+//     per-row queue in shared memory; when a queue is full the warp looks all its
+//     rows' queues over and inserts what qualifies into the rows'
+//     register-resident sorted lists in lockstep rounds;
 //   * a CTA takes items from its own work list: an item is a query tile's rows
 //     and one candidate range (masked at both ends), and may continue the
 //     previous item's tile, so one tile's lists are built over several ranges
@@ -72,20 +73,28 @@ constexpr uint32_t kTmemCols = 512;
 constexpr int kLowLowSteps = 2;  // K steps up to which the low parts' product is taken too
 constexpr long long kWaitCycles = 4000000000LL;  // ~2 s at 2 GHz
 
+// One queued group of 4 accumulator columns of every row: the values and the
+// candidate index of the first column.
+constexpr int kGroup = 4;
+constexpr uint32_t kFlushAt = 4;  // slots past which a queue is flushed after a tile
+struct QueueSlot {
+    float4 v[kEpiThreads];
+    int32_t first[kEpiThreads];
+};
+
 // Shared memory by the number of parts a row is held in: the query tile takes
-// 64 KB a part, so the two-part form has a ring of 2 stages and 16 queue slots
-// per row where the one-part form has 3 and 32 (both 224 KB in all).  Stages of
+// 64 KB a part, so the two-part form has a ring of 2 stages and 6 queue slots
+// per row where the one-part form has 3 and 12 (both 224 KB in all).  Stages of
 // 64 columns (half a part, twice as many) made the BF16 sweep of 1,024,000 x 100
 // 18% slower: the MMA warps then wait within a tile too.
 template <int kParts>
 struct SharedStorage {
     static constexpr int kStages = kParts == 1 ? 3 : 2;  // candidate ring (32 KB each)
-    static constexpr int kQueue = kParts == 1 ? 32 : 16;  // per-row insertion queue slots
+    static constexpr int kQueue = kParts == 1 ? 12 : 6;  // column groups queued per row
     // 1024-byte aligned tiles first (128B swizzle atoms repeat every 1024 B).
     uint8_t a[2][kParts][kMaxAtoms][kAtomBytes];
     uint8_t b[kStages][kMaxAtoms][kAtomBytes];
-    float queue_v[kQueue][kEpiThreads];    // queued candidate scores, [slot][thread]
-    int32_t queue_i[kQueue][kEpiThreads];  // and their candidate indices
+    QueueSlot queue[kQueue];
     uint64_t full[kStages];
     uint64_t empty[kStages];
     uint64_t a_full, a_empty;
@@ -274,24 +283,72 @@ __device__ __forceinline__ void list_push(float (&ls)[R], int32_t (&li)[R], floa
     if (v < ls[0]) ls[0] = v, li[0] = vi;
 }
 
-// Every queued candidate of the warp's rows goes into its row's list, in
-// lockstep rounds (one per slot of the fullest queue); queues end empty.
-template <int R>
+// Queues the 4 columns v[0..4) of a row, the first being candidate `first`, when
+// their best score gb is below the row's worst: `off` is the byte offset of the
+// row's next slot, and moves on; the columns are stored where it lies within the
+// queue (predicated stores, no branch).
+__device__ __forceinline__ void queue_group(uint32_t queue_v, uint32_t queue_i, uint32_t &off,
+                                            uint32_t bytes, float gb, float worst, const float *v,
+                                            int32_t first) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t.reg .u32 a, b;\n\t"
+        "setp.lt.f32 p, %1, %2;\n\t"
+        "setp.lt.and.u32 q, %0, %11, p;\n\t"
+        "add.u32 a, %3, %0;\n\t"
+        "add.u32 b, %4, %0;\n\t"
+        "@q st.shared.v4.f32 [a], {%5, %6, %7, %8};\n\t"
+        "@q st.shared.s32 [b], %9;\n\t"
+        "@p add.u32 %0, %0, %10;\n\t}"
+        : "+r"(off)
+        : "f"(gb), "f"(worst), "r"(queue_v), "r"(queue_i), "f"(v[0]), "f"(v[1]), "f"(v[2]),
+          "f"(v[3]), "r"(first), "n"(sizeof(QueueSlot)), "r"(bytes)
+        : "memory");
+}
+
+// Every queued candidate of the warp's rows that still beats its row's worst
+// goes into its row's list; queues end empty.  Each lane first marks its
+// qualifying values (a bit per queued column), then the warp inserts in lockstep
+// rounds, one marked value per row a round, so that a round serves every row
+// that has one left.
+template <int R, bool kIP, int kQueue>
 __device__ __forceinline__ void flush_queue(float (&ls)[R], int32_t (&li)[R], float &worst,
-                                            int &qlen, const float (*queue_v)[kEpiThreads],
-                                            const int32_t (*queue_i)[kEpiThreads], int etid) {
-    const int rounds = __reduce_max_sync(0xffffffffu, qlen);
+                                            uint32_t &off, const QueueSlot *queue, int etid) {
+    constexpr uint32_t kSlot = sizeof(QueueSlot);
+    const uint32_t most = __reduce_max_sync(0xffffffffu, off);
+    uint32_t marks[2] = {0u, 0u};  // slot b's columns: bits 4 (b % 8) .. of marks[b / 8]
+#pragma unroll
+    for (int b = 0; b < kQueue; ++b) {
+        if (b * kSlot >= most) break;
+        if (b * kSlot < off) {
+            const float4 x = queue[b].v[etid];
+            const float w[kGroup] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+            for (int j = 0; j < kGroup; ++j)
+                if ((kIP ? -w[j] : w[j]) < worst) marks[b >> 3] |= 1u << (4 * (b & 7) + j);
+        }
+    }
 #pragma unroll 1
-    for (int t = 0; t < rounds; ++t) {
-        if (t < qlen) {
-            const float x = queue_v[t][etid];
+    while (__any_sync(0xffffffffu, (marks[0] | marks[1]) != 0u)) {
+        if ((marks[0] | marks[1]) != 0u) {
+            int pos;
+            if (marks[0] != 0u) {
+                pos = __ffs(marks[0]) - 1;
+                marks[0] &= marks[0] - 1u;
+            } else {
+                pos = 31 + __ffs(marks[1]);
+                marks[1] &= marks[1] - 1u;
+            }
+            const QueueSlot &slot = queue[pos >> 2];
+            const int j = pos & 3;
+            const float raw = reinterpret_cast<const float *>(&slot.v[etid])[j];
+            const float x = kIP ? -raw : raw;
             if (x < worst) {
-                list_push<R>(ls, li, x, queue_i[t][etid]);
+                list_push<R>(ls, li, x, slot.first[etid] + j);
                 worst = ls[R - 1];
             }
         }
     }
-    qlen = 0;
+    off = 0u;
     __syncwarp();
 }
 
@@ -531,15 +588,19 @@ __global__ void __launch_bounds__(kThreads, 1)
         // Accumulator columns per tcgen05.ld: 32 with 32-entry lists; 64-entry
         // lists leave registers for 16.
         constexpr int kC = R <= 32 ? 32 : 16;
-        // Columns queued between two looks at the queue: half the queue, so
-        // that one that is at most half full takes them.
-        constexpr int kAppend = kQueue / 2;
+        constexpr int kG = kC / kGroup;  // column groups per load
+        constexpr uint32_t kQueueBytes = kQueue * sizeof(QueueSlot);
+        const uint32_t queue_v = smem_u32(&s.queue[0].v[etid]);
+        const uint32_t queue_i = smem_u32(&s.queue[0].first[etid]);
+        auto flush = [&](float (&ls)[R], int32_t (&li)[R], float &worst, uint32_t &off) {
+            flush_queue<R, kIP, kQueue>(ls, li, worst, off, s.queue, etid);
+        };
         uint32_t acc_phase = 0;
         int acc = 0;
         float ls[R];
         int32_t li[R];
         float worst = FLT_MAX;
-        int qlen = 0;
+        uint32_t qoff = 0u;
         for (int64_t it = 0; it < n_items; ++it) {
             // Lanes read the abort flag at different times: the warp stops as one.
             if (__any_sync(0xffffffffu, s.abort != 0)) break;
@@ -551,8 +612,9 @@ __global__ void __launch_bounds__(kThreads, 1)
                     ls[t] = FLT_MAX;
                     li[t] = -1;
                 }
-                worst = FLT_MAX;
-                qlen = 0;
+                // Nothing qualifies in rows that are not outputs.
+                worst = live ? FLT_MAX : -INFINITY;
+                qoff = 0u;
             }
             bool ok = true;
             for (int64_t ct = q.lo / kCandTile; ct * kCandTile < q.hi; ++ct) {
@@ -611,23 +673,19 @@ __global__ void __launch_bounds__(kThreads, 1)
                         for (int j = 0; j < kC; ++j)
                             if (cb + j < q.lo || cb + j >= q.hi) v[j] = kIP ? -FLT_MAX : FLT_MAX;
                     }
-                    // Best score of each 8-column group, then of the chunk.
-                    constexpr int kG = kC / 8;
+                    // Best score of each group of columns, then of the chunk.
                     float gb[kG];
 #pragma unroll
                     for (int g = 0; g < kG; ++g) {
-                        const float *w = v + 8 * g;
-                        gb[g] = kIP ? -max3f(max3f(w[0], w[1], w[2]), max3f(w[3], w[4], w[5]),
-                                             fmaxf(w[6], w[7]))
-                                    : min3f(min3f(w[0], w[1], w[2]), min3f(w[3], w[4], w[5]),
-                                            fminf(w[6], w[7]));
+                        const float *w = v + kGroup * g;
+                        gb[g] = kIP ? -fmaxf(max3f(w[0], w[1], w[2]), w[3])
+                                    : fminf(min3f(w[0], w[1], w[2]), w[3]);
                     }
                     const float best = tree_reduce<false, kG>(gb);
-                    const bool hit = live && best < worst;
-                    if (!__any_sync(0xffffffffu, hit)) continue;
+                    if (!__any_sync(0xffffffffu, best < worst)) continue;
                     if constexpr (R == 1) {
                         // The best alone: its column is looked for when it wins.
-                        if (hit) {
+                        if (best < worst) {
                             const float raw = kIP ? -best : best;
 #pragma unroll
                             for (int j = kC - 1; j >= 0; --j)
@@ -635,45 +693,42 @@ __global__ void __launch_bounds__(kThreads, 1)
                             ls[0] = worst = best;
                         }
                     } else {
-                        // Qualifying candidates are queued kAppend columns at a time,
-                        // looking only into the 8-column groups whose best beats
-                        // the row's worst; a queue past half full is flushed into
-                        // the lists first.
+                        // The groups whose best beats the row's worst are queued
+                        // whole: about 7 instructions a group, where looking at each
+                        // column of them here held the accumulator for longer.
+                        // When a row's groups run past the end of its queue the
+                        // queues are flushed and the groups gone over again: what
+                        // was stored now lies below offset 0 (and is not stored
+                        // again), what was not follows.
+                        const float before = worst;
+                        uint32_t start = qoff;
+                        for (;;) {
+                            qoff = start;
 #pragma unroll
-                        for (int part = 0; part < kC / kAppend; ++part) {
-                            if (__any_sync(0xffffffffu, qlen > kQueue - kAppend))
-                                flush_queue<R>(ls, li, worst, qlen, s.queue_v, s.queue_i, etid);
-                            if (hit) {
-#pragma unroll
-                                for (int g = part * kAppend / 8; g < (part + 1) * kAppend / 8; ++g) {
-                                    if (gb[g] < worst) {
-#pragma unroll
-                                        for (int j = 8 * g; j < 8 * g + 8; ++j) {
-                                            const float x = kIP ? -v[j] : v[j];
-                                            if (x < worst) {
-                                                s.queue_v[qlen][etid] = x;
-                                                s.queue_i[qlen][etid] = (int32_t)(cb + j);
-                                                ++qlen;
-                                            }
-                                        }
-                                    }
-                                }
-                            }
+                            for (int g = 0; g < kG; ++g)
+                                queue_group(queue_v, queue_i, qoff, kQueueBytes, gb[g], before,
+                                            v + kGroup * g, (int32_t)(cb + kGroup * g));
+                            if ((int32_t)qoff < 0) qoff = 0u;
+                            if (!__any_sync(0xffffffffu, qoff > kQueueBytes)) break;
+                            qoff = min(qoff, kQueueBytes);
+                            flush(ls, li, worst, qoff);
+                            start -= kQueueBytes;
                         }
                     }
                 }
                 acc ^= 1;
                 if (acc == 0) acc_phase ^= 1;
-                // Queues past half full are flushed here, after the accumulator
-                // is released, so that the MMAs of the next tiles go on meanwhile;
-                // a flush inside the tile happens only when one tile overfills a
-                // queue (early in the sweep).
-                if (__any_sync(0xffffffffu, qlen > kQueue - kAppend))
-                    flush_queue<R>(ls, li, worst, qlen, s.queue_v, s.queue_i, etid);
+                // Here, with the accumulator released, queues past kFlushAt slots
+                // are flushed.  Fewer slots insert for fewer rows a round, more
+                // hold the warp up for longer than the accumulators' two buffers
+                // cover: 131,072 x 100 BF16 6.54, 6.44, 6.45 and 6.53 ms with 1, 2, 4
+                // and 6, 60,013 x 100 FP32 2.59, 2.57, 2.54 and 2.65.
+                if (__any_sync(0xffffffffu, qoff > kFlushAt * sizeof(QueueSlot)))
+                    flush(ls, li, worst, qoff);
             }
             if (!ok) break;
             if (q.more) continue;  // the next item extends this query tile
-            flush_queue<R>(ls, li, worst, qlen, s.queue_v, s.queue_i, etid);
+            flush(ls, li, worst, qoff);
             // The item read again: where its lists go is not held in registers
             // over the sweep (the barrier keeps the two reads apart).
             int64_t again = it;
