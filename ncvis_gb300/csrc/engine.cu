@@ -1229,17 +1229,13 @@ int ncvis_init_embedding_device(size_t N, size_t d, const int64_t *d_row_ptr,
                 "init_embedding: need N >= 1, 1 <= d <= 32, n_init_epochs >= 0");
         cudaStream_t s = (cudaStream_t)stream;
         // The graph must be a CSR over N rows: offsets from 0, non-decreasing,
-        // columns in [0, N).
-        std::vector<int64_t> rp(N + 1);
-        NCVIS_CUDA(cudaMemcpyAsync(rp.data(), d_row_ptr, sizeof(int64_t) * (N + 1),
-                                   cudaMemcpyDeviceToHost, s));
-        NCVIS_CUDA(cudaStreamSynchronize(s));
-        require(rp[0] == 0, "init_embedding: row_ptr[0] must be 0");
-        for (size_t i = 0; i < N; ++i)
-            require(rp[i + 1] >= rp[i], "init_embedding: row_ptr must be non-decreasing");
-        require(rp[N] < (int64_t(1) << 31), "init_embedding: too many edges");
-        require(indices_in_range(d_cols, rp[N], (int64_t)N, s),
-                "init_embedding: a column index is outside [0, N)");
+        // columns in [0, N).  Checked on the device (copying 500,001 offsets to
+        // the host and going through them there took 6.3 of a call's 9.2 ms).
+        const int bad = check_graph((int64_t)N, d_row_ptr, d_cols, s);
+        require(!(bad & 1), "init_embedding: row_ptr[0] must be 0");
+        require(!(bad & 2), "init_embedding: row_ptr must be non-decreasing");
+        require(!(bad & 4), "init_embedding: too many edges");
+        require(!(bad & 8), "init_embedding: a column index is outside [0, N)");
         StreamBuffer ws(init_workspace_bytes((int64_t)N, (int)d), s);
         run_init_embedding((int64_t)N, (int)d, d_row_ptr, d_cols, seed, n_init_epochs, alpha, dY,
                            ws.p, s, sequential_stats != 0);

@@ -187,7 +187,12 @@ int64_t run_symmetrize(int64_t N, int k, const int32_t *inds, const float *dists
                        int64_t *row_ptr, int32_t *cols, float *vals, int32_t *src,
                        cudaStream_t s);
 
-// True when every a[0..n) lies in [0, N) (waits on the stream).
+// What is wrong with a CSR of N rows (waits on the stream): 0, or a sum of 1 (the
+// first offset is not 0), 2 (offsets decrease), 4 (2^31 edges or more) and 8 (a
+// column outside [0, N)); the columns are read only when the offsets are good.
+int check_graph(int64_t N, const int64_t *row_ptr, const int32_t *cols, cudaStream_t s);
+// True when every a[0..n), and b[0..n) unless it is null, lies in [0, N) (waits
+// on the stream).
 bool indices_in_range(const int32_t *a, int64_t n, int64_t N, cudaStream_t s);
 bool edges_in_range(const int32_t *a, const int32_t *b, int64_t n, int64_t N, cudaStream_t s);
 

@@ -70,6 +70,37 @@ __global__ void check_pairs(const int32_t *__restrict__ a, const int32_t *__rest
     }
 }
 
+// A CSR over N rows as a caller gives it: bit 0 of *bad when row_ptr[0] is not 0,
+// bit 1 when an offset is below the one before it, bit 2 when there are 2^31
+// edges or more.
+__global__ void check_offsets(const int64_t *__restrict__ row_ptr, int64_t N,
+                              int *__restrict__ bad) {
+    int found = 0;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i <= N;
+         i += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t at = row_ptr[i];
+        if (i == 0 && at != 0) found |= 1;
+        if (i > 0 && at < row_ptr[i - 1]) found |= 2;
+        if (i == N && at >= (int64_t(1) << 31)) found |= 4;
+    }
+    if (found) atomicOr(bad, found);
+}
+
+// Bit 3 of *bad when a column lies outside [0, N); only where the offsets, which
+// say how many there are, were found good.
+__global__ void check_columns(const int64_t *__restrict__ row_ptr, const int32_t *__restrict__ cols,
+                              int64_t N, int *__restrict__ bad) {
+    if (__ldcg(bad) & 7) return;
+    const int64_t E = row_ptr[N];
+    bool out = false;
+    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < E;
+         e += (int64_t)gridDim.x * blockDim.x) {
+        const int32_t c = cols[e];
+        out |= c < 0 || c >= N;
+    }
+    if (out) atomicOr(bad, 8);
+}
+
 __global__ void count_targets(const int32_t *__restrict__ inds, int64_t nk,
                               int32_t *__restrict__ indeg) {
     for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < nk;
@@ -571,6 +602,21 @@ bool edges_in_range(const int32_t *a, const int32_t *b, int64_t n, int64_t N, cu
     NCVIS_CUDA(cudaMemcpyAsync(&h, bad, sizeof(int), cudaMemcpyDeviceToHost, s));
     NCVIS_CUDA(cudaStreamSynchronize(s));
     return h == 0;
+}
+
+int check_graph(int64_t N, const int64_t *row_ptr, const int32_t *cols, cudaStream_t s) {
+    StreamBuffer flag(sizeof(int), s);
+    int *bad = (int *)flag.p;
+    NCVIS_CUDA(cudaMemsetAsync(bad, 0, sizeof(int), s));
+    const unsigned most = 16 * num_sms();
+    NCVIS_LAUNCH(check_offsets, (unsigned)std::min<int64_t>((N + 256) / 256, most), 256, 0, s,
+                 row_ptr, N, bad);
+    NCVIS_LAUNCH(check_columns, (unsigned)std::min<int64_t>((N * 16 + 255) / 256, most), 256, 0, s,
+                 row_ptr, cols, N, bad);
+    int h = 0;
+    NCVIS_CUDA(cudaMemcpyAsync(&h, bad, sizeof(int), cudaMemcpyDeviceToHost, s));
+    NCVIS_CUDA(cudaStreamSynchronize(s));
+    return h;
 }
 
 size_t symmetrize_workspace_bytes(int64_t N, int k) {
