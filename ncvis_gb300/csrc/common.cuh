@@ -39,6 +39,23 @@ inline void check_cuda(cudaError_t e, const char *what, const char *file, int li
 
 #define NCVIS_CUDA(call) ::ncvis_gpu::check_cuda((call), #call, __FILE__, __LINE__)
 
+// Unique id of the current context (0 when the thread has none yet).
+unsigned long long current_context_id();
+
+// The library's own stream-ordered memory pool on the current device.  The
+// device's default pool gives its memory back at every synchronisation, and the
+// stage calls synchronise, so that each of them mapped its workspace anew: 0.14 to
+// 0.44 ms a call (1,000 x 32 neighbours, 800,000 x 15 symmetrization).  This one
+// keeps at most kPoolKeeps bytes between calls; they go back when an engine is
+// destroyed and when an allocation finds no room.  The driver orders reuse between
+// streams and threads; a context made anew gets a new pool.
+constexpr size_t kPoolKeeps = size_t(1) << 30;
+cudaMemPool_t workspace_pool();
+// Gives back what the current device's pool keeps unused.
+void trim_workspace_pool();
+// Stream-ordered memory of `bytes` bytes from the pool (cudaFreeAsync frees it).
+void *pool_alloc(size_t bytes, cudaStream_t s);
+
 // A stream-ordered device allocation freed when it goes out of scope, on
 // every exit path (errors included).
 struct StreamBuffer {
@@ -46,7 +63,7 @@ struct StreamBuffer {
     cudaStream_t s;
     explicit StreamBuffer(cudaStream_t st) : s(st) {}
     StreamBuffer(size_t bytes, cudaStream_t st) : s(st) { alloc(bytes); }
-    void alloc(size_t bytes) { NCVIS_CUDA(cudaMallocAsync(&p, bytes > 0 ? bytes : 1, s)); }
+    void alloc(size_t bytes) { p = pool_alloc(bytes, s); }
     StreamBuffer(const StreamBuffer &) = delete;
     StreamBuffer &operator=(const StreamBuffer &) = delete;
     ~StreamBuffer() {

@@ -308,6 +308,7 @@ struct ncvis_engine {
     ~ncvis_engine() {
         if (arena) cudaFree(arena);
         if (own) cudaStreamDestroy(own);
+        if (arena) trim_workspace_pool();
     }
 
     char *ensure_arena(size_t bytes) {
@@ -323,7 +324,14 @@ struct ncvis_engine {
                 arena = nullptr;
                 arena_bytes = 0;
             }
-            NCVIS_CUDA(cudaMalloc(&arena, bytes));
+            cudaError_t r = cudaMalloc(&arena, bytes);
+            if (r == cudaErrorMemoryAllocation) {
+                // The stage calls' pool may hold what is missing.
+                cudaGetLastError();
+                trim_workspace_pool();
+                r = cudaMalloc(&arena, bytes);
+            }
+            NCVIS_CUDA(r);
             arena_bytes = bytes;
         }
         return (char *)arena;
@@ -1087,6 +1095,19 @@ int ncvis_get_stage_times(ncvis_handle h, ncvis_stage_times *out) {
 
 namespace {
 
+// A buffer from the device's default pool: the loss's partials, which a caller who
+// watches that pool expects to see there (the no-allocation entry point's are not).
+struct DefaultPoolBuffer {
+    void *p = nullptr;
+    cudaStream_t s;
+    DefaultPoolBuffer(size_t bytes, cudaStream_t st) : s(st) {
+        NCVIS_CUDA(cudaMallocAsync(&p, bytes, s));
+    }
+    DefaultPoolBuffer(const DefaultPoolBuffer &) = delete;
+    DefaultPoolBuffer &operator=(const DefaultPoolBuffer &) = delete;
+    ~DefaultPoolBuffer() { cudaFreeAsync(p, s); }
+};
+
 void knn_device(const float *dX, size_t N, size_t D, int distance, size_t k, int precision,
                 int rerank_factor, int lists, int probe, int32_t *d_inds, float *d_dists,
                 void *stream) {
@@ -1337,7 +1358,7 @@ int ncvis_nce_loss_device(size_t N, size_t d, size_t E, const int32_t *d_src, co
         cudaStream_t s = (cudaStream_t)stream;
         require(edges_in_range(d_src, d_dst, (int64_t)E, (int64_t)N, s),
                 "nce_loss: an edge endpoint is outside [0, N)");
-        StreamBuffer ws(nce_workspace_bytes((int64_t)E), s);
+        DefaultPoolBuffer ws(nce_workspace_bytes((int64_t)E), s);
         run_nce(0, (int64_t)N, (int)d, (int64_t)E, d_src, d_dst, dY, dQ, (int)n_noise, a, b, seed,
                 tag, edge_offset, nullptr, nullptr, d_loss, ws.p, s);
     });

@@ -303,8 +303,7 @@ struct DeviceArena {
             used += bytes;
             return p;
         }
-        void *p = nullptr;
-        NCVIS_CUDA(cudaMallocAsync(&p, bytes, s));
+        void *p = pool_alloc(bytes, s);
         ptrs.push_back(p);
         return (T *)p;
     }

@@ -50,33 +50,6 @@ static_assert(kScratchBytes == 65568, "the documented size of the scratch array"
 
 __device__ __align__(256) double g_noalloc_scratch[kScratchDoubles];
 
-using CtxGetCurrentFn = CUresult (*)(CUcontext *);
-using CtxGetIdFn = CUresult (*)(CUcontext, unsigned long long *);
-
-template <class Fn>
-Fn driver_entry(const char *name) {
-    void *p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    NCVIS_CUDA(cudaGetDriverEntryPointByVersion(name, &p, 12000, cudaEnableDefault, &q));
-    require(q == cudaDriverEntryPointSuccess && p != nullptr,
-            std::string("nce_loss_noalloc: driver entry point ") + name + " is unavailable",
-            kCudaError);
-    return (Fn)p;
-}
-
-// Unique id of the current context (0 when the thread has none yet).
-unsigned long long current_context_id() {
-    static const CtxGetCurrentFn get_current = driver_entry<CtxGetCurrentFn>("cuCtxGetCurrent");
-    static const CtxGetIdFn get_id = driver_entry<CtxGetIdFn>("cuCtxGetId");
-    CUcontext ctx = nullptr;
-    require(get_current(&ctx) == CUDA_SUCCESS, "nce_loss_noalloc: cuCtxGetCurrent failed",
-            kCudaError);
-    if (!ctx) return 0;
-    unsigned long long id = 0;
-    require(get_id(ctx, &id) == CUDA_SUCCESS, "nce_loss_noalloc: cuCtxGetId failed", kCudaError);
-    return id;
-}
-
 constexpr int kMaxDevices = 128;
 std::mutex g_mu;
 struct Setup {

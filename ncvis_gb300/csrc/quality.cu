@@ -221,7 +221,7 @@ extern "C" int ncvis_trustworthiness_device(const float *dX, size_t N, size_t D,
         const size_t o_thr = L.take(sizeof(float) * N * KQ);
         const size_t o_cnt = L.take(sizeof(int32_t) * N * KQ);
         const size_t o_sum = L.take(sizeof(double));
-        NCVIS_CUDA(cudaMallocAsync((void **)&base, L.total, s));
+        base = (char *)pool_alloc(L.total, s);
         int32_t *nbr = (int32_t *)(base + o_nbr);
         // kNN of the embedding (exact FP32, squared L2), rows without the point itself.
         int rc = ncvis_knn_device(dY, N, d, NCVIS_SQUARED_L2, k, NCVIS_KNN_FP32, 0, nbr,
