@@ -11,9 +11,10 @@
 //           order[j-1], where both are read from the row while it is being
 //           overwritten with the kept entries (src/knntable.cpp:85-93).
 // Here:
-//   1. count_targets / scan: in-degree of every row and bucket offsets;
-//   2. scatter_incoming: each table entry e = s*k + j appends e to its
-//      target's bucket (atomic cursor; arrival order is not deterministic);
+//   1. count_targets / scan: in-degree of every row and bucket offsets, and every
+//      entry's place in its bucket (arrival order is not deterministic);
+//   2. scatter_incoming: each table entry e = s*k + j goes to its place in its
+//      target's bucket;
 //   3. merge, in large tables one thread per row (merge_row.cuh): sorts its bucket by e,
 //      which restores the one-thread arrival order, builds the row's
 //      (distance, position) items, runs the libstdc++-equivalent introsort
@@ -52,16 +53,6 @@ constexpr int64_t kWparRows = 40000;
 constexpr int kWarps1 = 8;
 constexpr int kCap2 = 1024, kWarps2 = 2;
 constexpr int kCap3 = 8192, kWarps3 = 1;
-
-// Flags any index outside [0, N) (the table must name existing points).
-__global__ void check_indices(const int32_t *__restrict__ inds, int64_t nk, int64_t N,
-                              int *__restrict__ bad) {
-    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < nk;
-         e += (int64_t)gridDim.x * blockDim.x) {
-        const int32_t t = inds[e];
-        if (t < 0 || t >= N) atomicOr(bad, 1);
-    }
-}
 
 // bad = 1 if any entry of a or b (n each; b may be null) lies outside [0, N).
 __global__ void check_pairs(const int32_t *__restrict__ a, const int32_t *__restrict__ b,
@@ -105,22 +96,30 @@ __global__ void check_columns(const int64_t *__restrict__ row_ptr, const int32_t
     if (out) atomicOr(bad, 8);
 }
 
-__global__ void count_targets(const int32_t *__restrict__ inds, int64_t nk,
-                              int32_t *__restrict__ indeg) {
-    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < nk;
-         e += (int64_t)gridDim.x * blockDim.x)
-        atomicAdd(&indeg[inds[e]], 1);
-}
-
-__global__ void scatter_incoming(const int32_t *__restrict__ inds, int64_t nk,
-                                 const int64_t *__restrict__ in_off, int32_t *__restrict__ cursor,
-                                 int32_t *__restrict__ in_key) {
+// In-degree of every row, and each entry's place among its target's (the order of
+// arrival), which scatter_incoming needs no atomics of its own for then; flags any
+// index outside [0, N) (the table must name existing points).
+__global__ void count_targets(const int32_t *__restrict__ inds, int64_t nk, int64_t N,
+                              int32_t *__restrict__ indeg, int32_t *__restrict__ place,
+                              int *__restrict__ bad) {
+    bool out = false;
     for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < nk;
          e += (int64_t)gridDim.x * blockDim.x) {
         const int32_t t = inds[e];
-        const int32_t slot = atomicAdd(&cursor[t], 1);
-        in_key[in_off[t] + slot] = (int32_t)e;
+        if (t < 0 || t >= N)
+            out = true;
+        else
+            place[e] = atomicAdd(&indeg[t], 1);
     }
+    if (out) atomicOr(bad, 1);
+}
+
+__global__ void scatter_incoming(const int32_t *__restrict__ inds, int64_t nk,
+                                 const int64_t *__restrict__ in_off,
+                                 const int32_t *__restrict__ place, int32_t *__restrict__ in_key) {
+    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < nk;
+         e += (int64_t)gridDim.x * blockDim.x)
+        in_key[in_off[inds[e]] + place[e]] = (int32_t)e;
 }
 
 template <class V>
@@ -789,26 +788,44 @@ void launch_merge_warp(int k, const int32_t *inds, const float *dists, const int
                  g_items, out_col, out_val, kept, rows, n_rows, next, n_next);
 }
 
-__global__ void compact_rows(int64_t N, int k, const int64_t *__restrict__ in_off,
-                             const int32_t *__restrict__ kept, const int64_t *__restrict__ row_ptr,
-                             const int32_t *__restrict__ out_col, const float *__restrict__ out_val,
-                             int32_t *__restrict__ cols, float *__restrict__ vals,
-                             int32_t *__restrict__ src) {
-    const int lane = threadIdx.x & 31;
-    const int64_t i = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+// The kept entries from their row-aligned places to the CSR, kRowLanes lanes a row,
+// four entries a lane in flight (a whole warp per row, 25 entries of 32 lanes and
+// one load each, took 224 us at 800,000 x 15; so 104).
+constexpr int kRowLanes = 8;
+
+__global__ void __launch_bounds__(256) compact_rows(
+    int64_t N, int k, const int64_t *__restrict__ in_off, const int32_t *__restrict__ kept,
+    const int64_t *__restrict__ row_ptr, const int32_t *__restrict__ out_col,
+    const float *__restrict__ out_val, int32_t *__restrict__ cols, float *__restrict__ vals,
+    int32_t *__restrict__ src) {
+    const int sub = threadIdx.x % kRowLanes;
+    const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / kRowLanes;
     if (i >= N) return;
     const int64_t from = i * k + in_off[i];
     const int64_t to = row_ptr[i];
     const int n = kept[i];
-    for (int j = lane; j < n; j += 32) {
-        cols[to + j] = out_col[from + j];
-        vals[to + j] = out_val[from + j];
-        if (src) src[to + j] = (int32_t)i;
+    for (int j0 = 0; j0 < n; j0 += 4 * kRowLanes) {
+        int32_t c[4];
+        float v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int j = j0 + u * kRowLanes + sub;
+            if (j < n) c[u] = out_col[from + j], v[u] = out_val[from + j];
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int j = j0 + u * kRowLanes + sub;
+            if (j < n) {
+                cols[to + j] = c[u];
+                vals[to + j] = v[u];
+                if (src) src[to + j] = (int32_t)i;
+            }
+        }
     }
 }
 
 struct SymWs {
-    int32_t *indeg, *cursor, *in_key, *out_col, *kept, *bad, *tier1, *tier2, *n_tier;
+    int32_t *indeg, *tier3, *in_key, *out_col, *kept, *bad, *tier1, *tier2, *n_tier;
     int64_t *in_off;
     SortItem *items;
     float *out_val;
@@ -822,7 +839,7 @@ SymWs carve(void *ws, int64_t N, int k) {
     SymWs w;
     const int64_t nk = N * k;
     w.indeg = (int32_t *)p;    p += align256(sizeof(int32_t) * N);
-    w.cursor = (int32_t *)p;   p += align256(sizeof(int32_t) * N);
+    w.tier3 = (int32_t *)p;   p += align256(sizeof(int32_t) * N);
     w.kept = (int32_t *)p;     p += align256(sizeof(int32_t) * N);
     w.bad = (int32_t *)p;      p += align256(sizeof(int32_t));
     w.n_tier = (int32_t *)p;   p += align256(4 * sizeof(int32_t));
@@ -890,17 +907,16 @@ int64_t run_symmetrize(int64_t N, int k, const int32_t *inds, const float *dists
     SymWs w = carve(workspace, N, k);
     const int64_t nk = N * k;
     const unsigned grid = (unsigned)std::min<int64_t>((nk + 255) / 256, 16 * num_sms());
+    int32_t *place = reinterpret_cast<int32_t *>(w.items);  // free until the merges
     NCVIS_CUDA(cudaMemsetAsync(w.bad, 0, sizeof(int32_t), s));
-    NCVIS_LAUNCH(check_indices, grid, 256, 0, s, inds, nk, N, w.bad);
+    NCVIS_CUDA(cudaMemsetAsync(w.indeg, 0, sizeof(int32_t) * N, s));
+    NCVIS_LAUNCH(count_targets, grid, 256, 0, s, inds, nk, N, w.indeg, place, w.bad);
     int bad = 0;
     NCVIS_CUDA(cudaMemcpyAsync(&bad, w.bad, sizeof(int), cudaMemcpyDeviceToHost, s));
     NCVIS_CUDA(cudaStreamSynchronize(s));
     require(bad == 0, "symmetrize: the kNN table holds an index outside [0, N)");
-    NCVIS_CUDA(cudaMemsetAsync(w.indeg, 0, sizeof(int32_t) * N, s));
-    NCVIS_CUDA(cudaMemsetAsync(w.cursor, 0, sizeof(int32_t) * N, s));
-    NCVIS_LAUNCH(count_targets, grid, 256, 0, s, inds, nk, w.indeg);
     launch_exclusive_scan_i32_to_i64(w.indeg, w.in_off, N, w.scan, s);
-    NCVIS_LAUNCH(scatter_incoming, grid, 256, 0, s, inds, nk, w.in_off, w.cursor, w.in_key);
+    NCVIS_LAUNCH(scatter_incoming, grid, 256, 0, s, inds, nk, w.in_off, place, w.in_key);
     NCVIS_CUDA(cudaMemsetAsync(w.n_tier, 0, 4 * sizeof(int32_t), s));
     const bool by_thread = N > kWparRows;
     if (by_thread) {
@@ -911,17 +927,17 @@ int64_t run_symmetrize(int64_t N, int k, const int32_t *inds, const float *dists
                                    w.kept, w.tier1, w.n_tier, nullptr, nullptr, nullptr, nullptr,
                                    s);
     }
-    // From here on the first list's place and the cursors' hold the next lists.
+    // From here on the first list's place and a third hold the next lists.
     launch_merge_wpar<kWarps1>(N, k, inds, dists, w.in_off, w.in_key, w.out_col, w.out_val, w.kept,
                                by_thread ? w.tier2 : nullptr, w.n_tier + 1, w.tier1, w.n_tier + 2,
                                s);
     launch_merge_big<kCap2, kWarps2>(k, inds, dists, w.in_off, w.in_key, w.out_col, w.out_val,
-                                     w.kept, w.tier1, w.n_tier + 2, w.cursor, w.n_tier + 3, s);
+                                     w.kept, w.tier1, w.n_tier + 2, w.tier3, w.n_tier + 3, s);
     launch_merge_warp<kCap3, kWarps3>(k, inds, dists, w.in_off, w.in_key, w.items, w.out_col,
-                                      w.out_val, w.kept, w.cursor, w.n_tier + 3, nullptr, nullptr,
+                                      w.out_val, w.kept, w.tier3, w.n_tier + 3, nullptr, nullptr,
                                       s);
     launch_exclusive_scan_i32_to_i64(w.kept, row_ptr, N, w.scan, s);
-    NCVIS_LAUNCH(compact_rows, ceil_div(N, 8), 256, 0, s, N, k, w.in_off, w.kept, row_ptr,
+    NCVIS_LAUNCH(compact_rows, ceil_div((size_t)N * kRowLanes, 256), 256, 0, s, N, k, w.in_off, w.kept, row_ptr,
                  w.out_col, w.out_val, cols, vals, src);
     int64_t E = 0;
     NCVIS_CUDA(cudaMemcpyAsync(&E, row_ptr + N, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
