@@ -310,6 +310,20 @@ __device__ __forceinline__ void run_chain(float *Y, const int32_t *__restrict__ 
     put_row<D>(Y, cur, yi, yi0);
 }
 
+// Chain copies of Q, summed in FP64 per block (of at most kThreads threads).
+__device__ __forceinline__ void block_q(double v, double *__restrict__ q_part) {
+    __shared__ double red[kThreads / 32];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double t = 0;
+        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[w];
+        q_part[blockIdx.x] = t;
+    }
+}
+
 template <int D>
 __global__ void __launch_bounds__(kThreads) sgd_epoch(float *__restrict__ Y,
                                                       const int32_t *__restrict__ src,
@@ -318,23 +332,12 @@ __global__ void __launch_bounds__(kThreads) sgd_epoch(float *__restrict__ Y,
                                                       double *__restrict__ q_part, EpochConst k,
                                                       int epoch, uint32_t key0, uint32_t key1,
                                                       int64_t chunk, int64_t n_chains) {
-    const int64_t chain = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+    const int64_t chain = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t e0 = chain < n_chains ? min(E, chain * chunk) : E;
     const int64_t e1 = min(E, e0 + chunk);
     float Qc = *Q_in;
     run_chain<D>(Y, src, dst, e0, e1, N, 0u, k, Qc, key0, key1, (uint32_t)epoch);
-    // Chain copies of Q, summed in FP64 per block.
-    __shared__ double red[kThreads / 32];
-    double v = chain < n_chains ? (double)Qc : 0.0;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double t = 0;
-        for (int w = 0; w < kThreads / 32; ++w) t += red[w];
-        q_part[blockIdx.x] = t;
-    }
+    block_q(chain < n_chains ? (double)Qc : 0.0, q_part);
 }
 
 // Runtime-d variant (d > 4).
@@ -342,7 +345,7 @@ __global__ void __launch_bounds__(kThreads) sgd_epoch_generic(
     float *__restrict__ Y, int d, const int32_t *__restrict__ src, const int32_t *__restrict__ dst,
     int64_t E, uint32_t N, const float *__restrict__ Q_in, double *__restrict__ q_part, EpochConst k,
     int epoch, uint32_t key0, uint32_t key1, int64_t chunk, int64_t n_chains) {
-    const int64_t chain = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+    const int64_t chain = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t e0 = chain < n_chains ? chain * chunk : E;
     const int64_t e1 = min(E, e0 + chunk);
     float Qc = *Q_in;
@@ -366,17 +369,7 @@ __global__ void __launch_bounds__(kThreads) sgd_epoch_generic(
             }
         }
     }
-    __shared__ double red[kThreads / 32];
-    double v = chain < n_chains ? (double)Qc : 0.0;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double t = 0;
-        for (int w = 0; w < kThreads / 32; ++w) t += red[w];
-        q_part[blockIdx.x] = t;
-    }
+    block_q(chain < n_chains ? (double)Qc : 0.0, q_part);
 }
 
 // Batched problems: problem p owns rows [off[p], off[p+1]), edges
@@ -1059,6 +1052,7 @@ int sgd_default_chains(int64_t E, int64_t N, int d) {
 }
 
 size_t sgd_workspace_bytes(int chains) {
+    // Blocks of kThreads chains, or up to two of fewer per SM (run_sgd_hogwild).
     const int64_t most = std::max<int64_t>(chains, (int64_t)num_sms() * 2048);
     return sizeof(double) * ((most + kThreads - 1) / kThreads + 1);
 }
@@ -1067,7 +1061,13 @@ void run_sgd_hogwild(const SgdArgs &g, int epoch_begin, int epoch_end, const siz
                      int chains, void *workspace, cudaStream_t s) {
     require(g.N >= 2 && g.N < (int64_t(1) << 31), "optimize: N must be in [2, 2^31)");
     if (chains <= 0) chains = sgd_default_chains(g.E, g.N, g.d);
-    const int blocks = (int)ceil_div(chains, kThreads);
+    // Few chains are spread over all SMs: a sample's row gather and its reduction
+    // each take an SM's load unit a cycle a lane, so that 5,000 chains in blocks of
+    // 256 waited for 20 SMs (547 us an epoch of 20 noise samples at 10,000 points;
+    // 474 in blocks of 32).
+    const int sms = num_sms();
+    const int threads = std::max(32, std::min(kThreads, chains / sms / 32 * 32));
+    const int blocks = (int)ceil_div(chains, threads);
     const int64_t total_chains = chains;
     const int64_t chunk = ((g.E + total_chains - 1) / total_chains + 3) & ~(int64_t)3;
     double *q_part = (double *)workspace;
@@ -1078,23 +1078,23 @@ void run_sgd_hogwild(const SgdArgs &g, int epoch_begin, int epoch_end, const siz
         EpochConst k = epoch_const(g, ep, nu);
         switch (g.d) {
             case 1:
-                NCVIS_LAUNCH(sgd_epoch<1>, blocks, kThreads, 0, s, g.Y, g.src, g.dst, g.E,
+                NCVIS_LAUNCH(sgd_epoch<1>, blocks, threads, 0, s, g.Y, g.src, g.dst, g.E,
                              (uint32_t)g.N, g.Q, q_part, k, ep, key0, key1, chunk, total_chains);
                 break;
             case 2:
-                NCVIS_LAUNCH(sgd_epoch<2>, blocks, kThreads, 0, s, g.Y, g.src, g.dst, g.E,
+                NCVIS_LAUNCH(sgd_epoch<2>, blocks, threads, 0, s, g.Y, g.src, g.dst, g.E,
                              (uint32_t)g.N, g.Q, q_part, k, ep, key0, key1, chunk, total_chains);
                 break;
             case 3:
-                NCVIS_LAUNCH(sgd_epoch<3>, blocks, kThreads, 0, s, g.Y, g.src, g.dst, g.E,
+                NCVIS_LAUNCH(sgd_epoch<3>, blocks, threads, 0, s, g.Y, g.src, g.dst, g.E,
                              (uint32_t)g.N, g.Q, q_part, k, ep, key0, key1, chunk, total_chains);
                 break;
             case 4:
-                NCVIS_LAUNCH(sgd_epoch<4>, blocks, kThreads, 0, s, g.Y, g.src, g.dst, g.E,
+                NCVIS_LAUNCH(sgd_epoch<4>, blocks, threads, 0, s, g.Y, g.src, g.dst, g.E,
                              (uint32_t)g.N, g.Q, q_part, k, ep, key0, key1, chunk, total_chains);
                 break;
             default:
-                NCVIS_LAUNCH(sgd_epoch_generic, blocks, kThreads, 0, s, g.Y, g.d, g.src, g.dst,
+                NCVIS_LAUNCH(sgd_epoch_generic, blocks, threads, 0, s, g.Y, g.d, g.src, g.dst,
                              g.E, (uint32_t)g.N, g.Q, q_part, k, ep, key0, key1, chunk, total_chains);
         }
         NCVIS_LAUNCH(reduce_q, 1, 1024, 0, s, q_part, blocks, total_chains, g.Q);
