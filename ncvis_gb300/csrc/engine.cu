@@ -218,18 +218,19 @@ static BatchedTcWork plan_batched_tc(const std::vector<int64_t> &off, int ctas_m
 
 // The FP32 search of one problem: on the tensor cores over FP16 part rows where
 // the shape and the rows' norms allow it (split_scale), else K3 on the CUDA
-// cores.  The part rows, the further lists and the work list share one block
+// cores.  The part rows, the split rows' lists and the work list share one block
 // of memory.
 struct KnnF32Plan {
     KnnPlan simt{};
     KnnTcPlan tc{};
     TcSweep sweep;
     bool split = false;
-    size_t rows_bytes = 0, lists_bytes = 0, work_bytes = 0;
+    int keep = 0;  // candidates re-ranked per row
+    size_t rows_bytes = 0, sweep_size = 0;
     size_t cand_bytes(size_t N) const {
-        return sizeof(int32_t) * N * std::max(simt.C(), split ? tc.R : 0);
+        return sizeof(int32_t) * N * std::max(simt.C(), split ? keep : 0);
     }
-    size_t block_bytes() const { return split ? rows_bytes + lists_bytes + work_bytes : 0; }
+    size_t block_bytes() const { return split ? rows_bytes + sweep_size : 0; }
 };
 
 // From this many rows on the tensor cores are the faster of the two (a whole
@@ -246,43 +247,51 @@ static KnnF32Plan plan_knn_fp32(size_t N, size_t D, int k, int rerank_factor, in
     p.tc = plan_knn_split((int)D, p.simt.R, dist);
     p.sweep = plan_sweep((int64_t)N, num_sms());
     p.rows_bytes = align256(sizeof(__half) * (p.tc.fold ? 3 : 2) * N * p.tc.ldb);
-    p.lists_bytes = align256(sizeof(int32_t) * (size_t)p.sweep.split_rows *
-                             (p.sweep.lists - 1) * p.tc.R);
-    p.work_bytes = align256(sweep_work_bytes((int64_t)N, p.sweep));
+    p.sweep_size = sweep_bytes((int64_t)N, p.sweep, p.tc.R);
+    // Where every row has lists of several runs, the best 64 of them are
+    // re-ranked: the CUDA cores' search of so few rows keeps more than 32, too.
+    p.keep = p.sweep.lists > 1 && p.sweep.full_qt == 0 ? 64 : p.tc.R;
     return p;
 }
 
-// Where a search left its candidates: C per row, and the further lists.
-struct Candidates {
-    int C = 0;
-    TcLists lists;
-};
-
 // Runs the search into cand (plan.cand_bytes) with block (plan.block_bytes) as
-// scratch; norms: the words of launch_preprocess, on the host.
-static Candidates run_knn_fp32(const float *Xp, const float *sqn, size_t N, size_t D, int dist,
-                               const KnnF32Plan &plan, const uint32_t *norms, int32_t *cand,
-                               char *block, int *timeout_flag, cudaStream_t s) {
-    Candidates c;
+// scratch; norms: the words of launch_preprocess, on the host.  Returns the number
+// of candidates per row.
+static int run_knn_fp32(const float *Xp, const float *sqn, size_t N, size_t D, int dist,
+                        const KnnF32Plan &plan, const uint32_t *norms, int32_t *cand, char *block,
+                        int *timeout_flag, cudaStream_t s) {
     const float scale = plan.split ? split_scale(norms, dist) : 0.f;
     if (scale == 0.f) {
         launch_knn_select_f32(Xp, sqn, (int64_t)N, (int)D, dist, plan.simt, cand, s);
-        c.C = plan.simt.C();
-        return c;
+        return plan.simt.C();
     }
     __half *rows = (__half *)block;
     launch_split_rows(Xp, sqn, (int64_t)N, (int)D, scale, plan.tc, rows, (int64_t)N, s);
-    c.C = plan.tc.R;
-    c.lists.row0 = (int64_t)N - plan.sweep.split_rows;
-    c.lists.count = plan.sweep.lists - 1;
-    c.lists.extra = (int32_t *)(block + plan.rows_bytes);
-    if (plan.lists_bytes)
-        NCVIS_CUDA(cudaMemsetAsync(c.lists.extra, 0xff, plan.lists_bytes, s));
-    TcWork work = launch_sweep_work((int64_t)N, plan.sweep,
-                                    block + plan.rows_bytes + plan.lists_bytes, s);
-    work.lists = c.lists;
+    const TcWork work =
+        launch_sweep_work((int64_t)N, plan.sweep, plan.tc.R, block + plan.rows_bytes, s);
     launch_knn_select_split(rows, (int64_t)N, plan.tc, cand, timeout_flag, s, work);
-    return c;
+    launch_merge_lists((int64_t)N, plan.sweep, work.lists, plan.tc.R, plan.keep, nullptr, cand, s);
+    return plan.keep;
+}
+
+// How the BF16 search spreads its query tiles, and the block of memory for the
+// work list (in the caller's row order) and the split rows' lists.
+struct KnnBf16Sweep {
+    TcSweep sweep;
+    size_t bytes = 0;
+    KnnBf16Sweep(size_t N, const KnnTcPlan &tp, const KnnOrderPlan &op, bool split) {
+        sweep = split ? plan_sweep((int64_t)N, num_sms()) : whole_tiles((int64_t)N, num_sms());
+        bytes = op.C > 0 ? sweep_lists_bytes(sweep, tp.R) : sweep_bytes((int64_t)N, sweep, tp.R);
+    }
+};
+
+// The BF16 search in the caller's order; block: bs.bytes.
+static void run_knn_tc(const __nv_bfloat16 *Xb, const __nv_bfloat16 *Xc, const float *sqn,
+                       int64_t N, const KnnTcPlan &tp, int dist, const KnnBf16Sweep &bs,
+                       char *block, int32_t *cand, int *timeout_flag, cudaStream_t s) {
+    const TcWork work = launch_sweep_work(N, bs.sweep, tp.R, block, s);
+    launch_knn_select_tc(Xb, sqn, N, tp, dist, cand, timeout_flag, s, work, Xc);
+    launch_merge_lists(N, bs.sweep, work.lists, tp.R, tp.R, nullptr, cand, s);
 }
 
 struct ncvis_engine {
@@ -481,29 +490,33 @@ void ncvis_engine::fit(const float *X, size_t N, size_t D, float *Y, bool host) 
     const size_t o_stream = replay ? L.take(sizeof(int32_t) * std::max<size_t>(o.replay_len, 1)) : 0;
     const size_t ord_bytes = knn_order_workspace_bytes((int64_t)N, (int)D, tp, op);
     const size_t o_ord = ord_bytes ? L.take(ord_bytes) : 0;
-    const TcSweep whole = whole_tiles((int64_t)N, num_sms());
-    const size_t o_work =
-        bf16 && !ivf && op.C <= 0 ? L.take(sweep_work_bytes((int64_t)N, whole)) : 0;
-    // Last: the candidates, and the symmetrization's workspace, which the FP32
-    // search's part rows and lists share (they are read for the last time by
-    // the rerank before it).  Where memory, or the caller's limit, has no room
-    // for those the search takes the CUDA cores.
+    KnnBf16Sweep bs(N, tp, op, bf16 && !ivf);
+    // Last: the candidates, and the symmetrization's workspace, which the
+    // search's part rows, lists and work list share (they are read for the last
+    // time before it).  Where memory, or the caller's limit, has no room for those
+    // the FP32 search takes the CUDA cores and the BF16 one whole query tiles.
     const size_t o_ci = L.total;
     auto cand_bytes = [&] {
         return align256(bf16 ? sizeof(int32_t) * N * tp.R : fp.cand_bytes(N));
     };
     auto total_bytes = [&] {
         return o_ci + cand_bytes() +
-               align256(std::max(symmetrize_workspace_bytes((int64_t)N, k), fp.block_bytes()));
+               align256(std::max({symmetrize_workspace_bytes((int64_t)N, k), fp.block_bytes(),
+                                  bf16 && !ivf ? bs.bytes : 0}));
     };
-    if (fp.split && o.arena_limit && total_bytes() > o.arena_limit) fp.split = false;
+    auto take_less = [&] {
+        fp.split = false;
+        bs = KnnBf16Sweep(N, tp, op, false);
+    };
+    if (o.arena_limit && total_bytes() > o.arena_limit) take_less();
     char *base = nullptr;
     try {
         base = ensure_arena(total_bytes());
     } catch (const Error &) {
-        if (!fp.split) throw;
+        const size_t wanted = total_bytes();
+        take_less();
+        if (total_bytes() == wanted) throw;
         cudaGetLastError();
-        fp.split = false;
         base = ensure_arena(total_bytes());
     }
     const size_t o_sym = o_ci + cand_bytes();
@@ -542,8 +555,7 @@ void ncvis_engine::fit(const float *X, size_t N, size_t D, float *Y, bool host) 
     require(h_flag[0] == 0, "[ncvis] input contains non-finite values");
     nv.next("ncvis.knn");
     const int32_t *cell_order = nullptr;  // rows in k-means cell order (ordered sweep only)
-    Candidates found;
-    found.C = tp.R;
+    int C = tp.R;
     NCVIS_CUDA(cudaMemsetAsync(knn_i, 0xff, sizeof(int32_t) * nk, s));
     if (ivf)
         run_knn_ivf(Xp, Xb, Xc, (int64_t)N, (int)D, tp, dist,
@@ -551,17 +563,16 @@ void ncvis_engine::fit(const float *X, size_t N, size_t D, float *Y, bool host) 
                     cand_i, flag + 2, s);
     else if (op.C > 0)
         run_knn_tc_ordered(Xp, Xb, Xc, (int64_t)N, (int)D, tp, dist, op, (uint64_t)p.random_seed,
-                           cand_i, flag + 2, s, base + o_ord, ord_bytes, ev.ev[9], &cell_order);
+                           cand_i, flag + 2, s, base + o_ord, ord_bytes, ev.ev[9], &cell_order,
+                           bs.sweep.lists > 1 ? base + o_sym : nullptr);
     else if (bf16)
-        launch_knn_select_tc(Xb, sqn, (int64_t)N, tp, dist, cand_i, flag + 2, s,
-                             launch_sweep_work((int64_t)N, whole, base + o_work, s), Xc);
+        run_knn_tc(Xb, Xc, sqn, (int64_t)N, tp, dist, bs, base + o_sym, cand_i, flag + 2, s);
     else
-        found = run_knn_fp32(Xp, sqn, N, D, dist, fp, (const uint32_t *)h_flag + 4, cand_i,
-                             base + o_sym, flag + 2, s);
+        C = run_knn_fp32(Xp, sqn, N, D, dist, fp, (const uint32_t *)h_flag + 4, cand_i,
+                         base + o_sym, flag + 2, s);
     NCVIS_CUDA(cudaEventRecord(ev.ev[3], s));
     nv.next("ncvis.rerank");
-    launch_rerank(Xp, (int64_t)N, (int)D, dist, cand_i, found.C, k, knn_i, knn_d, s, cell_order,
-                  found.lists);
+    launch_rerank(Xp, (int64_t)N, (int)D, dist, cand_i, C, k, knn_i, knn_d, s, cell_order);
     NCVIS_CUDA(cudaEventRecord(ev.ev[4], s));
     nv.next("ncvis.symmetrize");
     if (bf16 || fp.split) {
@@ -1143,22 +1154,26 @@ void knn_device(const float *dX, size_t N, size_t D, int distance, size_t k, int
         const size_t o_Xb = bf16 ? L.take(sizeof(__nv_bfloat16) * N * tp.ldb) : 0;
         const size_t o_Xc = fold ? L.take(sizeof(__nv_bfloat16) * N * tp.ldb) : 0;
         const size_t o_ord = ord_bytes ? L.take(ord_bytes) : 0;
-        const TcSweep whole = whole_tiles((int64_t)N, num_sms());
-        const size_t o_work =
-            bf16 && !ivf && op.C <= 0 ? L.take(sweep_work_bytes((int64_t)N, whole)) : 0;
+        KnnBf16Sweep bs(N, tp, op, bf16 && !ivf);
         const size_t o_ci = L.total;
         auto cand_bytes = [&] {
             return align256(bf16 ? sizeof(int32_t) * N * tp.R : fp.cand_bytes(N));
         };
+        auto total_bytes = [&] {
+            return o_ci + cand_bytes() + (bf16 && !ivf ? bs.bytes : fp.block_bytes());
+        };
         StreamBuffer buf(s);
         try {
-            buf.alloc(o_ci + cand_bytes() + fp.block_bytes());
+            buf.alloc(total_bytes());
         } catch (const Error &) {
-            // No room for the part rows: the search on the CUDA cores needs less.
-            if (!fp.split) throw;
-            cudaGetLastError();
+            // No room for the part rows or the lists: the search on the CUDA cores,
+            // or by whole query tiles, needs less.
+            const size_t wanted = total_bytes();
             fp.split = false;
-            buf.alloc(o_ci + cand_bytes());
+            bs = KnnBf16Sweep(N, tp, op, false);
+            if (total_bytes() == wanted) throw;
+            cudaGetLastError();
+            buf.alloc(total_bytes());
         }
         const size_t o_block = o_ci + cand_bytes();
         char *base = (char *)buf.p;
@@ -1176,26 +1191,23 @@ void knn_device(const float *dX, size_t N, size_t D, int distance, size_t k, int
         require(!h_flag[0], "knn: input contains non-finite values");
         NCVIS_CUDA(cudaMemsetAsync(d_inds, 0xff, sizeof(int32_t) * N * k, s));
         const int32_t *cell_order = nullptr;
-        Candidates found;
-        found.C = tp.R;
+        int C = tp.R;
         if (ivf) {
             run_knn_ivf((float *)(base + o_Xp), Xb, Xc, (int64_t)N, (int)D, tp, distance,
                         plan_ivf((int64_t)N, lists, probe), 42, cand, flag + 2, s);
         } else if (op.C > 0) {
             run_knn_tc_ordered((float *)(base + o_Xp), Xb, Xc, (int64_t)N, (int)D, tp, distance,
                                op, 42, cand, flag + 2, s, base + o_ord, ord_bytes, nullptr,
-                               &cell_order);
+                               &cell_order, bs.sweep.lists > 1 ? base + o_block : nullptr);
         } else if (bf16) {
-            launch_knn_select_tc(Xb, (float *)(base + o_sqn), (int64_t)N, tp, distance, cand,
-                                 flag + 2, s,
-                                 launch_sweep_work((int64_t)N, whole, base + o_work, s), Xc);
+            run_knn_tc(Xb, Xc, (float *)(base + o_sqn), (int64_t)N, tp, distance, bs,
+                       base + o_block, cand, flag + 2, s);
         } else {
-            found = run_knn_fp32((float *)(base + o_Xp), (float *)(base + o_sqn), N, D, distance,
-                                 fp, (const uint32_t *)h_flag + 4, cand, base + o_block, flag + 2,
-                                 s);
+            C = run_knn_fp32((float *)(base + o_Xp), (float *)(base + o_sqn), N, D, distance, fp,
+                             (const uint32_t *)h_flag + 4, cand, base + o_block, flag + 2, s);
         }
-        launch_rerank((float *)(base + o_Xp), (int64_t)N, (int)D, distance, cand, found.C, (int)k,
-                      d_inds, d_dists, s, cell_order, found.lists);
+        launch_rerank((float *)(base + o_Xp), (int64_t)N, (int)D, distance, cand, C, (int)k,
+                      d_inds, d_dists, s, cell_order);
         // The tensor-core kernel without its own check of the timeout flag.
         if ((bf16 && !ivf && op.C <= 0) || fp.split) {
             int timeout = 0;

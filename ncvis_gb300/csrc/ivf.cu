@@ -583,7 +583,7 @@ size_t knn_order_workspace_bytes(int64_t N, int D, const KnnTcPlan &tp, const Kn
     if (op.C <= 0) return 0;
     auto a = [](size_t b) { return (std::max<size_t>(b, 1) + 255) & ~(size_t)255; };
     const size_t C = (size_t)op.C, ldb = (size_t)tp.ldb, n = (size_t)N;
-    const size_t tiles = (n + 255) / 256, ctas = 1024;  // work-list bounds (ctas <= SMs)
+    const size_t tiles = (n + 255) / 256, ctas = (size_t)num_sms();  // work-list bounds
     size_t b = 0;
     // kmeans_cells: centroids, sums, counts, centroid rows, the assignment work list.
     b += 2 * a(sizeof(float) * C * D) + a(sizeof(int) * C) + 2 * a(2 * C * ldb);
@@ -591,8 +591,9 @@ size_t knn_order_workspace_bytes(int64_t N, int D, const KnnTcPlan &tp, const Kn
     // sort_by_cell: counts, cursors, starts, permutation, sorted rows.
     b += 2 * a(sizeof(int) * C) + a(sizeof(int64_t) * (C + 1)) + a(sizeof(int32_t) * n);
     b += 2 * a(2 * n * ldb);
-    // the sweep's work list.
-    b += a(sizeof(int64_t) * (ctas + 1)) + a(sizeof(TcItem) * 2 * tiles);
+    // the sweep's work list: a query tile, or a CTA's piece of one of the last, is
+    // at most two items.
+    b += a(sizeof(int64_t) * (ctas + 1)) + a(sizeof(TcItem) * 2 * (tiles + ctas));
     return b;
 }
 
@@ -600,11 +601,9 @@ void run_knn_tc_ordered(const float *Xp, const __nv_bfloat16 *Xb, const __nv_bfl
                         int64_t N, int D, const KnnTcPlan &tp, int dist, const KnnOrderPlan &op,
                         uint64_t seed, int32_t *cand_i, int *timeout_flag, cudaStream_t s,
                         void *workspace, size_t workspace_bytes, cudaEvent_t sweep_start,
-                        const int32_t **cell_order) {
+                        const int32_t **cell_order, void *list_memory) {
     require(op.C > 0, "knn: ordered search without cells", kInternal);
     require(N < (int64_t(1) << 31), "knn: N must be below 2^31");
-    require(num_sms() <= 1024, "knn: more SMs than the ordered search's work list allows",
-            kUnsupported);
     const bool fold = tp.fold;
     DeviceArena arena(s, workspace, workspace_bytes);
     Cells cells;
@@ -614,22 +613,55 @@ void run_knn_tc_ordered(const float *Xp, const __nv_bfloat16 *Xb, const __nv_bfl
 
     // Work list: query tile t of the sorted rows against [s0, N) then [0, s0),
     // s0 = its first row's cell start rounded down to a candidate tile; tile t
-    // goes to CTA t mod ctas.
-    const int64_t tiles = (N + 255) / 256;
+    // goes to CTA t mod ctas.  The tiles of the last wave are shared out over all
+    // CTAs in runs of candidate tiles (counted from s0) whose lists are merged
+    // afterwards: 131,072 x 100 has 512 tiles on 152 SMs, and its sweep went from
+    // 4,255 to 3,918 us, that of 1,024,000 x 100 (48 tiles left) from 172 to 167 ms.  A
+    // run that does not begin at s0 first sees the rows around its own (kTcSeed),
+    // whose scores bound what it lists; without that it meets row after row of other
+    // cells that beat what it has (4,185 us; 60,013 x 100 1,504 and 1,287).
+    const TcSweep sweep = list_memory ? plan_sweep(N, num_sms()) : whole_tiles(N, num_sms());
+    const int64_t n_ct = (N + 127) / 128, n_qt = (N + 255) / 256;
     HostWork w;
-    w.ctas = (int)std::min<int64_t>(tiles, num_sms());
+    w.ctas = sweep.ctas;
     std::vector<std::vector<TcItem>> per(w.ctas);
+    // Candidate tiles [u0, u1) of query tile t, counted from s0.
+    auto add = [&](std::vector<TcItem> &v, int64_t t, int64_t s0, int64_t u0, int64_t u1, int slot) {
+        const int64_t wrap = n_ct - s0 / 128;  // tiles before the end of the rows
+        const int r0 = (int)(256 * t);
+        if (u0 < wrap) {
+            const int64_t hi = std::min(N, s0 + 128 * u1);
+            v.push_back(TcItem{r0, (int)N, (int)(s0 + 128 * u0), (int)hi, 0,
+                               u1 > wrap ? kTcMore : 0, slot, 0});
+        }
+        if (u1 > wrap) {
+            const int64_t lo = 128 * std::max<int64_t>(u0 - wrap, 0);
+            v.push_back(TcItem{r0, (int)N, (int)lo, (int)(128 * (u1 - wrap)), 0,
+                               u0 < wrap ? kTcContinue : 0, slot, 0});
+        }
+    };
+    constexpr int64_t kSeedTiles = 8;  // 131,072 x 100: 3,918 us, with 24 3,978
+    const TcRun run(N, sweep);
     int c = 0;
-    for (int64_t t = 0; t < tiles; ++t) {
-        const int64_t r0 = 256 * t;
-        while (cells.starts[c + 1] <= r0) ++c;
-        const int64_t s0 = cells.starts[c] / 128 * 128;
-        std::vector<TcItem> &v = per[t % w.ctas];
-        if (s0 == 0) {
-            v.push_back(TcItem{(int)r0, (int)N, 0, (int)N, 0, 0, 0, 0});
-        } else {
-            v.push_back(TcItem{(int)r0, (int)N, (int)s0, (int)N, 0, kTcMore, 0, 0});
-            v.push_back(TcItem{(int)r0, (int)N, 0, (int)s0, 0, kTcContinue, 0, 0});
+    for (int64_t t = 0; t < n_qt; ++t) {
+        while (cells.starts[c + 1] <= 256 * t) ++c;
+        const int64_t s0 = cells.starts[c] / 128 * 128, r = t - sweep.full_qt;
+        if (r < 0) {
+            add(per[t % w.ctas], t, s0, 0, n_ct, 0);
+            continue;
+        }
+        const int64_t first = run.first_cta(r), last = run.last_cta(r);
+        for (int64_t b = first; b <= last; ++b) {
+            const int64_t u0 = std::max<int64_t>(run.begin(b) - r * n_ct, 0);
+            const size_t at = per[b].size() + 1;
+            if (u0 > 0) {
+                const int64_t lo = std::max<int64_t>(0, 256 * t - 64 * (kSeedTiles - 2));
+                per[b].push_back(TcItem{(int)(256 * t), (int)N, (int)lo,
+                                        (int)std::min(N, lo + 128 * kSeedTiles), 0,
+                                        kTcMore | kTcSeed, (int)(b - first), 0});
+            }
+            add(per[b], t, s0, u0, std::min(n_ct, run.begin(b + 1) - r * n_ct), (int)(b - first));
+            if (u0 > 0) per[b][at].flags |= kTcContinue;
         }
     }
     w.begin.assign(w.ctas + 1, 0);
@@ -637,10 +669,12 @@ void run_knn_tc_ordered(const float *Xp, const __nv_bfloat16 *Xb, const __nv_bfl
         w.items.insert(w.items.end(), per[b].begin(), per[b].end());
         w.begin[b + 1] = (int64_t)w.items.size();
     }
-    const TcWork sweep = upload(w, cells.perm, arena);
+    TcWork work = upload(w, cells.perm, arena);
+    work.lists = sweep_lists(N, sweep, tp.R, list_memory);
     if (sweep_start) NCVIS_CUDA(cudaEventRecord(sweep_start, s));
     launch_knn_select_tc_pair(cells.Xs, N, fold ? cells.Xcs : cells.Xs, N, nullptr, tp, true,
-                              cand_i, timeout_flag, s, sweep);
+                              cand_i, timeout_flag, s, work);
+    launch_merge_lists(N, sweep, work.lists, tp.R, tp.R, cells.perm, cand_i, s);
     check_timeout(timeout_flag, s);
     // The rows in cell order (sorted position -> row), for the caller's
     // rerank; only from a caller's workspace, which outlives this call.

@@ -235,31 +235,34 @@ __global__ void __launch_bounds__(NT) knn_select_f32(const float *__restrict__ X
 // One warp per point.  The query row is spread over the lanes (coordinate
 // t in lane t % 32); each candidate row is read coalesced and its exact FP32
 // distance reduced across the warp (the same lane split for (i, j) and
-// (j, i), so d(i, j) == d(j, i)).  Candidates are then ranked; at most 1024.
-// Positions from lists.row0 on have lists.count more lists of C candidates.
-// T: ceil(D / 32) coordinates per lane, T <= 4; T == 0: any D.  kLists: some
-// rows have further lists (a form of its own, so that the other keeps 64
-// registers: with both in one the rerank of 1,024,000 rows took 3.5 ms, not 2.6).
-template <int T, bool kLists>
+// (j, i), so d(i, j) == d(j, i)).  Candidates are then ranked; at most 1024, and
+// entries outside [0, N) (-1: empty) are left out.
+// T: ceil(D / 32) coordinates per lane, T <= 4; T == 0: any D.
+// The sums of eight candidates go down the warp together: each step of the
+// butterfly hands over half of the values still held, so that they take 9 shuffles
+// where one after the other took 40 (the same additions in the same order).
+template <int T>
 __global__ void __launch_bounds__(128) rerank_rows(const float *__restrict__ Xp, int64_t N, int D,
                                                    int dist, const int32_t *__restrict__ cand_i,
-                                                   int C0, int k, int32_t *__restrict__ inds,
+                                                   int C, int k, int32_t *__restrict__ inds,
                                                    float *__restrict__ dists,
-                                                   const int32_t *__restrict__ order,
-                                                   TcLists lists) {
+                                                   const int32_t *__restrict__ order) {
     extern __shared__ __align__(16) char smem_raw[];
+    struct Pair {
+        float d;
+        int32_t i;
+    };
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t w = (int64_t)blockIdx.x * (blockDim.x >> 5) + warp;
-    const int most = kLists ? C0 * (1 + lists.count) : C0;
-    float *sd = (float *)smem_raw + (size_t)warp * most * 2;
-    int *si = (int *)(sd + most);
+    Pair *sp = (Pair *)smem_raw + (size_t)warp * C;
     if (w >= N) return;
-    const bool more = kLists && w >= lists.row0;
-    const int C = more ? most : C0;
-    const int32_t *extra = more ? lists.extra + (w - lists.row0) * lists.count * C0 : nullptr;
     // Rows in `order` (a permutation of [0, N)) when given: neighbouring points
     // then run together and share their candidates' rows in L2.
     const int64_t row = order ? (int64_t)order[w] : w;
+    for (int c = lane; c < C; c += 32) {
+        const int32_t i = cand_i[row * C + c];
+        sp[c] = {FLT_MAX, (uint32_t)i < (uint32_t)N ? i : -1};
+    }
     const float *q = Xp + row * D;
     const bool l2 = (dist == kSquaredL2);
     float qv[T > 0 ? T : 1];
@@ -270,6 +273,7 @@ __global__ void __launch_bounds__(128) rerank_rows(const float *__restrict__ Xp,
             qv[t] = c < D ? q[c] : 0.f;
         }
     }
+    __syncwarp();
     // Candidates in flight per warp: 8 (64 registers) took the rerank of
     // 1,024,000 rows x 32 candidates from 3.84 to 2.68 ms against 4; 16 (128
     // registers, half the resident warps) 4.02 ms.
@@ -279,11 +283,7 @@ __global__ void __launch_bounds__(128) rerank_rows(const float *__restrict__ Xp,
         float part[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            const int c = c0 + u;  // warp-uniform
-            if constexpr (kLists)
-                idx[u] = c < C0 ? cand_i[row * C0 + c] : (c < C ? extra[c - C0] : -1);
-            else
-                idx[u] = c < C0 ? cand_i[row * C0 + c] : -1;
+            idx[u] = c0 + u < C ? sp[c0 + u].i : -1;  // warp-uniform
             part[u] = 0.f;
         }
         if (T > 0) {
@@ -322,30 +322,36 @@ __global__ void __launch_bounds__(128) rerank_rows(const float *__restrict__ Xp,
                 }
             }
         }
+        // Lane l ends with the sum of candidate c0 + (l >> 2).
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
+        for (int h = U / 2, o = 16; h > 0; h >>= 1, o >>= 1) {
+            const bool up = lane & o;
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1)
-                part[u] = __fadd_rn(part[u], __shfl_xor_sync(0xffffffffu, part[u], o));
-            if (lane == 0 && c0 + u < C) {
-                sd[c0 + u] = idx[u] >= 0 ? (l2 ? part[u] : __fsub_rn(1.f, part[u])) : FLT_MAX;
-                si[c0 + u] = idx[u];
+            for (int u = 0; u < h; ++u) {
+                const float give = up ? part[u] : part[u + h], keep = up ? part[u + h] : part[u];
+                part[u] = __fadd_rn(keep, __shfl_xor_sync(0xffffffffu, give, o));
             }
         }
+#pragma unroll
+        for (int o = 2; o > 0; o >>= 1)
+            part[0] = __fadd_rn(part[0], __shfl_xor_sync(0xffffffffu, part[0], o));
+        const int c = c0 + (lane >> 2);
+        if ((lane & 3) == 0 && c < C && sp[c].i >= 0)
+            sp[c].d = l2 ? part[0] : __fsub_rn(1.f, part[0]);
     }
     __syncwarp();
     for (int c = lane; c < C; c += 32) {
-        const int idx = si[c];
-        if (idx < 0) continue;
-        const float dv = sd[c];
+        const Pair me = sp[c];
+        if (me.i < 0) continue;
         int rank = 0;
+#pragma unroll 4
         for (int t = 0; t < C; ++t) {
-            const int it = si[t];
-            rank += (it >= 0 && pair_less(sd[t], it, dv, idx)) ? 1 : 0;
+            const Pair it = sp[t];
+            rank += (it.i >= 0 && pair_less(it.d, it.i, me.d, me.i)) ? 1 : 0;
         }
         if (rank >= 1 && rank <= k) {
-            inds[row * k + (k - rank)] = idx;
-            dists[row * k + (k - rank)] = dv;
+            inds[row * k + (k - rank)] = me.i;
+            dists[row * k + (k - rank)] = me.d;
         }
     }
 }
@@ -386,34 +392,25 @@ void launch_knn_select_f32(const float *Xp, const float *sqnorm, int64_t N, int 
 }
 
 void launch_rerank(const float *Xp, int64_t N, int D, int dist, const int32_t *cand_i, int C,
-                   int k, int32_t *inds, float *dists, cudaStream_t s, const int32_t *order,
-                   const TcLists &lists) {
-    const int most = C * (1 + lists.count);
-    require(most <= 1024, "rerank: too many candidates per point");
+                   int k, int32_t *inds, float *dists, cudaStream_t s, const int32_t *order) {
+    require(C <= 1024, "rerank: too many candidates per point");
     const int warps = 4;
-    const size_t smem = (size_t)warps * most * 8;
+    const size_t smem = (size_t)warps * C * 8;
     const unsigned grid = ceil_div(N, warps);
     // The shared-memory attribute is set on every launch (per device; no
     // cached flag shared between host threads).
     auto go = [&](auto kernel) {
         NCVIS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         NCVIS_LAUNCH(kernel, grid, warps * 32, smem, s, Xp, N, D, dist, cand_i, C, k, inds, dists,
-                     order, lists);
+                     order);
     };
-    auto by_width = [&](auto more) {
-        constexpr bool kLists = decltype(more)::value;
-        switch ((D + 31) / 32) {
-            case 1: go(rerank_rows<1, kLists>); break;
-            case 2: go(rerank_rows<2, kLists>); break;
-            case 3: go(rerank_rows<3, kLists>); break;
-            case 4: go(rerank_rows<4, kLists>); break;
-            default: go(rerank_rows<0, kLists>);
-        }
-    };
-    if (lists.count > 0)
-        by_width(std::true_type());
-    else
-        by_width(std::false_type());
+    switch ((D + 31) / 32) {
+        case 1: go(rerank_rows<1>); break;
+        case 2: go(rerank_rows<2>); break;
+        case 3: go(rerank_rows<3>); break;
+        case 4: go(rerank_rows<4>); break;
+        default: go(rerank_rows<0>);
+    }
 }
 
 }  // namespace ncvis_gpu

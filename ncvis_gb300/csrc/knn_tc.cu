@@ -27,7 +27,8 @@
 //     (batched problems: the tile's own problem; the inverted file: the tile's
 //     probed cells), with an optional map from sorted rows back to the caller's
 //     numbering; items of several CTAs may share a query tile, each writing a
-//     list of its own (sweep_items: the last wave of one problem's tiles);
+//     list of its own, with its scores, of which the best are kept afterwards
+//     (sweep_items, merge_lists: the last wave of one problem's tiles);
 //   * squared L2 with D <= 126 folds the candidate norms into the product:
 //     candidates come from a second BF16 copy whose columns D, D + 1 hold
 //     -|c|^2 / 2 as a BF16 high and low part, the queries' copy 1, 1 there, so
@@ -355,10 +356,11 @@ __device__ __forceinline__ void flush_queue(float (&ls)[R], int32_t (&li)[R], fl
 // One item of work (TcItem): the query tile of 256 rows from row0 (rows at or
 // past qend are not outputs) against candidate rows [lo, hi); `cont`: the item
 // extends the previous item's query tile (no reload, lists carry over);
-// `more`: a later item extends this one (lists written after the last).
+// `more`: a later item extends this one (lists written after the last); `seed`:
+// the next item starts from empty lists bounded by this one's worst scores.
 struct QueryTile {
     int32_t row0, qend, lo, hi;  // N < 2^31
-    bool cont, more;
+    bool cont, more, seed;
 };
 
 __device__ __forceinline__ QueryTile work_item(const TcItem *__restrict__ work, int64_t it) {
@@ -370,6 +372,7 @@ __device__ __forceinline__ QueryTile work_item(const TcItem *__restrict__ work, 
     q.hi = w.hi;
     q.cont = (w.flags & kTcContinue) != 0;
     q.more = (w.flags & kTcMore) != 0;
+    q.seed = (w.flags & kTcSeed) != 0;
     return q;
 }
 
@@ -378,10 +381,10 @@ __device__ __forceinline__ QueryTile work_item(const TcItem *__restrict__ work, 
 // tiles' (query tile, candidate tile) pairs, an item per query tile it meets.
 __global__ void sweep_items(int64_t N, TcSweep w, int stride, int64_t *__restrict__ begin,
                             int64_t *__restrict__ end, TcItem *__restrict__ items) {
-    const int64_t b = blockIdx.x, G = w.rest_ctas;
-    const int64_t n_qt = (N + kQueryTile - 1) / kQueryTile, n_ct = (N + kCandTile - 1) / kCandTile;
-    const int64_t rest = (n_qt - w.full_qt) * n_ct;
-    const int64_t r0 = b < G ? rest * b / G : 0, r1 = b < G ? rest * (b + 1) / G : 0;
+    const int64_t b = blockIdx.x;
+    const TcRun run(N, w);
+    const int64_t n_ct = run.n_ct;
+    const int64_t r0 = b < run.G ? run.begin(b) : 0, r1 = b < run.G ? run.begin(b + 1) : 0;
     const int64_t whole = b < w.full_qt ? (w.full_qt - 1 - b) / w.ctas + 1 : 0;
     const int64_t n = whole + (r1 > r0 ? (r1 - 1) / n_ct - r0 / n_ct + 1 : 0);
     TcItem *mine = items + b * stride;
@@ -398,7 +401,7 @@ __global__ void sweep_items(int64_t N, TcSweep w, int stride, int64_t *__restric
             q.hi = (int32_t)min(N, (u1 - t * n_ct) * kCandTile);
             // The tile's first pair is in the run of the last CTA that begins
             // at or before it; the CTAs after it write the next lists.
-            q.slot = (int32_t)(b - ((t * n_ct + 1) * G - 1) / rest);
+            q.slot = (int32_t)(b - run.first_cta(t));
         }
         mine[it] = q;
     }
@@ -428,8 +431,8 @@ __global__ void __launch_bounds__(kThreads, 1)
                   const float *__restrict__ sqnorm, int ksteps, int katoms,
                   const int64_t *__restrict__ work_begin, const int64_t *__restrict__ work_end,
                   const TcItem *__restrict__ work, const int32_t *__restrict__ row_map,
-                  int32_t *__restrict__ cand_i, int32_t *__restrict__ extra, int64_t extra_row0,
-                  int extra_lists, int *__restrict__ err, long long wait_limit, int stall) {
+                  int32_t *__restrict__ cand_i, const TcLists lists, int *__restrict__ err,
+                  long long wait_limit, int stall) {
     using Shared = SharedStorage<kParts>;
     constexpr int kStages = Shared::kStages;
     constexpr int kQueue = Shared::kQueue;
@@ -727,8 +730,20 @@ __global__ void __launch_bounds__(kThreads, 1)
                     flush(ls, li, worst, qoff);
             }
             if (!ok) break;
-            if (q.more) continue;  // the next item extends this query tile
+            if (q.more && !q.seed) continue;  // the next item extends this query tile
             flush(ls, li, worst, qoff);
+            if (q.seed) {
+                // R candidates score `worst` or better, so that the row's R best do:
+                // entries from the next larger score on are as good as empty ones.
+                const float bound = ls[R - 1] < FLT_MAX ? nextafterf(ls[R - 1], FLT_MAX) : FLT_MAX;
+#pragma unroll
+                for (int t = 0; t < R; ++t) {
+                    ls[t] = bound;
+                    li[t] = -1;
+                }
+                if (live) worst = bound;
+                continue;
+            }
             // The item read again: where its lists go is not held in registers
             // over the sweep (the barrier keeps the two reads apart).
             int64_t again = it;
@@ -737,10 +752,13 @@ __global__ void __launch_bounds__(kThreads, 1)
             const int64_t grow = o.row0 + row_in_tile;
             if (grow < o.qend) {
                 const int64_t orow = row_map ? (int64_t)row_map[grow] : grow + o.out_off;
-                int32_t *out =
-                    o.slot == 0
-                        ? cand_i + orow * R
-                        : extra + ((grow - extra_row0) * extra_lists + (o.slot - 1)) * R;
+                int32_t *out = cand_i + orow * R;
+                if (lists.count > 0 && grow >= lists.row0) {
+                    const int64_t at = ((grow - lists.row0) * lists.count + o.slot) * R;
+                    out = lists.idx + at;
+#pragma unroll
+                    for (int t = 0; t < R; ++t) lists.score[at + t] = ls[t];
+                }
 #pragma unroll
                 for (int t = 0; t < R; ++t)
                     out[t] = li[t] < 0 ? -1
@@ -815,19 +833,27 @@ TcSweep plan_sweep(int64_t N, int ctas) {
     const int64_t left = n_qt - w.full_qt;
     w.ctas = ctas;
     if (left == 0) return w;
-    if (10 * left > 9 * ctas) {  // the last wave is nearly full
-        return whole_tiles(N, ctas);
-    }
-    // Runs of at least two candidate tiles and a sixth of a sweep: shorter ones
-    // give the rows more candidates to re-rank than they save.
+    // The last wave's tiles whole, in p equal runs each (of at least two candidate
+    // tiles, and a sixth of a sweep), or in ctas equal runs, which then mostly reach
+    // over two tiles and fill two sets of lists: filling one from nothing takes
+    // about as long as scanning kFill candidate tiles afterwards.  Selection in us,
+    // whole / p runs / ctas runs: 10,000 x 64 BF16 (40 tiles, p = 3) 271 / 183 / 243,
+    // 131,072 x 100 (56 left, p = 2) 4,255 / 3,918 / 4,081, 20,000 x 100 (79) 386 /
+    // - / 420, 32,768 x 100 (128) 487 / - / 885, 60,013 x 100 FP32 (83 left) 2,082 / -
+    // / 1,838, 30,000 x 100 FP32 (118) 595 / - / 650.  A last wave more than three
+    // quarters full stays whole: 500,000 x 64 (130 left) 39.1 ms whole, 40.4 in runs
+    // (300,000 x 100, 108 left, 18.8 and 18.7).
+    constexpr int64_t kFill = 200;
     const int64_t rest = left * n_ct;
-    w.rest_ctas = (int)std::max<int64_t>(1, std::min<int64_t>({ctas, rest / 2, 6 * left}));
+    const int64_t p = std::max<int64_t>(1, std::min<int64_t>({ctas / left, 6, n_ct / 2}));
+    int64_t G = p * left, cost = n_ct / p + kFill;
+    if (ctas > G && 4 * left < 3 * ctas && ctas <= 6 * left && ctas <= rest / 2 && rest / ctas + 2 * kFill < cost) G = ctas;
+    if (G == left) return whole_tiles(N, ctas);
+    w.rest_ctas = (int)G;
     if (w.full_qt == 0) w.ctas = w.rest_ctas;
-    const int64_t G = w.rest_ctas;
-    for (int64_t t = 0; t < left; ++t) {
-        const int64_t first = ((t * n_ct + 1) * G - 1) / rest, last = ((t + 1) * n_ct * G - 1) / rest;
-        w.lists = std::max<int>(w.lists, (int)(last - first + 1));
-    }
+    const TcRun run(N, w);
+    for (int64_t t = 0; t < left; ++t)
+        w.lists = std::max<int>(w.lists, (int)(run.last_cta(t) - run.first_cta(t) + 1));
     w.split_rows = N - w.full_qt * kQueryTile;
     return w;
 }
@@ -839,14 +865,79 @@ TcSweep whole_tiles(int64_t N, int ctas) {
     return w;
 }
 
-size_t sweep_work_bytes(int64_t N, const TcSweep &w) {
-    return 16 * (((size_t)w.ctas + 1) / 2 * 2) + sizeof(TcItem) * (size_t)w.ctas * sweep_stride(N, w);
+namespace {
+
+size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
+
+// The best `keep` of a split row's lists, a warp a row: every entry's place is its
+// own in its list and, by a binary search in each other one, the number of entries
+// before it there (equal scores: those of the lists before its own).  Bound by the
+// latency of the searches' steps: 14,336 rows x 2 lists 9 us, 10,000 x 3 11 us, 6,144
+// x 7 22 us; re-ranking all the lists instead took 100 us more at 10,000 x 3.
+template <int R>
+__global__ void __launch_bounds__(128) merge_lists(int64_t N, TcSweep w, TcLists lists, int keep,
+                                                   const int32_t *__restrict__ order,
+                                                   int32_t *__restrict__ cand_i) {
+    extern __shared__ float scores[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t row = lists.row0 + (int64_t)blockIdx.x * (blockDim.x >> 5) + warp;
+    if (row >= N) return;
+    const TcRun run(N, w);
+    const int64_t tile = row / kQueryTile - w.full_qt;
+    const int n = (int)(run.last_cta(tile) - run.first_cta(tile)) + 1;
+    const int64_t at = (row - lists.row0) * lists.count * R;
+    float *sc = scores + (size_t)warp * lists.count * R;
+    for (int c = lane; c < n * R; c += 32) sc[c] = lists.score[at + c];
+    __syncwarp();
+    int32_t *out = cand_i + (order ? (int64_t)order[row] : row) * keep;
+    for (int c = lane; c < n * R; c += 32) {
+        const int a = c / R;
+        const float x = sc[c];
+        int place = c % R;
+        for (int b = 0; b < n; ++b) {
+            if (b == a) continue;
+            const float *y = sc + b * R;
+            int before = 0;
+#pragma unroll
+            for (int step = R; step > 0; step >>= 1) {
+                const int i = before + step - 1;
+                if (i < R && (b < a ? y[i] <= x : y[i] < x)) before += step;
+            }
+            place += before;
+        }
+        if (place < keep) out[place] = lists.idx[at + c];
+    }
+    for (int c = n * R + lane; c < keep; c += 32) out[c] = -1;
 }
 
-TcWork launch_sweep_work(int64_t N, const TcSweep &w, void *workspace, cudaStream_t s) {
+}  // namespace
+
+size_t sweep_lists_bytes(const TcSweep &w, int R) {
+    return w.lists > 1 ? 2 * align256(sizeof(int32_t) * (size_t)w.split_rows * w.lists * R) : 0;
+}
+
+size_t sweep_bytes(int64_t N, const TcSweep &w, int R) {
+    return sweep_lists_bytes(w, R) +
+           align256(16 * (((size_t)w.ctas + 1) / 2 * 2) +
+                    sizeof(TcItem) * (size_t)w.ctas * sweep_stride(N, w));
+}
+
+TcLists sweep_lists(int64_t N, const TcSweep &w, int R, void *workspace) {
+    TcLists l;
+    if (w.lists <= 1) return l;
+    l.count = w.lists;
+    l.row0 = N - w.split_rows;
+    l.idx = (int32_t *)workspace;
+    l.score = (float *)((char *)workspace + sweep_lists_bytes(w, R) / 2);
+    return l;
+}
+
+TcWork launch_sweep_work(int64_t N, const TcSweep &w, int R, void *workspace, cudaStream_t s) {
     TcWork work;
     work.ctas = w.ctas;
-    int64_t *begin = (int64_t *)workspace, *end = begin + (w.ctas + 1) / 2 * 2;
+    work.lists = sweep_lists(N, w, R, workspace);
+    int64_t *begin = (int64_t *)((char *)workspace + sweep_lists_bytes(w, R));
+    int64_t *end = begin + (w.ctas + 1) / 2 * 2;
     TcItem *items = (TcItem *)(end + (w.ctas + 1) / 2 * 2);
     NCVIS_LAUNCH(sweep_items, (unsigned)w.ctas, 32, 0, s, N, w, sweep_stride(N, w), begin, end,
                  items);
@@ -854,6 +945,19 @@ TcWork launch_sweep_work(int64_t N, const TcSweep &w, void *workspace, cudaStrea
     work.end = end;
     work.items = items;
     return work;
+}
+
+void launch_merge_lists(int64_t N, const TcSweep &w, const TcLists &lists, int R, int keep,
+                        const int32_t *order, int32_t *cand_i, cudaStream_t s) {
+    if (lists.count == 0) return;
+    require(R == 32 || R == 64, "knn: lists of 32 or 64 candidates", kInternal);
+    const int warps = 4;
+    const size_t smem = sizeof(float) * warps * lists.count * R;  // at most 8 lists: 8 KB
+    const unsigned grid = (unsigned)ceil_div(N - lists.row0, warps);
+    if (R == 32)
+        NCVIS_LAUNCH(merge_lists<32>, grid, warps * 32, smem, s, N, w, lists, keep, order, cand_i);
+    else
+        NCVIS_LAUNCH(merge_lists<64>, grid, warps * 32, smem, s, N, w, lists, keep, order, cand_i);
 }
 
 bool knn_tc_supported(int D, int R) { return D >= 1 && D <= 64 * kMaxAtoms && (R == 32 || R == 64); }
@@ -890,8 +994,7 @@ void launch_select(const CUtensorMap &map, const CUtensorMap &map_c, const TcPar
         NCVIS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         (int)smem));
         NCVIS_LAUNCH(kernel, grid, kThreads, smem, s, map, map_c, parts, sqnorm, ksteps, katoms,
-                     work.begin, work.end, work.items, work.map, cand_i, work.lists.extra,
-                     work.lists.row0, work.lists.count, timeout_flag,
+                     work.begin, work.end, work.items, work.map, cand_i, work.lists, timeout_flag,
                      plan.wait_cycles > 0 ? plan.wait_cycles : kWaitCycles, plan.stall ? 1 : 0);
     };
     constexpr size_t one = sizeof(SharedStorage<1>), two = sizeof(SharedStorage<2>);

@@ -47,23 +47,13 @@ void launch_knn_select_f32(const float *Xp, const float *sqnorm, int64_t N, int 
                            const KnnPlan &plan, int32_t *cand_i, cudaStream_t s,
                            const Segments &seg = Segments());
 int knn_f32_query_tile();
-// Lists beyond a row's first one, where several items of a tensor-core launch
-// share a query tile: rows (in the launch's numbering) from row0 on have
-// `count` more lists at extra[(row - row0) * count * R], R candidates each; -1
-// marks an empty slot.
-struct TcLists {
-    int32_t *extra = nullptr;
-    int64_t row0 = 0;
-    int count = 0;
-};
 // Exact distances of the candidates, top k+1 by (distance, index), smallest
 // dropped, k written in descending order: inds/dists [N, k].  `order` (a
 // permutation of the rows, or nullptr) is the order the rows are processed
-// in; the result does not depend on it.  `lists`: further lists of C
-// candidates of the rows from lists.row0 on (in that order).
+// in; the result does not depend on it.
 void launch_rerank(const float *Xp, int64_t N, int D, int dist, const int32_t *cand_i, int C,
                    int k, int32_t *inds, float *dists, cudaStream_t s,
-                   const int32_t *order = nullptr, const TcLists &lists = TcLists());
+                   const int32_t *order = nullptr);
 
 // ---- K2 BF16 tensor-core candidate selection ---------------------------------
 struct KnnTcPlan {
@@ -86,13 +76,26 @@ bool knn_tc_supported(int D, int R);
 // the previous item's query tile (same row0: the tile is not reloaded and its
 // lists carry over); kTcMore: a later item continues this one (the lists are
 // written after the last item of a query tile).
+// kTcSeed (with kTcMore): what the items so far found leaves the lists, which stay
+// empty but only take scores up to their worst.
 constexpr int kTcContinue = 1;
 constexpr int kTcMore = 2;
+constexpr int kTcSeed = 4;
 struct alignas(16) TcItem {
     int32_t row0, qend, lo, hi;
     int32_t out_off, flags;
     int32_t slot;  // which of the query tile's lists the item writes (TcLists)
     int32_t pad;
+};
+// The lists of the rows whose query tiles several items share (`count` > 0): rows
+// (in the launch's numbering) from row0 on have a list per slot, R candidates and
+// their scores at [((row - row0) * count + slot) * R], best first; -1 marks an
+// empty entry, with the largest score.
+struct TcLists {
+    int32_t *idx = nullptr;
+    float *score = nullptr;
+    int64_t row0 = 0;
+    int count = 0;
 };
 // Work of one launch (device arrays): CTA b takes items[begin[b] .. end[b]).
 struct TcWork {
@@ -105,16 +108,36 @@ struct TcWork {
 // How the query tiles of one problem of N rows are spread over at most `ctas`
 // CTAs: the first full_qt whole and round-robin, the rest in equal runs of
 // candidate tiles over the first rest_ctas, so that the last wave fills the
-// GPU; rows of the last `split_rows` have up to `lists` lists.
+// GPU; rows of the last `split_rows` have up to `lists` lists (whole tiles: one,
+// and no split rows).
 struct TcSweep {
     int64_t full_qt = 0, split_rows = 0;
     int ctas = 0, rest_ctas = 1, lists = 1;
 };
 TcSweep plan_sweep(int64_t N, int ctas);
 TcSweep whole_tiles(int64_t N, int ctas);  // every query tile whole
-// Its work list, written by a kernel into `workspace` (16-byte aligned).
-size_t sweep_work_bytes(int64_t N, const TcSweep &w);
-TcWork launch_sweep_work(int64_t N, const TcSweep &w, void *workspace, cudaStream_t s);
+// Its work list, written by a kernel, and the split rows' lists of R candidates,
+// both in `workspace` (256-byte aligned, sweep_bytes).
+size_t sweep_bytes(int64_t N, const TcSweep &w, int R);
+TcWork launch_sweep_work(int64_t N, const TcSweep &w, int R, void *workspace, cudaStream_t s);
+TcLists sweep_lists(int64_t N, const TcSweep &w, int R, void *workspace);
+size_t sweep_lists_bytes(const TcSweep &w, int R);
+// The candidate tiles [first, last) of split query tile t (from full_qt on) that
+// CTA b's run of them covers, and the slot of its list, for the CTAs b of
+// [tile_first_cta, tile_last_cta].
+struct TcRun {
+    int64_t n_ct, G, rest;
+    __host__ __device__ TcRun(int64_t N, const TcSweep &w)
+        : n_ct((N + 127) / 128), G(w.rest_ctas), rest(((N + 255) / 256 - w.full_qt) * n_ct) {}
+    __host__ __device__ int64_t begin(int64_t b) const { return rest * b / G; }  // in pairs of tiles
+    __host__ __device__ int64_t first_cta(int64_t t) const { return ((t * n_ct + 1) * G - 1) / rest; }
+    __host__ __device__ int64_t last_cta(int64_t t) const { return ((t + 1) * n_ct * G - 1) / rest; }
+};
+// The best `keep` candidates of every split row's lists (by score, then by list)
+// into cand_i[row * keep], -1 behind them where there are fewer; rows are
+// order[row] when `order` is given.
+void launch_merge_lists(int64_t N, const TcSweep &w, const TcLists &lists, int R, int keep,
+                        const int32_t *order, int32_t *cand_i, cudaStream_t s);
 void launch_knn_select_tc(const __nv_bfloat16 *Xb, const float *sqnorm, int64_t N,
                           const KnnTcPlan &plan, int dist, int32_t *cand_i, int *timeout_flag,
                           cudaStream_t s, const TcWork &work, const __nv_bfloat16 *Xc = nullptr);
@@ -169,7 +192,8 @@ void run_knn_tc_ordered(const float *Xp, const __nv_bfloat16 *Xb, const __nv_bfl
                         int64_t N, int D, const KnnTcPlan &tp, int dist, const KnnOrderPlan &op,
                         uint64_t seed, int32_t *cand_i, int *timeout_flag, cudaStream_t s,
                         void *workspace = nullptr, size_t workspace_bytes = 0,
-                        cudaEvent_t sweep_start = nullptr, const int32_t **cell_order = nullptr);
+                        cudaEvent_t sweep_start = nullptr, const int32_t **cell_order = nullptr,
+                        void *list_memory = nullptr);
 
 // Queries from Q (nq rows) against candidates from Cm (nc rows), both bf16
 // [rows, plan.ldb]; c_sqnorm: candidate squared norms (used for squared L2
