@@ -671,6 +671,7 @@ void run_knn_tc_ordered(const float *Xp, const __nv_bfloat16 *Xb, const __nv_bfl
     }
     TcWork work = upload(w, cells.perm, arena);
     work.lists = sweep_lists(N, sweep, tp.R, list_memory);
+    work.fill = N < kFillMaxRows;
     if (sweep_start) NCVIS_CUDA(cudaEventRecord(sweep_start, s));
     launch_knn_select_tc_pair(cells.Xs, N, fold ? cells.Xcs : cells.Xs, N, nullptr, tp, true,
                               cand_i, timeout_flag, s, work);

@@ -20,7 +20,8 @@
 //     a group of 4 columns that holds a qualifying candidate goes whole to a
 //     per-row queue in shared memory; when a queue is full the warp looks all its
 //     rows' queues over and inserts what qualifies into the rows'
-//     register-resident sorted lists in lockstep rounds;
+//     register-resident sorted lists in lockstep rounds (the first tiles of a
+//     short sweep: single candidates, merged in 16 at a time by a network);
 //   * a CTA takes items from its own work list: an item is a query tile's rows
 //     and one candidate range (masked at both ends), and may continue the
 //     previous item's tile, so one tile's lists are built over several ranges
@@ -53,6 +54,7 @@
 #include <algorithm>
 #include <cfloat>
 #include <string>
+#include <type_traits>
 
 #include "common.cuh"
 #include "stages.cuh"
@@ -69,18 +71,23 @@ constexpr int kThreads = 352;
 constexpr int kEpiWarp0 = 2;
 constexpr int kEpiWarps = 8;
 constexpr int kMmaWarp1 = 10;  // issues the second query half's MMAs (warp 1 the first)
-constexpr int kEpiThreads = kEpiWarps * 32;
 constexpr uint32_t kTmemCols = 512;
 constexpr int kLowLowSteps = 2;  // K steps up to which the low parts' product is taken too
 constexpr long long kWaitCycles = 4000000000LL;  // ~2 s at 2 GHz
 
-// One queued group of 4 accumulator columns of every row: the values and the
+// One queued group of 4 accumulator columns of a warp's rows: the values and the
 // candidate index of the first column.
 constexpr int kGroup = 4;
 constexpr uint32_t kFlushAt = 4;  // slots past which a queue is flushed after a tile
+// Pending entries past which lists are merged after a tile: 10,000 x 64 144, 134, 129 us
+// with 5, 8 and 11.
+constexpr uint32_t kMergeAt = 11;
+// Candidate tiles that fill a list: 131,072 x 100 4.53, 4.55 and 4.69 ms with 16, 32 and
+// 64, 60,013 x 100 FP32 1.76, 1.78 and 1.86.
+constexpr int kFillTiles = 16;
 struct QueueSlot {
-    float4 v[kEpiThreads];
-    int32_t first[kEpiThreads];
+    float4 v[32];
+    int32_t first[32];
 };
 
 // Shared memory by the number of parts a row is held in: the query tile takes
@@ -95,7 +102,7 @@ struct SharedStorage {
     // 1024-byte aligned tiles first (128B swizzle atoms repeat every 1024 B).
     uint8_t a[2][kParts][kMaxAtoms][kAtomBytes];
     uint8_t b[kStages][kMaxAtoms][kAtomBytes];
-    QueueSlot queue[kQueue];
+    QueueSlot queue[kEpiWarps][kQueue];  // each warp's own: it may hold entries instead
     uint64_t full[kStages];
     uint64_t empty[kStages];
     uint64_t a_full, a_empty;
@@ -267,6 +274,20 @@ __device__ __forceinline__ float tree_reduce(const float (&a)[n]) {
     }
 }
 
+__device__ __forceinline__ uint32_t ld_shared(uint32_t a) {
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ float4 ld_shared_v4(uint32_t a) {
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "r"(a)
+                 : "memory");
+    return v;
+}
+
 // Insert (v, vi) into the ascending list (ls, li) of R entries, dropping the
 // largest.  Every slot's new entry comes from the old ones alone (its own, its
 // left neighbour's or the new value, by two compares), so the R slots are
@@ -313,7 +334,7 @@ __device__ __forceinline__ void queue_group(uint32_t queue_v, uint32_t queue_i, 
 // that has one left.
 template <int R, bool kIP, int kQueue>
 __device__ __forceinline__ void flush_queue(float (&ls)[R], int32_t (&li)[R], float &worst,
-                                            uint32_t &off, const QueueSlot *queue, int etid) {
+                                            uint32_t &off, uint32_t queue_v, uint32_t queue_i) {
     constexpr uint32_t kSlot = sizeof(QueueSlot);
     const uint32_t most = __reduce_max_sync(0xffffffffu, off);
     uint32_t marks[2] = {0u, 0u};  // slot b's columns: bits 4 (b % 8) .. of marks[b / 8]
@@ -321,7 +342,7 @@ __device__ __forceinline__ void flush_queue(float (&ls)[R], int32_t (&li)[R], fl
     for (int b = 0; b < kQueue; ++b) {
         if (b * kSlot >= most) break;
         if (b * kSlot < off) {
-            const float4 x = queue[b].v[etid];
+            const float4 x = ld_shared_v4(queue_v + b * kSlot);
             const float w[kGroup] = {x.x, x.y, x.z, x.w};
 #pragma unroll
             for (int j = 0; j < kGroup; ++j)
@@ -331,7 +352,7 @@ __device__ __forceinline__ void flush_queue(float (&ls)[R], int32_t (&li)[R], fl
 #pragma unroll 1
     while (__any_sync(0xffffffffu, (marks[0] | marks[1]) != 0u)) {
         if ((marks[0] | marks[1]) != 0u) {
-            int pos;
+            uint32_t pos;
             if (marks[0] != 0u) {
                 pos = __ffs(marks[0]) - 1;
                 marks[0] &= marks[0] - 1u;
@@ -339,12 +360,14 @@ __device__ __forceinline__ void flush_queue(float (&ls)[R], int32_t (&li)[R], fl
                 pos = 31 + __ffs(marks[1]);
                 marks[1] &= marks[1] - 1u;
             }
-            const QueueSlot &slot = queue[pos >> 2];
-            const int j = pos & 3;
-            const float raw = reinterpret_cast<const float *>(&slot.v[etid])[j];
+            const uint32_t slot = (pos >> 2) * kSlot, j = pos & 3;
+            const float raw = __uint_as_float(ld_shared(queue_v + slot + 4 * j));
+            uint32_t first = 0u;  // loaded ahead where there are registers for it
+            if (R <= 32) first = ld_shared(queue_i + slot);
             const float x = kIP ? -raw : raw;
             if (x < worst) {
-                list_push<R>(ls, li, x, slot.first[etid] + j);
+                if (R > 32) first = ld_shared(queue_i + slot);
+                list_push<R>(ls, li, x, (int32_t)(first + j));
                 worst = ls[R - 1];
             }
         }
@@ -353,14 +376,141 @@ __device__ __forceinline__ void flush_queue(float (&ls)[R], int32_t (&li)[R], fl
     __syncwarp();
 }
 
+// ---- the filling of a list of 32 --------------------------------------------------
+// While a row's list fills, its qualifying candidates wait in shared memory, an entry
+// (raw score, index) each, and are merged into the list up to kPending at a time: a
+// sorting network over the pending ones, then a bitonic merge, the same instructions
+// in every lane.  Inserting them one by one in lockstep rounds (flush_queue) takes
+// 180 instructions a round, and the fullest of a warp's 32 rows sets the number of
+// rounds: about 570 in the first 80 tiles, where the average row inserts 270.  Later,
+// when a tile brings a few rows one candidate each, queueing whole column groups
+// and inserting is the faster way (131,072 x 100 in the caller's order 4.6 ms, 5.4 with
+// merging all along), as it is for lists of 64, whose networks do not fit the registers.
+// The filling is the kernel's form kFill.  Selection without and with it: 1,000 x 32
+// 68 and 43 us, 10,000 x 64 175 and 133, 48 problems of 200 to 9,000 1,717 and 1,430,
+// 131,072 x 100 3,800 and 3,600.  Sweeps over kFillMaxRows rows or more (TcWork::fill)
+// go without: its loop beside theirs costs them more than the filling gives (whole
+// calls without and with it: 150,000 x 100 5.98 and 5.92 ms, 150,000 x 32 4.90 and
+// 5.08, 250,000 x 64 11.4 and 12.0, 500,000 x 64 38.0 and 41.5).
+constexpr int kPending = 16;
+
+// Orders entries a and b by score, equal scores by index (the order they are met
+// in, but for a sweep that wraps around).
+__device__ __forceinline__ bool entry_less(float av, int32_t ai, float bv, int32_t bi) {
+    return (av < bv) | ((av == bv) & (ai < bi));
+}
+__device__ __forceinline__ void order_pair(float &av, int32_t &ai, float &bv, int32_t &bi) {
+    const bool swap = entry_less(bv, bi, av, ai);
+    const float lv = swap ? bv : av, hv = swap ? av : bv;
+    const int32_t li = swap ? bi : ai, hi = swap ? ai : bi;
+    av = lv, ai = li, bv = hv, bi = hi;
+}
+
+// Queues the 4 columns v[0..4) of a row, the first being candidate `first`: those
+// that beat the row's worst (for raw inner products: `limit` is its negative) take
+// the entry at byte offset `off`, which moves on; an entry is stored where it lies
+// within the first `cap` bytes (predicated stores, no branch).
+template <bool kIP>
+__device__ __forceinline__ void push_group(uint32_t pend_v, uint32_t pend_i, uint32_t &off,
+                                           uint32_t cap, float limit, const float *v,
+                                           int32_t first) {
+    constexpr int kEntry = 32 * 4;
+#pragma unroll
+    for (int j = 0; j < kGroup; ++j) {
+        if constexpr (kIP)
+            asm volatile(
+                "{\n\t.reg .pred p, q;\n\t.reg .u32 a, b;\n\t"
+                "setp.gt.f32 p, %1, %2;\n\t"
+                "setp.lt.and.u32 q, %0, %6, p;\n\t"
+                "add.u32 a, %3, %0;\n\t"
+                "add.u32 b, %4, %0;\n\t"
+                "@q st.shared.f32 [a], %1;\n\t"
+                "@q st.shared.s32 [b], %5;\n\t"
+                "@p add.u32 %0, %0, %7;\n\t}"
+                : "+r"(off)
+                : "f"(v[j]), "f"(limit), "r"(pend_v), "r"(pend_i), "r"(first + j), "r"(cap),
+                  "n"(kEntry)
+                : "memory");
+        else
+            asm volatile(
+                "{\n\t.reg .pred p, q;\n\t.reg .u32 a, b;\n\t"
+                "setp.lt.f32 p, %1, %2;\n\t"
+                "setp.lt.and.u32 q, %0, %6, p;\n\t"
+                "add.u32 a, %3, %0;\n\t"
+                "add.u32 b, %4, %0;\n\t"
+                "@q st.shared.f32 [a], %1;\n\t"
+                "@q st.shared.s32 [b], %5;\n\t"
+                "@p add.u32 %0, %0, %7;\n\t}"
+                : "+r"(off)
+                : "f"(v[j]), "f"(limit), "r"(pend_v), "r"(pend_i), "r"(first + j), "r"(cap),
+                  "n"(kEntry)
+                : "memory");
+    }
+}
+
+// Batcher's odd-even merge sort of the pending entries, from its step (p, k) on.
+template <int p, int k>
+__device__ __forceinline__ void sort_pending(float (&pv)[kPending], int32_t (&pi)[kPending]) {
+#pragma unroll
+    for (int x = k % p; x + k < kPending; ++x)
+        if ((x - k % p) / k % 2 == 0 && x / (2 * p) == (x + k) / (2 * p))
+            order_pair(pv[x], pi[x], pv[x + k], pi[x + k]);
+    if constexpr (k > 1)
+        sort_pending<p, k / 2>(pv, pi);
+    else if constexpr (2 * p < kPending)
+        sort_pending<2 * p, 2 * p>(pv, pi);
+}
+
+// The bitonic merge of R entries, from distance st on.
+template <int st, int R>
+__device__ __forceinline__ void merge_bitonic(float (&ls)[R], int32_t (&li)[R]) {
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+        if (!(i & st)) order_pair(ls[i], li[i], ls[i + st], li[i + st]);
+    if constexpr (st > 1) merge_bitonic<st / 2, R>(ls, li);
+}
+
+// The row's `off` bytes of pending entries (at most kEntries) into its ascending
+// list of 32: the pending ones sorted, the smaller of list entry 31 - t and pending
+// entry t for the 16 last places (the 32 best of both, a bitonic sequence), merged.
+template <int R, bool kIP, int kEntries>
+__device__ __forceinline__ void merge_pending(float (&ls)[R], int32_t (&li)[R], float &worst,
+                                              uint32_t &off, uint32_t pend_v,
+                                              uint32_t pend_i) {
+    static_assert(kEntries <= kPending, "pending entries");
+    constexpr uint32_t kEntry = 32 * 4;
+    float pv[kPending];
+    int32_t pi[kPending];
+#pragma unroll
+    for (int b = 0; b < kPending; ++b) {
+        pv[b] = FLT_MAX;
+        pi[b] = -1;
+        if (b < kEntries && b * kEntry < off) {
+            const float raw = __uint_as_float(ld_shared(pend_v + b * kEntry));
+            pv[b] = kIP ? -raw : raw;
+            pi[b] = (int32_t)ld_shared(pend_i + b * kEntry);
+        }
+    }
+    sort_pending<1, 1>(pv, pi);
+#pragma unroll
+    for (int t = 0; t < kPending; ++t) {
+        const int at = R - 1 - t;
+        const bool take = entry_less(pv[t], pi[t], ls[at], li[at]);
+        ls[at] = take ? pv[t] : ls[at];
+        li[at] = take ? pi[t] : li[at];
+    }
+    merge_bitonic<R / 2>(ls, li);
+    if (off > 0u) worst = ls[R - 1];
+    off = 0u;
+}
+
 // One item of work (TcItem): the query tile of 256 rows from row0 (rows at or
 // past qend are not outputs) against candidate rows [lo, hi); `cont`: the item
 // extends the previous item's query tile (no reload, lists carry over);
-// `more`: a later item extends this one (lists written after the last); `seed`:
-// the next item starts from empty lists bounded by this one's worst scores.
+// `more`: a later item extends this one (lists written after the last).
 struct QueryTile {
     int32_t row0, qend, lo, hi;  // N < 2^31
-    bool cont, more, seed;
+    bool cont, more;
 };
 
 __device__ __forceinline__ QueryTile work_item(const TcItem *__restrict__ work, int64_t it) {
@@ -372,7 +522,6 @@ __device__ __forceinline__ QueryTile work_item(const TcItem *__restrict__ work, 
     q.hi = w.hi;
     q.cont = (w.flags & kTcContinue) != 0;
     q.more = (w.flags & kTcMore) != 0;
-    q.seed = (w.flags & kTcSeed) != 0;
     return q;
 }
 
@@ -424,7 +573,7 @@ struct TcParts {
     int32_t q[2], c[2];
 };
 
-template <int R, bool kIP, int kParts>
+template <int R, bool kIP, int kParts, bool kFill>
 __global__ void __launch_bounds__(kThreads, 1)
     knn_select_tc(const __grid_constant__ CUtensorMap tmap,
                   const __grid_constant__ CUtensorMap tmap_c, const TcParts parts,
@@ -441,7 +590,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                                             ~(uintptr_t)1023);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t n_items = work_end[blockIdx.x] - work_begin[blockIdx.x];
-    work += work_begin[blockIdx.x];
+    const TcItem *const mine = work + work_begin[blockIdx.x];
     const uint32_t a_bytes = 2u * kParts * katoms * kAtomBytes;
     const uint32_t b_bytes = (uint32_t)katoms * kAtomBytes;
 
@@ -488,7 +637,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         uint32_t a_parity = 0;
         if (stall) mbar_wait(s.abort, &s.never, 0, err, 7, wait_limit);
         for (int64_t it = 0; it < n_items && !s.abort; ++it) {
-            const QueryTile q = work_item(work, it);
+            const QueryTile q = work_item(mine, it);
             if (!q.cont) {
                 if (!mbar_wait(s.abort, &s.a_empty, a_phase ^ 1, err, 1, wait_limit)) break;
                 mbar_expect_tx(&s.a_full, a_bytes);
@@ -537,7 +686,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         uint32_t phase = 0, a_phase = 0, acc_phase = 0;
         int acc = 0;
         for (int64_t it = 0; it < n_items && !s.abort; ++it) {
-            const QueryTile q = work_item(work, it);
+            const QueryTile q = work_item(mine, it);
             if (!q.cont) {
                 if (!mbar_wait(s.abort, &s.a_full, a_phase, err, 3, wait_limit)) break;
                 a_phase ^= 1;
@@ -586,17 +735,22 @@ __global__ void __launch_bounds__(kThreads, 1)
         // ---------------------------------------------------------- epilogue
         const int h = (warp - kEpiWarp0) >> 2;
         const int quad = warp & 3;
-        const int etid = threadIdx.x - kEpiWarp0 * 32;
         const int row_in_tile = h * 128 + quad * 32 + lane;
         // Accumulator columns per tcgen05.ld: 32 with 32-entry lists; 64-entry
         // lists leave registers for 16.
         constexpr int kC = R <= 32 ? 32 : 16;
         constexpr int kG = kC / kGroup;  // column groups per load
+        // A list's first tiles (lists of 32): its row's pending candidates, else
+        // queued column groups, in the same memory.
+        constexpr bool kMerge = R == 32 && kFill;
+        constexpr int kFits = sizeof(s.queue[0]) / (8 * 32);
+        constexpr int kEntries = kFits < kPending ? kFits : kPending;
         constexpr uint32_t kQueueBytes = kQueue * sizeof(QueueSlot);
-        const uint32_t queue_v = smem_u32(&s.queue[0].v[etid]);
-        const uint32_t queue_i = smem_u32(&s.queue[0].first[etid]);
+        constexpr uint32_t kPendBytes = kEntries * 32 * 4;
+        const uint32_t queue_v = smem_u32(&s.queue[warp - kEpiWarp0][0].v[lane]);
+        const uint32_t queue_i = smem_u32(&s.queue[warp - kEpiWarp0][0].first[lane]);
         auto flush = [&](float (&ls)[R], int32_t (&li)[R], float &worst, uint32_t &off) {
-            flush_queue<R, kIP, kQueue>(ls, li, worst, off, s.queue, etid);
+            flush_queue<R, kIP, kQueue>(ls, li, worst, off, queue_v, queue_i);
         };
         uint32_t acc_phase = 0;
         int acc = 0;
@@ -604,11 +758,11 @@ __global__ void __launch_bounds__(kThreads, 1)
         int32_t li[R];
         float worst = FLT_MAX;
         uint32_t qoff = 0u;
-        for (int64_t it = 0; it < n_items; ++it) {
+        const int32_t it_end = (int32_t)work_end[blockIdx.x];
+        for (int32_t it = (int32_t)work_begin[blockIdx.x]; it < it_end; ++it) {
             // Lanes read the abort flag at different times: the warp stops as one.
             if (__any_sync(0xffffffffu, s.abort != 0)) break;
             const QueryTile q = work_item(work, it);
-            const bool live = q.row0 + row_in_tile < q.qend;
             if (!q.cont) {
 #pragma unroll
                 for (int t = 0; t < R; ++t) {
@@ -616,140 +770,190 @@ __global__ void __launch_bounds__(kThreads, 1)
                     li[t] = -1;
                 }
                 // Nothing qualifies in rows that are not outputs.
-                worst = live ? FLT_MAX : -INFINITY;
+                worst = q.row0 + row_in_tile < q.qend ? FLT_MAX : -INFINITY;
                 qoff = 0u;
             }
-            bool ok = true;
-            for (int64_t ct = q.lo / kCandTile; ct * kCandTile < q.hi; ++ct) {
-                const bool got = mbar_wait(s.abort, &s.acc_full[acc][h], acc_phase, err, 6, wait_limit);
-                if (!__all_sync(0xffffffffu, got)) {
-                    ok = false;
-                    break;
-                }
-                tmem_fence_after();
-                const int64_t c0 = ct * kCandTile;
-                // A tile reaching outside [lo, hi): its outside columns are masked.
-                const bool tail = c0 < q.lo || c0 + kCandTile > q.hi;
+            // Candidate tiles [ct, ct_end), the first ones of a list (kFilling) or later
+            // ones; false if a wait ran out.  Two loops: in one loop with a branch for
+            // each the later tiles took 25% longer.
+            auto scan = [&](auto filling, int32_t ct, const int32_t ct_end) {
+                constexpr bool kFilling = decltype(filling)::value;
+                for (; ct < ct_end; ++ct) {
+                    const bool got = mbar_wait(s.abort, &s.acc_full[acc][h], acc_phase, err, 6, wait_limit);
+                    if (!__all_sync(0xffffffffu, got)) return false;
+                    tmem_fence_after();
+                    const int32_t c0 = ct * kCandTile;
+                    // A tile reaching outside [lo, hi): its outside columns are masked.
+                    const bool tail = c0 < q.lo || c0 + kCandTile > q.hi;
 #pragma unroll 1
-                for (int chunk = 0; chunk < kCandTile / kC; ++chunk) {
-                    float v[kC];
-                    __syncwarp();
-                    tmem_ld(tmem + ((uint32_t)(quad * 32) << 16) +
-                                (uint32_t)(acc * 256 + h * 128 + chunk * kC),
-                            v);
-                    if (chunk == kCandTile / kC - 1) {
-                        // The tile's last columns are in registers: the
-                        // accumulator goes back to the MMA warp before their
-                        // scan, so the next MMAs into it start meanwhile.
-                        tmem_fence_before();
+                    for (int chunk = 0; chunk < kCandTile / kC; ++chunk) {
+                        float v[kC];
                         __syncwarp();
-                        if (lane == 0) mbar_arrive(&s.acc_empty[acc][h]);
-                    }
-                    const int64_t cb = c0 + chunk * kC;
-                    // Scores, lower is better: |c|^2 - 2<q,c> (squared L2) or
-                    // -<q,c> (kept as +<q,c>, compared against -worst).
-                    if constexpr (!kIP) {
-                        // The chunk's candidate norms, the same for every lane:
-                        // 16-byte loads where the chunk lies inside the rows.
-                        if (cb >= q.lo && cb + kC <= q.hi) {
+                        tmem_ld(tmem + ((uint32_t)(quad * 32) << 16) +
+                                    (uint32_t)(acc * 256 + h * 128 + chunk * kC),
+                                v);
+                        if (chunk == kCandTile / kC - 1) {
+                            // The tile's last columns are in registers: the
+                            // accumulator goes back to the MMA warp before their
+                            // scan, so the next MMAs into it start meanwhile.
+                            tmem_fence_before();
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive(&s.acc_empty[acc][h]);
+                        }
+                        const int32_t cb = c0 + chunk * kC;
+                        // Scores, lower is better: |c|^2 - 2<q,c> (squared L2) or
+                        // -<q,c> (kept as +<q,c>, compared against -worst).
+                        if constexpr (!kIP) {
+                            // The chunk's candidate norms, the same for every lane:
+                            // 16-byte loads where the chunk lies inside the rows.
+                            if (cb >= q.lo && cb + kC <= q.hi) {
 #pragma unroll
-                            for (int j = 0; j < kC; j += 4) {
-                                const float4 nc =
-                                    __ldg(reinterpret_cast<const float4 *>(sqnorm + cb + j));
-                                v[j] = fmaf(-2.f, v[j], nc.x);
-                                v[j + 1] = fmaf(-2.f, v[j + 1], nc.y);
-                                v[j + 2] = fmaf(-2.f, v[j + 2], nc.z);
-                                v[j + 3] = fmaf(-2.f, v[j + 3], nc.w);
+                                for (int j = 0; j < kC; j += 4) {
+                                    const float4 nc =
+                                        __ldg(reinterpret_cast<const float4 *>(sqnorm + cb + j));
+                                    v[j] = fmaf(-2.f, v[j], nc.x);
+                                    v[j + 1] = fmaf(-2.f, v[j + 1], nc.y);
+                                    v[j + 2] = fmaf(-2.f, v[j + 2], nc.z);
+                                    v[j + 3] = fmaf(-2.f, v[j + 3], nc.w);
+                                }
+                            } else {
+#pragma unroll
+                                for (int j = 0; j < kC; ++j) {
+                                    const int32_t c = cb + j;
+                                    const float nc =
+                                        (c >= q.lo && c < q.hi) ? __ldg(sqnorm + c) : 0.f;
+                                    v[j] = fmaf(-2.f, v[j], nc);
+                                }
+                            }
+                        }
+                        if (tail) {
+#pragma unroll
+                            for (int j = 0; j < kC; ++j)
+                                if (cb + j < q.lo || cb + j >= q.hi) v[j] = kIP ? -FLT_MAX : FLT_MAX;
+                        }
+                        // Best score of each group of columns, then of the chunk.
+                        float gb[kG];
+#pragma unroll
+                        for (int g = 0; g < kG; ++g) {
+                            const float *w = v + kGroup * g;
+                            gb[g] = kIP ? -fmaxf(max3f(w[0], w[1], w[2]), w[3])
+                                        : fminf(min3f(w[0], w[1], w[2]), w[3]);
+                        }
+                        const float best = tree_reduce<false, kG>(gb);
+                        if constexpr (R == 1) {
+                            // The best alone: its column is looked for when it wins.
+                            if (!__any_sync(0xffffffffu, best < worst)) continue;
+                            if (best < worst) {
+                                const float raw = kIP ? -best : best;
+#pragma unroll
+                                for (int j = kC - 1; j >= 0; --j)
+                                    if (v[j] == raw) li[0] = cb + j;
+                                ls[0] = worst = best;
+                            }
+                        } else if constexpr (kFilling) {
+                            // The columns that beat the row's worst are queued one by
+                            // one, and merged into the lists when a row's queue would
+                            // overflow, after a tile when one has more than kMergeAt,
+                            // and after the last tile.
+                            const bool hit = __any_sync(0xffffffffu, best < worst);
+                            const bool tile_end = chunk == kCandTile / kC - 1;
+                            if (!hit && !tile_end) continue;
+                            const uint32_t limit = !tile_end           ? kPendBytes
+                                                   : ct + 1 == ct_end ? 0u
+                                                                       : kMergeAt * 32 * 4;
+                            const uint32_t pend_v = smem_u32(s.queue[warp - kEpiWarp0]) + 4 * lane;
+                            const uint32_t pend_i = pend_v + kPendBytes;
+                            const float before = worst;
+                            uint32_t start = qoff;
+                            for (;;) {
+                                if (hit) {
+                                    qoff = start;
+#pragma unroll
+                                    for (int g = 0; g < kG; ++g)
+                                        if (__any_sync(0xffffffffu, gb[g] < before))
+                                            push_group<kIP>(pend_v, pend_i,
+                                                            qoff, kPendBytes,
+                                                            kIP ? -before : before, v + kGroup * g,
+                                                            cb + kGroup * g);
+                                    if ((int32_t)qoff < 0) qoff = 0u;
+                                }
+                                if (!__any_sync(0xffffffffu, qoff > limit)) break;
+                                // Past the end: the chunk is gone over again after the
+                                // merge: what was stored now lies below offset 0 (and
+                                // is not stored again), what was not follows.
+                                const bool over = __any_sync(0xffffffffu, qoff > kPendBytes);
+                                qoff = min(qoff, kPendBytes);
+                                merge_pending<R, kIP, kEntries>(ls, li, worst, qoff, pend_v,
+                                                             pend_i);
+                                if (!over) break;
+                                start -= kPendBytes;
                             }
                         } else {
+                            // The groups whose best beats the row's worst are queued
+                            // whole: about 7 instructions a group, where looking at
+                            // each column of them here held the accumulator for longer.
+                            // A queue that would overflow: as above.
+                            if (!__any_sync(0xffffffffu, best < worst)) continue;
+                            const float before = worst;
+                            uint32_t start = qoff;
+                            for (;;) {
+                                qoff = start;
 #pragma unroll
-                            for (int j = 0; j < kC; ++j) {
-                                const int64_t c = cb + j;
-                                const float nc =
-                                    (c >= q.lo && c < q.hi) ? __ldg(sqnorm + c) : 0.f;
-                                v[j] = fmaf(-2.f, v[j], nc);
+                                for (int g = 0; g < kG; ++g)
+                                    queue_group(queue_v, queue_i, qoff, kQueueBytes, gb[g], before,
+                                                v + kGroup * g, cb + kGroup * g);
+                                if ((int32_t)qoff < 0) qoff = 0u;
+                                if (!__any_sync(0xffffffffu, qoff > kQueueBytes)) break;
+                                qoff = min(qoff, kQueueBytes);
+                                flush(ls, li, worst, qoff);
+                                start -= kQueueBytes;
                             }
                         }
                     }
-                    if (tail) {
-#pragma unroll
-                        for (int j = 0; j < kC; ++j)
-                            if (cb + j < q.lo || cb + j >= q.hi) v[j] = kIP ? -FLT_MAX : FLT_MAX;
-                    }
-                    // Best score of each group of columns, then of the chunk.
-                    float gb[kG];
-#pragma unroll
-                    for (int g = 0; g < kG; ++g) {
-                        const float *w = v + kGroup * g;
-                        gb[g] = kIP ? -fmaxf(max3f(w[0], w[1], w[2]), w[3])
-                                    : fminf(min3f(w[0], w[1], w[2]), w[3]);
-                    }
-                    const float best = tree_reduce<false, kG>(gb);
-                    if (!__any_sync(0xffffffffu, best < worst)) continue;
-                    if constexpr (R == 1) {
-                        // The best alone: its column is looked for when it wins.
-                        if (best < worst) {
-                            const float raw = kIP ? -best : best;
-#pragma unroll
-                            for (int j = kC - 1; j >= 0; --j)
-                                if (v[j] == raw) li[0] = (int32_t)(cb + j);
-                            ls[0] = worst = best;
-                        }
-                    } else {
-                        // The groups whose best beats the row's worst are queued
-                        // whole: about 7 instructions a group, where looking at each
-                        // column of them here held the accumulator for longer.
-                        // When a row's groups run past the end of its queue the
-                        // queues are flushed and the groups gone over again: what
-                        // was stored now lies below offset 0 (and is not stored
-                        // again), what was not follows.
-                        const float before = worst;
-                        uint32_t start = qoff;
-                        for (;;) {
-                            qoff = start;
-#pragma unroll
-                            for (int g = 0; g < kG; ++g)
-                                queue_group(queue_v, queue_i, qoff, kQueueBytes, gb[g], before,
-                                            v + kGroup * g, (int32_t)(cb + kGroup * g));
-                            if ((int32_t)qoff < 0) qoff = 0u;
-                            if (!__any_sync(0xffffffffu, qoff > kQueueBytes)) break;
-                            qoff = min(qoff, kQueueBytes);
+                    acc ^= 1;
+                    if (acc == 0) acc_phase ^= 1;
+                    // Here, with the accumulator released, queues past kFlushAt slots
+                    // are flushed.  Fewer slots insert for fewer rows a round, more
+                    // hold the warp up for longer than the accumulators' two buffers
+                    // cover: 131,072 x 100 BF16 6.54, 6.44, 6.45 and 6.53 ms with 1, 2, 4
+                    // and 6, 60,013 x 100 FP32 2.59, 2.57, 2.54 and 2.65.
+                    if constexpr (!kFilling)
+                        if (__any_sync(0xffffffffu, qoff > kFlushAt * sizeof(QueueSlot)))
                             flush(ls, li, worst, qoff);
-                            start -= kQueueBytes;
-                        }
-                    }
                 }
-                acc ^= 1;
-                if (acc == 0) acc_phase ^= 1;
-                // Here, with the accumulator released, queues past kFlushAt slots
-                // are flushed.  Fewer slots insert for fewer rows a round, more
-                // hold the warp up for longer than the accumulators' two buffers
-                // cover: 131,072 x 100 BF16 6.54, 6.44, 6.45 and 6.53 ms with 1, 2, 4
-                // and 6, 60,013 x 100 FP32 2.59, 2.57, 2.54 and 2.65.
-                if (__any_sync(0xffffffffu, qoff > kFlushAt * sizeof(QueueSlot)))
-                    flush(ls, li, worst, qoff);
+                return true;
+            };
+            int32_t ct = q.lo / kCandTile;
+            const int32_t ct_end = (q.hi - 1) / kCandTile + 1;
+            bool ok = true;
+            if (kMerge && !q.cont) {
+                const int32_t filled = min(ct_end, ct + kFillTiles);
+                ok = scan(std::true_type(), ct, filled);
+                ct = filled;
             }
+            if (ok) ok = scan(std::false_type(), ct, ct_end);
             if (!ok) break;
-            if (q.more && !q.seed) continue;  // the next item extends this query tile
+            // The item read again: its rows, its flags and where its lists go are not
+            // held in registers over the sweep (the barrier keeps the two reads apart).
+            int32_t again = it;
+            asm volatile("" : "+r"(again));
+            const TcItem o = work[again];
+            const int64_t grow = o.row0 + row_in_tile;
+            const bool seed = (o.flags & kTcSeed) != 0;
+            if ((o.flags & kTcMore) && !seed) continue;  // the next item extends this tile
             flush(ls, li, worst, qoff);
-            if (q.seed) {
+            if (seed) {
                 // R candidates score `worst` or better, so that the row's R best do:
                 // entries from the next larger score on are as good as empty ones.
-                const float bound = ls[R - 1] < FLT_MAX ? nextafterf(ls[R - 1], FLT_MAX) : FLT_MAX;
+                const float bound = worst < FLT_MAX ? nextafterf(worst, FLT_MAX) : FLT_MAX;
 #pragma unroll
                 for (int t = 0; t < R; ++t) {
                     ls[t] = bound;
                     li[t] = -1;
                 }
-                if (live) worst = bound;
+                if (grow < o.qend) worst = bound;
                 continue;
             }
-            // The item read again: where its lists go is not held in registers
-            // over the sweep (the barrier keeps the two reads apart).
-            int64_t again = it;
-            asm volatile("" : "+l"(again));
-            const TcItem o = work[again];
-            const int64_t grow = o.row0 + row_in_tile;
             if (grow < o.qend) {
                 const int64_t orow = row_map ? (int64_t)row_map[grow] : grow + o.out_off;
                 int32_t *out = cand_i + orow * R;
@@ -837,13 +1041,14 @@ TcSweep plan_sweep(int64_t N, int ctas) {
     // tiles, and a sixth of a sweep), or in ctas equal runs, which then mostly reach
     // over two tiles and fill two sets of lists: filling one from nothing takes
     // about as long as scanning kFill candidate tiles afterwards.  Selection in us,
-    // whole / p runs / ctas runs: 10,000 x 64 BF16 (40 tiles, p = 3) 271 / 183 / 243,
-    // 131,072 x 100 (56 left, p = 2) 4,255 / 3,918 / 4,081, 20,000 x 100 (79) 386 /
-    // - / 420, 32,768 x 100 (128) 487 / - / 885, 60,013 x 100 FP32 (83 left) 2,082 / -
-    // / 1,838, 30,000 x 100 FP32 (118) 595 / - / 650.  A last wave more than three
+    // whole / p runs / ctas runs, before lists were filled by merging: 10,000 x 64 BF16
+    // (40 tiles, p = 3) 271 / 183 / 243, 131,072 x 100 (56 left, p = 2) 4,255 / 3,918 /
+    // 4,081, 20,000 x 100 (79) 386 / - / 420, 32,768 x 100 (128) 487 / - / 885, 60,013 x
+    // 100 FP32 (83 left) 2,082 / - / 1,838, 30,000 x 100 FP32 (118) 595 / - / 650; since
+    // then 131,072 x 100 - / 3,786 / 3,600.  A last wave more than three
     // quarters full stays whole: 500,000 x 64 (130 left) 39.1 ms whole, 40.4 in runs
     // (300,000 x 100, 108 left, 18.8 and 18.7).
-    constexpr int64_t kFill = 200;
+    constexpr int64_t kFill = 100;
     const int64_t rest = left * n_ct;
     const int64_t p = std::max<int64_t>(1, std::min<int64_t>({ctas / left, 6, n_ct / 2}));
     int64_t G = p * left, cost = n_ct / p + kFill;
@@ -944,6 +1149,7 @@ TcWork launch_sweep_work(int64_t N, const TcSweep &w, int R, void *workspace, cu
     work.begin = begin;
     work.end = end;
     work.items = items;
+    work.fill = N < kFillMaxRows;
     return work;
 }
 
@@ -998,14 +1204,24 @@ void launch_select(const CUtensorMap &map, const CUtensorMap &map_c, const TcPar
                      plan.wait_cycles > 0 ? plan.wait_cycles : kWaitCycles, plan.stall ? 1 : 0);
     };
     constexpr size_t one = sizeof(SharedStorage<1>), two = sizeof(SharedStorage<2>);
-    if (plan.parts == 2)
-        plan.R == 32 ? go(knn_select_tc<32, true, 2>, two) : go(knn_select_tc<64, true, 2>, two);
-    else if (plan.R == 1)
-        go(knn_select_tc<1, true, 1>, one);
-    else if (plan.R == 32)
-        ip ? go(knn_select_tc<32, true, 1>, one) : go(knn_select_tc<32, false, 1>, one);
-    else
-        ip ? go(knn_select_tc<64, true, 1>, one) : go(knn_select_tc<64, false, 1>, one);
+    if (plan.parts == 2) {
+        if (plan.R == 64)
+            go(knn_select_tc<64, true, 2, false>, two);
+        else if (work.fill)
+            go(knn_select_tc<32, true, 2, true>, two);
+        else
+            go(knn_select_tc<32, true, 2, false>, two);
+    } else if (plan.R == 1) {
+        go(knn_select_tc<1, true, 1, false>, one);
+    } else if (plan.R == 64) {
+        ip ? go(knn_select_tc<64, true, 1, false>, one) : go(knn_select_tc<64, false, 1, false>, one);
+    } else if (!ip) {
+        go(knn_select_tc<32, false, 1, true>, one);
+    } else if (work.fill) {
+        go(knn_select_tc<32, true, 1, true>, one);
+    } else {
+        go(knn_select_tc<32, true, 1, false>, one);
+    }
 }
 
 void check_plan(const KnnTcPlan &plan) {

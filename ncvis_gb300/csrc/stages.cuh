@@ -104,7 +104,9 @@ struct TcWork {
     const TcItem *items = nullptr;
     const int32_t *map = nullptr;  // optional row map (sorted row -> output row)
     TcLists lists;
+    bool fill = true;  // the kernel's form: lists filled by merging (short sweeps)
 };
+constexpr int64_t kFillMaxRows = 147456;  // from here on sweeps are long
 // How the query tiles of one problem of N rows are spread over at most `ctas`
 // CTAs: the first full_qt whole and round-robin, the rest in equal runs of
 // candidate tiles over the first rest_ctas, so that the last wave fills the

@@ -1,6 +1,7 @@
 """The BF16 search with the last wave's query tiles shared out over several CTAs
 (src/ncvis.cpp:72-153 for what it replaces): every row's kept candidates are the
-best R by BF16 score over all rows, whichever CTA met them.
+best R by BF16 score over all rows, whichever CTA met them and whether the list was
+filled by merging (below 147,456 rows, lists of 32) or by single insertions.
 
 The reference scores the rounded rows in 64 bits, keeps the best R and ranks them
 by their exact distances.  Rows are unit vectors, so a score sums D products of
@@ -16,7 +17,8 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("N,D,ordered", [
     (257, 8, True), (1000, 32, True), (4097, 17, True), (10000, 64, True), (12289, 33, True),
     (38913, 16, False), (38913, 16, True), (60013, 24, True), (60013, 24, False),
-    (78000, 32, True), (131072, 20, True)])
+    (78000, 32, True), (131072, 20, True), (147455, 9, True), (147456, 9, True),
+    (2049, 8, True)])
 def test_kept_candidates_of_split_rows(cuda, N, D, ordered, k):
     from ncvis_gb300 import DISTANCES, stages
     g = cuda.Generator(device="cuda").manual_seed(N + D)
