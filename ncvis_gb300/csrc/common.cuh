@@ -47,7 +47,7 @@ unsigned long long current_context_id();
 // stage calls synchronise, so that each of them mapped its workspace anew: 0.14 to
 // 0.44 ms a call (1,000 x 32 neighbours, 800,000 x 15 symmetrization).  This one
 // keeps at most kPoolKeeps bytes between calls; they go back when an engine is
-// destroyed and when an allocation finds no room.  The driver orders reuse between
+// destroyed and when an allocation finds no room.  CUDA orders reuse between
 // streams and threads; a context made anew gets a new pool.
 constexpr size_t kPoolKeeps = size_t(1) << 30;
 cudaMemPool_t workspace_pool();
