@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(kThreads) nce_edges_t(int mode, int64_t E, uin
 #pragma unroll
             for (int t = 0; t < kG; t += 2)
                 if (n0 + t < c.nu)
-                    noise_pair<false>(c.k0, c.k1, eg, c.tag, (uint32_t)(n0 + t) >> 1, (uint32_t)i, N, o[t],
+                    noise_pair(c.k0, c.k1, eg, c.tag, (uint32_t)(n0 + t) >> 1, (uint32_t)i, N, o[t],
                                o[t + 1]);
 #pragma unroll
             for (int t = 0; t < kG; ++t)
