@@ -117,9 +117,9 @@ __device__ __forceinline__ void put_row(float *Y, int64_t i, const Vec<D> &yi, c
 }
 
 struct EpochConst {
-    float step, nu_f, a, b, alpha_Q, pow_b1_at_zero;
+    float step, nu_f, a, b, ab, alpha_Q, pow_b1_at_zero;
     int nu;
-    float b1, ab2_step;  // b - 1 and 2ab step
+    float b1, ab2;  // b - 1 and 2ab
 };
 
 // The SFU's approximations (PTX ISA) of 2^x, log2 x and 1 / x with subnormal inputs
@@ -168,32 +168,29 @@ __device__ __forceinline__ float nce_weight(float d2, bool positive, const Epoch
         p1 = k.pow_b1_at_zero;
     }
     const float denom = fmaf(k.a, p, 1.f);
-    const float nm = __fmul_rn(k.nu_f, ex2_approx(__fmul_rn(Qc, 1.4426950408889634f)));
-    const float t = fmaf(nm, denom, 1.f);
+    const float eQ = ex2_approx(__fmul_rn(Qc, 1.4426950408889634f));
+    const float t = fmaf(__fmul_rn(k.nu_f, eQ), denom, 1.f);
     const float r = rcp_approx(__fmul_rn(t, denom));  // t, denom >= 1
+    float w;
     if (positive) {
-        const float w = fmaf(-r, denom, 1.f);  // 1 - 1/t
+        w = fmaf(-r, denom, 1.f);  // 1 - 1/t
         Qc = fmaf(-w, k.alpha_Q, Qc);
-        return __fmul_rn(__fmul_rn(w, p1), __fmul_rn(k.ab2_step, __fmul_rn(r, t)));  // r t = 1/denom
+        w = __fmul_rn(__fmul_rn(w, p1), __fmul_rn(k.ab2, __fmul_rn(r, t)));  // r t = 1/denom
+    } else {
+        Qc = fmaf(__fmul_rn(r, denom), k.alpha_Q, Qc);  // r denom = 1/t
+        w = -__fmul_rn(__fmul_rn(p1, k.ab2), r);
     }
-    Qc = fmaf(__fmul_rn(r, denom), k.alpha_Q, Qc);  // r denom = 1/t
-    return __fmul_rn(__fmul_rn(p1, -k.ab2_step), r);
-}
-
-// y - x, and the square of its length.
-template <int D>
-__device__ __forceinline__ Vec<D> row_diff(const Vec<D> &x, const Vec<D> &y) {
-    Vec<D> r;
-#pragma unroll
-    for (int c = 0; c < D; ++c) r.v[c] = y.v[c] - x.v[c];
-    return r;
+    return __fmul_rn(w, k.step);
 }
 
 template <int D>
-__device__ __forceinline__ float sq_norm(const Vec<D> &x) {
+__device__ __forceinline__ float sq_dist(const Vec<D> &x, const Vec<D> &y) {
     float d2 = 0.f;
 #pragma unroll
-    for (int c = 0; c < D; ++c) d2 = fmaf(x.v[c], x.v[c], d2);
+    for (int c = 0; c < D; ++c) {
+        const float t = x.v[c] - y.v[c];
+        d2 = fmaf(t, t, d2);
+    }
     return d2;
 }
 
@@ -255,11 +252,11 @@ __device__ __forceinline__ void run_edge(float *Y, Vec<D> &yi, uint32_t i, uint3
 #pragma unroll
             for (int u = 0; u < t; ++u) dup |= (o[u] == o[t]);
             if (dup) yo[t] = load_row<D>(Y, o[t]);
-            Vec<D> dx = row_diff<D>(yi, yo[t]);
-            const float ws = nce_weight(sq_norm<D>(dx), t == 0 && s == 0, k, Qc);
+            const float ws = nce_weight(sq_dist<D>(yi, yo[t]), t == 0 && s == 0, k, Qc);
+            Vec<D> dx;
 #pragma unroll
             for (int c = 0; c < D; ++c) {
-                dx.v[c] = clip4(dx.v[c] * ws);
+                dx.v[c] = clip4((yo[t].v[c] - yi.v[c]) * ws);
                 yi.v[c] += dx.v[c];
             }
             sub_row<D>(Y, o[t], dx);
@@ -494,29 +491,12 @@ __device__ __forceinline__ uint32_t segment_start(uint32_t k0, uint32_t k1, uint
 // `whole`, the problem's rows in order (W == N).
 struct WindowSpec {
     const uint32_t *seg;
-    const uint32_t *near;  // mark_near's bits, or null: every sample is looked at
     uint32_t W, N, base;
     bool whole;
 };
 
 __device__ __forceinline__ uint32_t spec_row(const WindowSpec &w, uint32_t u) {
     return w.base + (w.whole ? u : window_row(w.seg, u, w.N));
-}
-
-// The 256-row blocks of [0, N) that a staged window's segments touch, as bits by
-// block number modulo kNearBits: a source row whose bit is clear is in no segment,
-// and its noise samples need no look for it (window_redraw's test is 8 of a sample's
-// 73 instructions).  At 1,000,000 rows 32 of 3,907 blocks are touched.
-constexpr uint32_t kNearBits = 4096;
-
-__device__ __forceinline__ void mark_near(uint32_t *bits, uint32_t row) {
-    const uint32_t b = row / kSegRows % kNearBits;
-    atomicOr(bits + b / 32, 1u << (b % 32));
-}
-
-__device__ __forceinline__ bool may_be_near(const uint32_t *bits, uint32_t row) {
-    const uint32_t b = row / kSegRows % kNearBits;
-    return bits[b / 32] >> (b % 32) & 1u;
 }
 
 // Whether window row u is row i: its unwrapped row less i is 0 or N.
@@ -597,11 +577,11 @@ template <int D>
 __device__ __forceinline__ void window_sample(float *win, uint32_t u, Vec<D> &yi,
                                               const EpochConst &k, float &Qc) {
     const Vec<D> yo = load_win<D>(win, u);
-    Vec<D> dx = row_diff<D>(yi, yo), yn;
-    const float ws = nce_weight(sq_norm<D>(dx), false, k, Qc);
+    const float ws = nce_weight(sq_dist<D>(yi, yo), false, k, Qc);
+    Vec<D> dx, yn;
 #pragma unroll
     for (int c = 0; c < D; ++c) {
-        dx.v[c] = clip4(dx.v[c] * ws);
+        dx.v[c] = clip4((yo.v[c] - yi.v[c]) * ws);
         yi.v[c] += dx.v[c];
         yn.v[c] = yo.v[c] - dx.v[c];
     }
@@ -615,11 +595,11 @@ template <int D>
 __device__ __forceinline__ void edge_positive(float *Y, uint32_t i, uint32_t j, const Vec<D> &yj,
                                               const EpochConst &k, float &Qc, Vec<D> &yi) {
     if (j != i) {
-        Vec<D> dx = row_diff<D>(yi, yj);
-        const float w = nce_weight(sq_norm<D>(dx), true, k, Qc);
+        const float w = nce_weight(sq_dist<D>(yi, yj), true, k, Qc);
+        Vec<D> dx;
 #pragma unroll
         for (int c = 0; c < D; ++c) {
-            dx.v[c] = clip4(dx.v[c] * w);
+            dx.v[c] = clip4((yj.v[c] - yi.v[c]) * w);
             yi.v[c] += dx.v[c];
         }
         sub_row<D>(Y, j, dx);
@@ -657,15 +637,13 @@ __device__ __forceinline__ void edge_noise(int64_t e, uint32_t i, const EpochCon
             }
         }
     } else {
-        const bool near = may_be_near(ws.near, i);
         for (int s0 = 0; s0 < k.nu; s0 += 8) {
             const Philox4x32 r = window_block(key0, key1, (uint64_t)e, tag, (uint32_t)(s0 >> 3));
 #pragma unroll
             for (int t = 0; t < 8; ++t) {
                 if (s0 + t >= k.nu) break;
-                uint32_t u = window_pick(r, t, ws.W);
-                if (near)
-                    u = window_redraw(key0, key1, (uint64_t)e, tag, (uint32_t)(s0 + t), u, i, ws);
+                const uint32_t u = window_redraw(key0, key1, (uint64_t)e, tag, (uint32_t)(s0 + t),
+                                                 window_pick(r, t, ws.W), i, ws);
                 window_sample<D>(win, u, yi, k, Qc);
             }
         }
@@ -820,7 +798,6 @@ __global__ void __launch_bounds__(kWinThreads, 2) sgd_epoch_window(
     float *win = win_smem;                                    // current window rows [W][D]
     float *loaded = win_smem + (size_t)W * D;                 // the rows as loaded [W][D]
     uint32_t *seg = reinterpret_cast<uint32_t *>(loaded + (size_t)W * D);  // [W / kSegRows]
-    uint32_t *near = seg + W / kSegRows;                                   // [kNearBits / 32]
     const int64_t chain = (int64_t)blockIdx.x * kWinThreads + threadIdx.x;
     const int64_t e0 = chain < n_chains ? min(E, chain * chunk) : E;
     const int64_t e1 = min(E, e0 + chunk);
@@ -833,21 +810,9 @@ __global__ void __launch_bounds__(kWinThreads, 2) sgd_epoch_window(
 #pragma unroll
     for (int c = 0; c < D; ++c) yi.v[c] = yi0.v[c] = 0.f;
     for (int r = 0; r < rounds; ++r) {
-        if (threadIdx.x < nseg)
-            seg[threadIdx.x] = segment_start(key0, key1, blockIdx.x, (uint32_t)r, (uint32_t)epoch,
-                                             threadIdx.x, N);
-        if (threadIdx.x < kNearBits / 32) near[threadIdx.x] = 0u;
+        for (uint32_t t = threadIdx.x; t < nseg; t += kWinThreads)
+            seg[t] = segment_start(key0, key1, blockIdx.x, (uint32_t)r, (uint32_t)epoch, t, N);
         __syncthreads();
-        if (threadIdx.x < nseg) {
-            mark_near(near, seg[threadIdx.x]);
-            mark_near(near, window_row(seg, threadIdx.x * kSegRows + kSegRows - 1, N));
-            // A segment across the end of the rows is in their last block and their
-            // first as well.
-            if (seg[threadIdx.x] + kSegRows > N) {
-                mark_near(near, N - 1);
-                mark_near(near, 0u);
-            }
-        }
         for (uint32_t u = threadIdx.x; u < W; u += kWinThreads) {
             const Vec<D> v = load_row<D>(Y, window_row(seg, u, N));
             store_win<D>(win, u, v);
@@ -856,7 +821,7 @@ __global__ void __launch_bounds__(kWinThreads, 2) sgd_epoch_window(
         __syncthreads();
         const int64_t a = min(e1, e0 + (int64_t)r * round_edges);
         const int64_t b = min(e1, a + round_edges);
-        const WindowSpec ws{seg, near, W, N, 0u, false};
+        const WindowSpec ws{seg, W, N, 0u, false};
         window_edges<D, false, kGrouped>(Y, src, dst, a, b, k, Qc, key0, key1, (uint32_t)epoch,
                                          win, ws, have, ci, yi, yi0);
         __syncthreads();
@@ -919,7 +884,7 @@ __global__ void __launch_bounds__(T) sgd_epoch_window_batched(
     const bool whole = Np <= kBatWindow;
     const uint32_t W = whole ? Np : kBatWindow;
     const int rounds = (int)((chunk + round_edges - 1) / round_edges);
-    const WindowSpec ws{seg, nullptr, W, Np, base, whole};
+    const WindowSpec ws{seg, W, Np, base, whole};
     float Qc = Qs[p];
     bool have = false;
     uint32_t ci = 0;
@@ -1058,10 +1023,11 @@ EpochConst epoch_const(const SgdArgs &g, int epoch, int nu) {
     k.nu_f = (float)nu;
     k.a = g.a;
     k.b = g.b;
+    k.ab = g.a * g.b;
     k.alpha_Q = g.alpha_Q;
     k.pow_b1_at_zero = std::pow(0.f, g.b - 1.f);
     k.b1 = g.b - 1.f;
-    k.ab2_step = (float)(2.0 * g.a * g.b * k.step);
+    k.ab2 = 2.f * g.a * g.b;
     return k;
 }
 
@@ -1158,10 +1124,10 @@ uint32_t sgd_window_rows(int d) {
 }
 
 // Dynamic shared memory of sgd_epoch_window: the window and its loaded copy,
-// the segment starts and the bits of the blocks they touch.
+// the segment starts.
 size_t window_smem_bytes(int d) {
     const uint32_t W = sgd_window_rows(d);
-    return (size_t)W * d * 8 + (W / kSegRows) * 4 + kNearBits / 8;
+    return (size_t)W * d * 8 + (W / kSegRows) * 4;
 }
 
 bool sgd_window_applies(int64_t N, int d) {
