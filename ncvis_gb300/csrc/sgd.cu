@@ -196,71 +196,81 @@ __device__ __forceinline__ float sq_dist(const Vec<D> &x, const Vec<D> &y) {
 
 __device__ __forceinline__ float clip4(float v) { return fminf(fmaxf(v, -4.f), 4.f); }
 
-// One edge of a chain: its positive sample (sample 0) and its nu noise samples
-// (samples 1 .. nu), with y_i held in registers by the caller.  The rows of kGroup
-// samples are gathered per round trip (eight for D <= 3; four for D = 4, where
-// eight 4-float rows in flight spill registers); a row loaded before an earlier
-// sample of the same group stored it is read again, so a chain always sees its own
-// updates.  One loop body for every group, the first one's positive sample
-// included, and the redraws out of line: with a form for the first group beside one
-// for the others, and the redraws inlined, an edge ran through some 35 KB of
-// instructions, and a chain, alone on its scheduler at 10,000 points, waited for
-// their fetch 40% of its time (474 us an epoch of 20 noise samples, 335 so).
+// Samples of a group whose row was loaded before an earlier sample of the
+// same group stored it are reloaded, so a chain always sees its own updates.
+template <int D, int G>
+__device__ __forceinline__ void run_group(float *Y, Vec<D> &yi, const uint32_t (&o)[G], int count,
+                                          bool first_is_positive, const EpochConst &k, float &Qc) {
+    Vec<D> yo[G];
+#pragma unroll
+    for (int t = 0; t < G; ++t)
+        if (t < count) yo[t] = load_row<D>(Y, o[t]);
+#pragma unroll
+    for (int t = 0; t < G; ++t) {
+        if (t >= count) break;
+        bool dup = false;
+#pragma unroll
+        for (int u = 0; u < t; ++u) dup |= (o[u] == o[t]);
+        if (dup) yo[t] = load_row<D>(Y, o[t]);
+        const float ws = nce_weight(sq_dist<D>(yi, yo[t]), first_is_positive && t == 0, k, Qc);
+        Vec<D> dx;
+#pragma unroll
+        for (int c = 0; c < D; ++c) {
+            dx.v[c] = clip4((yo[t].v[c] - yi.v[c]) * ws);
+            yi.v[c] += dx.v[c];
+        }
+        sub_row<D>(Y, o[t], dx);
+    }
+}
+
+// One edge of a chain: the positive sample and its noise samples, with y_i
+// held in registers by the caller.
 template <int D>
 __device__ __forceinline__ void run_edge(float *Y, Vec<D> &yi, uint32_t i, uint32_t j, int64_t e,
                                          uint32_t N, uint32_t lo, const EpochConst &k, float &Qc,
                                          uint32_t key0, uint32_t key1, uint32_t tag) {
+    // Rows gathered per round trip: eight for D <= 3; four for D = 4, where
+    // eight 4-float rows in flight spill registers.
     constexpr int kGroup = D <= 3 ? 8 : 4;
-    // A noise sample's Philox block serves two: the second of a group's last one
-    // is the first sample of the next.
-    uint32_t carry = j;
-#pragma unroll 1
-    for (int s = 0; s <= k.nu; s += kGroup) {
-        const int count = min(kGroup, k.nu + 1 - s);
-        uint32_t o[kGroup + 1];
-        o[0] = carry;
+    int s = 0;  // next noise sample
+    if (j != i) {
+        // The positive sample and the first kGroup - 2 noise samples share one
+        // group (one round trip per edge while nu <= kGroup - 2).
+        uint32_t o[kGroup - 1];
+        o[0] = j;
+        const int first = min(k.nu, kGroup - 2);
+#pragma unroll
+        for (int p = 0; p < kGroup / 2 - 1; ++p) {
+            o[1 + 2 * p] = o[2 + 2 * p] = 0u;
+            if (2 * p < first) {
+                noise_pair(key0, key1, (uint64_t)e, tag, (uint32_t)p, i - lo, N, o[1 + 2 * p],
+                           o[2 + 2 * p]);
+                o[1 + 2 * p] += lo;
+                o[2 + 2 * p] += lo;
+            }
+        }
+        run_group<D, kGroup - 1>(Y, yi, o, 1 + first, true, k, Qc);
+        s = first;
+    } else {
+        // A self edge: y_i += dx then y_i -= dx on one row (src/ncvis.cpp:337-338).
+        const float ws = nce_weight(0.f, true, k, Qc);
+#pragma unroll
+        for (int c = 0; c < D; ++c) {
+            const float dx = clip4(0.f * ws);
+            yi.v[c] = (yi.v[c] + dx) - dx;
+        }
+    }
+    // Remaining noise samples in groups of kGroup (kGroup / 2 Philox blocks).
+    for (; s < k.nu; s += kGroup) {
+        uint32_t o[kGroup];
 #pragma unroll
         for (int p = 0; p < kGroup / 2; ++p) {
-            // Noise samples s + 2p and s + 2p + 1 of the edge.
-            o[1 + 2 * p] = o[2 + 2 * p] = 0u;
-            if (2 * p < count)
-                noise_pair(key0, key1, (uint64_t)e, tag, (uint32_t)(s >> 1) + p, i - lo, N,
-                           o[1 + 2 * p], o[2 + 2 * p]);
-            o[1 + 2 * p] += lo;
-            o[2 + 2 * p] += lo;
+            noise_pair(key0, key1, (uint64_t)e, tag, (uint32_t)(s >> 1) + p, i - lo, N, o[2 * p],
+                       o[2 * p + 1]);
+            o[2 * p] += lo;
+            o[2 * p + 1] += lo;
         }
-        carry = o[kGroup];
-        Vec<D> yo[kGroup];
-#pragma unroll
-        for (int t = 0; t < kGroup; ++t)
-            if (t < count) yo[t] = load_row<D>(Y, o[t]);
-#pragma unroll
-        for (int t = 0; t < kGroup; ++t) {
-            if (t >= count) break;
-            if (t == 0 && s == 0 && j == i) {
-                // A self edge: y_i += dx then y_i -= dx on one row
-                // (src/ncvis.cpp:337-338).
-                const float ws = nce_weight(0.f, true, k, Qc);
-#pragma unroll
-                for (int c = 0; c < D; ++c) {
-                    const float dx = clip4(0.f * ws);
-                    yi.v[c] = (yi.v[c] + dx) - dx;
-                }
-                continue;
-            }
-            bool dup = false;
-#pragma unroll
-            for (int u = 0; u < t; ++u) dup |= (o[u] == o[t]);
-            if (dup) yo[t] = load_row<D>(Y, o[t]);
-            const float ws = nce_weight(sq_dist<D>(yi, yo[t]), t == 0 && s == 0, k, Qc);
-            Vec<D> dx;
-#pragma unroll
-            for (int c = 0; c < D; ++c) {
-                dx.v[c] = clip4((yo[t].v[c] - yi.v[c]) * ws);
-                yi.v[c] += dx.v[c];
-            }
-            sub_row<D>(Y, o[t], dx);
-        }
+        run_group<D, kGroup>(Y, yi, o, min(kGroup, k.nu - s), false, k, Qc);
     }
 }
 
