@@ -122,22 +122,10 @@ struct EpochConst {
     float b1, ab2;  // b - 1 and 2ab
 };
 
-// The SFU's approximations (PTX ISA) of 2^x, log2 x and 1 / x with subnormal inputs
-// and results taken as 0, which leaves out the scaling that __expf, __log2f and
-// __fdividef bring for them (8 of the 81 instructions of a staged noise sample).
+// 2^x by the SFU's approximation (ex2.approx.ftz.f32, PTX ISA).
 __device__ __forceinline__ float ex2_approx(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-__device__ __forceinline__ float lg2_approx(float x) {
-    float y;
-    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-__device__ __forceinline__ float rcp_approx(float x) {
-    float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
 
@@ -155,11 +143,7 @@ __device__ __forceinline__ float nce_weight(float d2, bool positive, const Epoch
     // same bits for the same inputs.
     if (k.nu == 0) return k.step;
     float p, p1;
-    if (d2 >= FLT_MIN) {
-        const float lg = lg2_approx(d2);
-        p = ex2_approx(__fmul_rn(k.b, lg));
-        p1 = ex2_approx(__fmul_rn(k.b1, lg));
-    } else if (d2 > 0.f) {  // subnormal
+    if (d2 > 0.f) {
         const float lg = __log2f(d2);
         p = ex2_approx(__fmul_rn(k.b, lg));
         p1 = ex2_approx(__fmul_rn(k.b1, lg));
@@ -168,9 +152,8 @@ __device__ __forceinline__ float nce_weight(float d2, bool positive, const Epoch
         p1 = k.pow_b1_at_zero;
     }
     const float denom = fmaf(k.a, p, 1.f);
-    const float eQ = ex2_approx(__fmul_rn(Qc, 1.4426950408889634f));
-    const float t = fmaf(__fmul_rn(k.nu_f, eQ), denom, 1.f);
-    const float r = rcp_approx(__fmul_rn(t, denom));  // t, denom >= 1
+    const float t = fmaf(__fmul_rn(k.nu_f, __expf(Qc)), denom, 1.f);
+    const float r = __fdividef(1.f, __fmul_rn(t, denom));
     float w;
     if (positive) {
         w = fmaf(-r, denom, 1.f);  // 1 - 1/t
@@ -509,13 +492,6 @@ __device__ __forceinline__ uint32_t spec_row(const WindowSpec &w, uint32_t u) {
     return w.base + (w.whole ? u : window_row(w.seg, u, w.N));
 }
 
-// Whether window row u is row i: its unwrapped row less i is 0 or N.
-__device__ __forceinline__ bool spec_is(const WindowSpec &w, uint32_t u, uint32_t i) {
-    if (w.whole) return w.base + u == i;
-    const uint32_t off = w.seg[u / kSegRows] + u % kSegRows - (i - w.base);
-    return off == 0u || off == w.N;
-}
-
 // A noise sample whose window row is the edge source i is redrawn from
 // blocks (e_lo, e_hi ^ retry<<16, tag, s/2 | 3<<30) under key (k0 ^ retry, k1),
 // up to 64 times; then the next window row is taken.
@@ -523,7 +499,7 @@ __device__ __forceinline__ uint32_t window_redraw(uint32_t k0, uint32_t k1, uint
                                                   uint32_t s, uint32_t u, uint32_t i,
                                                   const WindowSpec &ws) {
     const uint32_t W = ws.W;
-    for (uint32_t retry = 1; spec_is(ws, u, i); ++retry) {
+    for (uint32_t retry = 1; spec_row(ws, u) == i; ++retry) {
         if (retry > 64) {
             u = (u + 1 == W) ? 0 : u + 1;
             break;
