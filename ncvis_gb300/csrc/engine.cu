@@ -265,11 +265,13 @@ static int run_knn_fp32(const float *Xp, const float *sqn, size_t N, size_t D, i
         launch_knn_select_f32(Xp, sqn, (int64_t)N, (int)D, dist, plan.simt, cand, s);
         return plan.simt.C();
     }
+    KnnTcPlan tc = plan.tc;
+    tc.low_low = norms[2] != 0;
     __half *rows = (__half *)block;
-    launch_split_rows(Xp, sqn, (int64_t)N, (int)D, scale, plan.tc, rows, (int64_t)N, s);
+    launch_split_rows(Xp, sqn, (int64_t)N, (int)D, scale, tc, rows, (int64_t)N, s);
     const TcWork work =
         launch_sweep_work((int64_t)N, plan.sweep, plan.tc.R, block + plan.rows_bytes, s);
-    launch_knn_select_split(rows, (int64_t)N, plan.tc, cand, timeout_flag, s, work);
+    launch_knn_select_split(rows, (int64_t)N, tc, cand, timeout_flag, s, work);
     launch_merge_lists((int64_t)N, plan.sweep, work.lists, plan.tc.R, plan.keep, nullptr, cand, s);
     return plan.keep;
 }
@@ -866,6 +868,7 @@ void ncvis_engine::fit_batched(const float *dX, size_t D, const int64_t *offsets
             // problems are never read as outputs or candidates (the work
             // items' ends mask them).
             C = sp.R;
+            sp.low_low = h_flag[6] != 0;
             __half *rows = (__half *)(base + o_sym);
             launch_split_rows(Xp, sqn, total, (int)D, scale, sp, rows, total_pad, s, d_off, d_pad,
                               (int)B);

@@ -39,8 +39,8 @@
 //     is an FP16 high and low part (split_rows, preprocess.cu), a candidate
 //     tile is taken in two parts, and its product is the sum of three FP16
 //     products accumulated in FP32, the small ones first: q_hi c_lo, then
-//     q_lo c_hi and q_hi c_hi (rows of up to 32 columns q_lo c_lo as well, which
-//     is not below the others' rounding there).
+//     q_lo c_hi and q_hi c_hi (q_lo c_lo as well for rows of up to 32 columns,
+//     where it is not below the others' rounding, and for plans with low_low).
 // Every mbarrier wait is bounded in time: on expiry the CTA sets *err,
 // stops, drains its MMAs and in-flight TMA copies, frees TMEM and returns.
 // The waits between roles use the plan's limit (default ~2 s); the drain
@@ -577,7 +577,7 @@ template <int R, bool kIP, int kParts, bool kFill>
 __global__ void __launch_bounds__(kThreads, 1)
     knn_select_tc(const __grid_constant__ CUtensorMap tmap,
                   const __grid_constant__ CUtensorMap tmap_c, const TcParts parts,
-                  const float *__restrict__ sqnorm, int ksteps, int katoms,
+                  const float *__restrict__ sqnorm, int ksteps, int katoms, int low_low_steps,
                   const int64_t *__restrict__ work_begin, const int64_t *__restrict__ work_end,
                   const TcItem *__restrict__ work, const int32_t *__restrict__ row_map,
                   int32_t *__restrict__ cand_i, const TcLists lists, int *__restrict__ err,
@@ -714,7 +714,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                             accumulate = 1u;
                         }
                     };
-                    if (kParts == 2 && (p == 0 || ksteps <= kLowLowSteps)) product(kParts - 1);
+                    if (kParts == 2 && (p == 0 || ksteps <= low_low_steps)) product(kParts - 1);
                     product(0);
                     umma_commit(&s.empty[stage]);
                     if (++stage == kStages) stage = 0, phase ^= 1;
@@ -1200,7 +1200,7 @@ void launch_select(const CUtensorMap &map, const CUtensorMap &map_c, const TcPar
         NCVIS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         (int)smem));
         NCVIS_LAUNCH(kernel, grid, kThreads, smem, s, map, map_c, parts, sqnorm, ksteps, katoms,
-                     work.begin, work.end, work.items, work.map, cand_i, work.lists, timeout_flag,
+                     plan.low_low ? ksteps : kLowLowSteps, work.begin, work.end, work.items, work.map, cand_i, work.lists, timeout_flag,
                      plan.wait_cycles > 0 ? plan.wait_cycles : kWaitCycles, plan.stall ? 1 : 0);
     };
     constexpr size_t one = sizeof(SharedStorage<1>), two = sizeof(SharedStorage<2>);

@@ -20,6 +20,19 @@ __device__ __forceinline__ float warp_sum(float v) {
     return v;
 }
 
+// The value of x's lowest set bit (0 for 0).
+__device__ __forceinline__ float low_bit(float x) {
+    const uint32_t b = __float_as_uint(x) & 0x7fffffffu;
+    const float v = __uint_as_float(b);
+    return (b & 0x7fffffu) ? v - __uint_as_float(b & (b - 1u)) : v;
+}
+
+// A row whose coordinates are multiples of u and whose squared norm is at most
+// kExactNorm u^2 has exact FP32 sums with every other such row: their products and
+// squared norms are whole numbers of u^2 below 2^24.  Integers, one-hot columns and
+// 8-bit pixels are such rows; ties among their distances are exact and go by index.
+constexpr float kExactNorm = 0x1p24f;
+
 __global__ void __launch_bounds__(256) preprocess_rows(const float *__restrict__ X, int64_t N,
                                                        int D, int dist, float *__restrict__ Xp,
                                                        float *__restrict__ sqnorm,
@@ -52,11 +65,13 @@ __global__ void __launch_bounds__(256) preprocess_rows(const float *__restrict__
     const bool normalise = (dist == kCorrelation || dist == kCosine) && sq != 0.f;
     if (normalise) scale_div = sqrtf(sq);
     float sq_out = 0.f;
+    bool bits12 = false;  // a coordinate of exactly 12 significant bits
     for (int t = lane; t < D; t += 32) {
         float v = x[t] - mean;
         if (normalise) v = v / scale_div;
         out[t] = v;
         sq_out += v * v;
+        bits12 |= (__float_as_uint(v) & 0x1fffu) == 0x1000u;
         if (Xb) Xb[row * ldb + t] = __float2bfloat16_rn(v);
         if (Xc) Xc[row * ldb + t] = __float2bfloat16_rn(v);
     }
@@ -69,6 +84,16 @@ __global__ void __launch_bounds__(256) preprocess_rows(const float *__restrict__
     if (Xc)
         for (int t = D + extra + lane; t < ldb; t += 32) Xc[row * ldb + t] = __float2bfloat16_rn(0.f);
     sq_out = warp_sum(sq_out);
+    if (norms && __any_sync(0xffffffffu, bits12)) {
+        // One row in eighty of arbitrary numbers comes here; its lowest bit is
+        // far too low.
+        float u = INFINITY;
+        for (int t = lane; t < D; t += 32)
+            if (out[t] != 0.f) u = fminf(u, low_bit(out[t]));
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) u = fminf(u, __shfl_xor_sync(0xffffffffu, u, o));
+        if (lane == 0 && sq_out <= kExactNorm * u * u) norms[2] = 1u;
+    }
     if (lane == 0) {
         sqnorm[row] = sq_out;
         if (norms) {
@@ -97,7 +122,10 @@ __global__ void __launch_bounds__(256) preprocess_rows(const float *__restrict__
 // in FP32's last place.  The tensor cores' FP32 accumulator truncates: a product
 // loses about 0.6 units in its 24th place per 16 columns (measured: 0.36 on unit
 // rows to 0.85 on rows far from the origin), which lo makes up for on both sides
-// (`lift` = half of that, relative).  Squared L2 (fold): w = -|s c|^2 / 2 goes into three
+// (`lift` = half of that, relative).  A coordinate that may belong to a row of exact
+// sums (kExactNorm) takes no lift: nothing is truncated there, and a lift would tell
+// equal distances apart (60,000 rows of 32 zeros and ones: 8% of the rows had other
+// neighbours than (distance, index) says).  Squared L2 (fold): w = -|s c|^2 / 2 goes into three
 // columns, w = 2^14 a + 2^3 b + 2^-8 c with a, b, c in FP16, each part's
 // remainder exact; the powers keep all three within FP16's normal range for
 // norms from 2^1 to 2^14.
@@ -117,6 +145,7 @@ __global__ void __launch_bounds__(256) split_rows(
         to = pad[p] + (row - off[p]);
     }
     const float *x = Xp + row * D;
+    const float sq = __ldg(sqnorm + row);
     float v[8];
     if ((D & 3) == 0 && c0 + 8 <= D) {
         const float4 a = __ldg(reinterpret_cast<const float4 *>(x + c0));
@@ -131,12 +160,14 @@ __global__ void __launch_bounds__(256) split_rows(
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
         const float y = v[j] * scale;
+        const float low = low_bit(v[j]);
+        const bool exact = sq <= kExactNorm * low * low;
         h[j] = __float2half_rn(y);
-        l[j] = __float2half_rn(fmaf(y, lift, y - __half2float(h[j])));
+        l[j] = __float2half_rn(fmaf(y, exact ? 0.f : lift, y - __half2float(h[j])));
         c[j] = h[j];
     }
     if (fold && c0 + 8 > D) {
-        const float w = -0.5f * sqnorm[row] * scale * scale;
+        const float w = -0.5f * sq * scale * scale;
         const __half a = __float2half_rn(w * 0x1p-14f);
         const float r1 = w - __half2float(a) * 0x1p14f;
         const __half b = __float2half_rn(r1 * 0x1p-3f);
@@ -156,7 +187,7 @@ __global__ void __launch_bounds__(256) split_rows(
 
 }  // namespace
 
-float split_scale(const uint32_t norms[2], int dist) {
+float split_scale(const uint32_t norms[3], int dist) {
     // Unit rows (and rows of zeros).
     if (dist == kCosine || dist == kCorrelation) return 0x1p14f;
     if (norms[0] == 0u) return 1.f;

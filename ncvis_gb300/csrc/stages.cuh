@@ -19,8 +19,9 @@ enum Distance { kSquaredL2 = 0, kInnerProduct = 1, kCosine = 2, kCorrelation = 3
 // is set to 1 if any input is not finite.
 // Xc (optional, squared L2 on the tensor cores): candidate copy whose columns
 // D, D + 1 hold -|x|^2 / 2 as BF16 high + low parts; Xb then holds 1, 1 there.
-// norms (optional, two device words that start at 0): the bits of the largest
-// |xp|^2, and kInfBits minus the bits of the smallest that is not 0.
+// norms (optional, three device words that start at 0): the bits of the largest
+// |xp|^2, kInfBits minus the bits of the smallest that is not 0, and 1 if a row
+// whose sums are exact in FP32 has a coordinate of 12 significant bits.
 constexpr uint32_t kInfBits = 0x7f800000u;
 void launch_preprocess(const float *X, int64_t N, int D, int dist, float *Xp, float *sqnorm,
                        __nv_bfloat16 *Xb, int ldb, int *bad_flag, cudaStream_t s,
@@ -61,6 +62,9 @@ struct KnnTcPlan {
     int ldb;     // padded row length of Xb (16-bit elements)
     bool fold;   // squared L2 with the norms folded into the product (needs Xc)
     int parts = 1;  // 1: BF16 rows; 2: FP16 high and low parts (the FP32 search)
+    // Two parts: the product of the low parts is taken for rows of any length.  Rows
+    // of exact sums need it once a coordinate has a low part, which their ties go by.
+    bool low_low = false;
     // Diagnostics: limit of the kernel's waits between its roles in SM cycles
     // (<= 0: about 2 s), and a stall on a barrier nothing completes (the
     // timeout path's test).
@@ -153,7 +157,7 @@ void launch_knn_select_tc(const __nv_bfloat16 *Xb, const float *sqnorm, int64_t 
 // where no s serves them all: hi + lo holds s x to one unit in FP32's last
 // place only while |s x| >= 2^-3, so every row's norm must stay within 2^13 of
 // the largest (and that be finite).
-float split_scale(const uint32_t norms[2], int dist);
+float split_scale(const uint32_t norms[3], int dist);
 KnnTcPlan plan_knn_split(int D, int R, int dist);
 bool knn_split_supported(int64_t N, int D, int R, int dist);
 void launch_split_rows(const float *Xp, const float *sqnorm, int64_t N, int D, float scale,
