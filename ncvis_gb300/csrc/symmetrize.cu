@@ -213,7 +213,7 @@ __global__ void __launch_bounds__(T, 1) merge_rows_thread(
     }
 }
 
-// The longest rows rows[0 .. *n_rows) of the list, one warp each (W warps per
+// The longest rows and those that hold a NaN, rows[0 .. *n_rows), one warp each (W warps per
 // block, C items per warp in shared memory: [W][C] sort items, then [W][C]
 // indices).  The warp
 // loads the row, sorts its incoming ids (each id's rank among the row's ids;
@@ -304,6 +304,9 @@ __global__ void __launch_bounds__(32 * W, 1) merge_rows_warp(
 //     (item j kept or not from the kept items of the previous guess), which
 //     agrees with the sequential loop from the start up to one more item per
 //     step.
+// A row that holds a NaN, whose comparisons are all false, goes on to the last tier:
+// the ranks in a leaf are no permutation then, and std::sort's own steps, which end
+// and stay within the row whatever the keys are, decide its order.
 // Rows of up to 128 items: four words of 32 positions, whose ballots stay in
 // registers (a second form of two words beside it costs more registers than it
 // saves steps: 387 -> 465 us at 80,000 rows of 49 to 128).  Shared memory per
@@ -374,7 +377,8 @@ __device__ __forceinline__ int32_t warp_partition(WparRow &w, int32_t lo, int32_
 }
 
 // Row i of L <= 32 NW items, its incoming ids (of which there are nin) already in
-// w.orig[k ..).  Returns the number of kept entries, written to out_col, out_val.
+// w.orig[k ..).  Returns the number of kept entries, written to out_col, out_val, or
+// -1 for a row that holds a NaN.
 template <int NW>
 __device__ __forceinline__ int merge_row_warp(WparRow &w, int64_t i, int L, int nin, int k,
                                               const int32_t *__restrict__ inds,
@@ -390,19 +394,20 @@ __device__ __forceinline__ int merge_row_warp(WparRow &w, int64_t i, int L, int 
         w.ids[rk] = e;
     }
     __syncwarp();
+    bool nan = false;
 #pragma unroll
     for (int m = 0; m < NW; ++m) {
         const int p = lane + 32 * m;
-        if (p < k) {
-            w.items[p] = SortItem{dists[i * k + p], p};
-            w.orig[p] = inds[i * k + p];
-        } else if (p < L) {
-            const int32_t e = w.ids[p - k];
-            w.items[p] = SortItem{dists[e], p};
-            w.orig[p] = e / k;
+        if (p < L) {
+            const int32_t e = p < k ? 0 : w.ids[p - k];
+            const float key = dists[p < k ? i * k + p : (int64_t)e];
+            w.items[p] = SortItem{key, p};
+            w.orig[p] = p < k ? inds[i * k + p] : e / k;
+            nan |= key != key;
         }
     }
     __syncwarp();
+    if (__any_sync(0xffffffffu, nan)) return -1;
     // The introsort's partitions and leaves (a warp-uniform range stack).
     int32_t st_lo[16], st_hi[16], st_d[16];
     int top = 0;
@@ -527,7 +532,12 @@ __global__ void __launch_bounds__(32 * W, 1) merge_rows_wpar(
         __syncwarp();
         const int n = merge_row_warp<kWparCap / 32>(w, i, L, nin, k, inds, dists, out_col + base,
                                                     out_val + base, lane);
-        if (lane == 0) kept[i] = n;
+        if (lane == 0) {
+            if (n >= 0)
+                kept[i] = n;
+            else
+                next[atomicAdd(n_next, 1)] = (int32_t)i;
+        }
     }
 }
 
@@ -621,17 +631,19 @@ __global__ void __launch_bounds__(32 * W) merge_rows_big(
             ids[rk] = e;
         }
         __syncwarp();
+        bool nan = false;
         for (int p = lane; p < L; p += 32) {
-            if (p < k) {
-                w.items[p] = SortItem{dists[i * k + p], p};
-                w.orig[p] = inds[i * k + p];
-            } else {
-                const int32_t e = ids[p - k];
-                w.items[p] = SortItem{dists[e], p};
-                w.orig[p] = e / k;
-            }
+            const int32_t e = p < k ? 0 : ids[p - k];
+            const float key = dists[p < k ? i * k + p : (int64_t)e];
+            w.items[p] = SortItem{key, p};
+            w.orig[p] = p < k ? inds[i * k + p] : e / k;
+            nan |= key != key;
         }
         __syncwarp();
+        if (__any_sync(0xffffffffu, nan)) {
+            if (lane == 0) next[atomicAdd(n_next, 1)] = (int32_t)i;
+            continue;
+        }
         // The right parts wait while the left ones are gone on with: at most one
         // a level of the depth budget.
         int32_t st_lo[32], st_hi[32], st_d[32];
