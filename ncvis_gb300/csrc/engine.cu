@@ -453,8 +453,8 @@ void ncvis_engine::fit(const float *X, size_t N, size_t D, float *Y, bool host) 
     KnnF32Plan fp;
     if (!bf16) fp = plan_knn_fp32(N, D, k, o.rerank_factor, dist);
     KnnTcPlan tp = plan_knn_tc((int64_t)N, (int)D, k, o.rerank_factor, dist);
-    tp.wait_cycles = o.wait_limit_cycles;
-    tp.stall = o.inject_stall != 0;
+    tp.wait_cycles = fp.tc.wait_cycles = o.wait_limit_cycles;
+    tp.stall = fp.tc.stall = o.inject_stall != 0;
     if (bf16)
         require(knn_tc_supported((int)D, tp.R),
                 "[ncvis] the BF16 tensor-core kNN supports D <= 128", kUnsupported);
@@ -726,6 +726,8 @@ void ncvis_engine::fit_batched(const float *dX, size_t D, const int64_t *offsets
         tw = plan_batched_tc(h_off, num_sms());
         split = knn_split_supported(tw.pad[B], (int)D, kp.R, dist);
         if (split) sp = plan_knn_split((int)D, kp.R, dist);
+        sp.wait_cycles = tp.wait_cycles;
+        sp.stall = tp.stall;
     }
     const int64_t max_chains = std::max<int64_t>(sgd_batched_resident_chains(d), (int64_t)B);
 
