@@ -46,13 +46,13 @@ unsigned long long current_context_id();
 // device's default pool gives its memory back at every synchronisation, and the
 // stage calls synchronise, so that each of them mapped its workspace anew: 0.14 to
 // 0.44 ms a call (1,000 x 32 neighbours, 800,000 x 15 symmetrization).  This one
-// keeps at most kPoolKeeps bytes between calls; they go back when an engine is
-// destroyed and when an allocation finds no room.  CUDA orders reuse between
-// streams and threads; a context made anew gets a new pool.
+// keeps at most kPoolKeeps bytes between calls; they go back when an engine that has
+// fitted on the device is destroyed and when an allocation finds no room.  CUDA orders
+// reuse between streams and threads; each context has a pool of its own.
 constexpr size_t kPoolKeeps = size_t(1) << 30;
 cudaMemPool_t workspace_pool();
-// Gives back what the current device's pool keeps unused.
-void trim_workspace_pool();
+// Gives back what the pool of device `dev` keeps unused.
+void trim_workspace_pool(int dev);
 // Stream-ordered memory of `bytes` bytes from the pool (cudaFreeAsync frees it).
 void *pool_alloc(size_t bytes, cudaStream_t s);
 

@@ -306,6 +306,7 @@ struct ncvis_engine {
     cudaStream_t own = nullptr;
     void *arena = nullptr;
     size_t arena_bytes = 0;
+    int arena_dev = 0;  // the device the arena is on
 
     // The engine's own stream is created on first use, so that constructing
     // an engine touches no GPU (as constructing the reference's NCVis only
@@ -319,7 +320,7 @@ struct ncvis_engine {
     ~ncvis_engine() {
         if (arena) cudaFree(arena);
         if (own) cudaStreamDestroy(own);
-        if (arena) trim_workspace_pool();
+        if (arena) trim_workspace_pool(arena_dev);
     }
 
     char *ensure_arena(size_t bytes) {
@@ -335,11 +336,12 @@ struct ncvis_engine {
                 arena = nullptr;
                 arena_bytes = 0;
             }
+            NCVIS_CUDA(cudaGetDevice(&arena_dev));
             cudaError_t r = cudaMalloc(&arena, bytes);
             if (r == cudaErrorMemoryAllocation) {
                 // The stage calls' pool may hold what is missing.
                 cudaGetLastError();
-                trim_workspace_pool();
+                trim_workspace_pool(arena_dev);
                 r = cudaMalloc(&arena, bytes);
             }
             NCVIS_CUDA(r);

@@ -2,8 +2,10 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <map>
 #include <mutex>
 #include <string>
+#include <utility>
 
 #include "common.cuh"
 
@@ -24,13 +26,10 @@ Fn driver_entry(const char *name) {
     return (Fn)p;
 }
 
-constexpr int kMaxDevices = 128;
-struct Pool {
-    unsigned long long ctx_id = 0;
-    cudaMemPool_t pool = nullptr;
-};
 std::mutex g_mu;
-Pool g_pools[kMaxDevices];
+// By device and context id; ids are not used again, so the entry of a context that
+// was destroyed, whose pool went with it, is never met.
+std::map<std::pair<int, unsigned long long>, cudaMemPool_t> g_pools;
 
 }  // namespace
 
@@ -48,11 +47,16 @@ unsigned long long current_context_id() {
 cudaMemPool_t workspace_pool() {
     int dev = 0;
     NCVIS_CUDA(cudaGetDevice(&dev));
-    require(dev >= 0 && dev < kMaxDevices, "device index out of range");
+    unsigned long long id = current_context_id();
+    if (id == 0) {
+        // A thread that has made no call which needs a context yet.
+        NCVIS_CUDA(cudaFree(nullptr));
+        id = current_context_id();
+        require(id != 0, "workspace pool: no current context", kCudaError);
+    }
     std::lock_guard<std::mutex> lock(g_mu);
-    const unsigned long long id = current_context_id();
-    Pool &e = g_pools[dev];
-    if (id == 0 || e.ctx_id != id || !e.pool) {
+    cudaMemPool_t &known = g_pools[{dev, id}];
+    if (!known) {
         cudaMemPoolProps props{};
         props.allocType = cudaMemAllocationTypePinned;
         props.location.type = cudaMemLocationTypeDevice;
@@ -66,22 +70,22 @@ cudaMemPool_t workspace_pool() {
             cudaMemPoolDestroy(pool);
             NCVIS_CUDA(set);
         }
-        e.pool = pool;  // a pool of an earlier context went with it
-        e.ctx_id = current_context_id();
+        known = pool;
     }
-    return e.pool;
+    return known;
 }
 
-void trim_workspace_pool() {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return;
-    std::lock_guard<std::mutex> lock(g_mu);
-    const Pool &e = g_pools[dev];
-    if (!e.pool) return;
+void trim_workspace_pool(int dev) {
+    int current = 0;
+    if (cudaGetDevice(&current) != cudaSuccess) return;
+    if (dev != current && cudaSetDevice(dev) != cudaSuccess) return;
     try {
-        if (e.ctx_id == current_context_id()) cudaMemPoolTrimTo(e.pool, 0);
+        std::lock_guard<std::mutex> lock(g_mu);
+        const auto known = g_pools.find({dev, current_context_id()});
+        if (known != g_pools.end() && known->second) cudaMemPoolTrimTo(known->second, 0);
     } catch (const Error &) {  // no context any more: nothing is kept either
     }
+    if (dev != current) cudaSetDevice(current);
 }
 
 void *pool_alloc(size_t bytes, cudaStream_t s) {
