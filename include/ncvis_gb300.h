@@ -319,6 +319,14 @@ int ncvis_trustworthiness_device(const float *dX, size_t N, size_t D, int distan
 int ncvis_measure_update_rate(size_t rows, size_t d, double *gathers_per_s, double *updates_per_s,
                               void *stream);
 
+/* The stage-level entry points take their workspaces from a memory pool of the
+ * library's own, one per device and context, which keeps up to 1 GiB between calls.
+ * This gives back what the current device's pool holds unused (after the calls in
+ * flight are waited for: work that still runs holds its workspace).  Destroying an
+ * engine that has fitted on the device does the same.  No reference counterpart.
+ * Errors: ncvis_get_last_error(). */
+int ncvis_release_workspace(void);
+
 /* Number of kernels this library has launched in the process so far. */
 uint64_t ncvis_kernel_launch_count(void);
 

@@ -143,6 +143,7 @@ SIGNATURES = {
                                                C.POINTER(C.c_double), C.c_void_p]),
     "ncvis_measure_update_rate": (C.c_int, [C.c_size_t, C.c_size_t, C.POINTER(C.c_double),
                                             C.POINTER(C.c_double), C.c_void_p]),
+    "ncvis_release_workspace": (C.c_int, []),
     "ncvis_kernel_launch_count": (C.c_uint64, []),
     "ncvis_version": (C.c_char_p, []),
 }

@@ -1425,6 +1425,14 @@ int ncvis_nce_noise_device(size_t N, size_t E, const int32_t *d_src, size_t n_no
     });
 }
 
+int ncvis_release_workspace(void) {
+    return guarded(nullptr, [&] {
+        int dev = 0;
+        NCVIS_CUDA(cudaGetDevice(&dev));
+        trim_workspace_pool(dev);
+    });
+}
+
 uint64_t ncvis_kernel_launch_count(void) { return launch_counter().load(); }
 
 const char *ncvis_version(void) { return "ncvis_gb300 0.1.0 (sm_103a)"; }

@@ -151,5 +151,12 @@ def optimize_replay(Y, Q, src, dst, stream, stream_offset: int, epoch: int, n_ep
     return Y, Q
 
 
+def release_workspace() -> None:
+    """Gives back what the current device's workspace pool keeps between stage calls
+    (at most 1 GiB); the calls in flight are waited for first."""
+    _torch().cuda.synchronize()
+    _lib.check(_lib.lib().ncvis_release_workspace())
+
+
 def launch_count() -> int:
     return int(_lib.lib().ncvis_kernel_launch_count())
