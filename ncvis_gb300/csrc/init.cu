@@ -170,10 +170,15 @@ struct Sum2 {
 };
 
 // Thread c < D gets the block's sum of sum[c]: over the warps' lanes, then over
-// the warps in FP64.
-template <int D>
-__device__ __forceinline__ double block_sum(Sum2 (&sum)[D]) {
+// the warps in FP64.  Where a value or a sum left FP32's range (which turns the two
+// numbers into NaN), the block sums its values, value(i) for rows i of [begin, end),
+// in FP64 instead: an infinite sum stays one.
+template <int D, class Value>
+__device__ __forceinline__ double block_sum(Sum2 (&sum)[D], int64_t begin, int64_t end,
+                                            Value value) {
     __shared__ double red[D][kThreads / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    bool out_of_range = false;
 #pragma unroll
     for (int c = 0; c < D; ++c) {
 #pragma unroll
@@ -182,14 +187,39 @@ __device__ __forceinline__ double block_sum(Sum2 (&sum)[D]) {
             const float l = __shfl_xor_sync(0xffffffffu, sum[c].lo, o);
             sum[c].add(h, l);
         }
-        if ((threadIdx.x & 31) == 0)
-            red[c][threadIdx.x >> 5] = (double)sum[c].hi + (double)sum[c].lo;
+        out_of_range |= !isfinite(sum[c].hi);
+        if (lane == 0) red[c][warp] = (double)sum[c].hi + (double)sum[c].lo;
     }
-    __syncthreads();
+    if (__syncthreads_or(out_of_range)) {
+        double exact[D];
+#pragma unroll
+        for (int c = 0; c < D; ++c) exact[c] = 0.0;
+        for (int64_t i = begin + threadIdx.x; i < end; i += kThreads) {
+            const RowVec<D> v = value(i);
+#pragma unroll
+            for (int c = 0; c < D; ++c) exact[c] += (double)v.v[c];
+        }
+#pragma unroll
+        for (int c = 0; c < D; ++c) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) exact[c] += __shfl_xor_sync(0xffffffffu, exact[c], o);
+            if (lane == 0) red[c][warp] = exact[c];
+        }
+        __syncthreads();
+    }
     double s = 0.0;
     if (threadIdx.x < D)
         for (int w = 0; w < kThreads / 32; ++w) s += red[threadIdx.x][w];
     return s;
+}
+
+// Row i as this block wrote it (not through the read-only path).
+template <int D>
+__device__ __forceinline__ RowVec<D> written_row(const float *Y, int64_t i) {
+    RowVec<D> r;
+#pragma unroll
+    for (int c = 0; c < D; ++c) r.v[c] = __ldcg(Y + i * kPitch<D> + c);
+    return r;
 }
 
 // One init epoch's neighbour sums for d <= 4 and their means, one thread per row:
@@ -239,7 +269,9 @@ __global__ void __launch_bounds__(kThreads) spmm_mean(
 #pragma unroll
         for (int c = 0; c < D; ++c) sum[c].hi = acc.v[c];
     }
-    finish_stat<true>(D, block_sum<D>(sum), part, done, b, mean);
+    const double s = block_sum<D>(sum, b.row, b.end,
+                                  [&](int64_t r) { return written_row<D>(Ynew, r); });
+    finish_stat<true>(D, s, part, done, b, mean);
 }
 
 // The same for few rows, where the longest row is what an epoch waits for: a row's
@@ -378,7 +410,9 @@ __global__ void __launch_bounds__(kThreads) spmm_mean_share(
         const RowVec<D> acc = long_row_sum<D>(lp, (int)(row_ptr[li + 1] - lp), cols, alpha, Yold);
         if (lane == 0) finish(li, acc);
     }
-    finish_stat<true>(D, block_sum<D>(sum), part, done, b, mean);
+    const double s = block_sum<D>(sum, b.row, b.end,
+                                  [&](int64_t r) { return written_row<D>(Ynew, r); });
+    finish_stat<true>(D, s, part, done, b, mean);
 }
 
 // sigma from the rows and their mean: (y - mean)^2 rounded to FP32 as the
@@ -395,15 +429,21 @@ __global__ void __launch_bounds__(kThreads) centred_sigma(RowBlocks blocks,
     float m[D];
 #pragma unroll
     for (int c = 0; c < D; ++c) m[c] = mean[b.problem * D + c];
-    for (int64_t i = b.row + threadIdx.x; i < b.end; i += kThreads) {
-        const RowVec<D> y = load_row<D>(Y, i);
+    auto term = [&](int64_t i) {
+        RowVec<D> t = load_row<D>(Y, i);
 #pragma unroll
         for (int c = 0; c < D; ++c) {
-            const float dev = __fsub_rn(y.v[c], m[c]);
-            sum[c].add(__fmul_rn(dev, dev), 0.f);
+            const float dev = __fsub_rn(t.v[c], m[c]);
+            t.v[c] = __fmul_rn(dev, dev);
         }
+        return t;
+    };
+    for (int64_t i = b.row + threadIdx.x; i < b.end; i += kThreads) {
+        const RowVec<D> t = term(i);
+#pragma unroll
+        for (int c = 0; c < D; ++c) sum[c].add(t.v[c], 0.f);
     }
-    finish_stat<false>(D, block_sum<D>(sum), part, done, b, sigma);
+    finish_stat<false>(D, block_sum<D>(sum, b.row, b.end, term), part, done, b, sigma);
 }
 
 // The two for any d, one thread per row and dimension: neighbouring threads read
