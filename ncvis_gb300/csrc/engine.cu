@@ -835,7 +835,8 @@ void ncvis_engine::fit_batched(const float *dX, size_t D, const int64_t *offsets
     NCVIS_CUDA(cudaMemcpyAsync(h_flag, flag, sizeof(h_flag), cudaMemcpyDeviceToHost, s));
     NCVIS_CUDA(cudaStreamSynchronize(s));
     require(h_flag[0] == 0, "[ncvis] input contains non-finite values");
-    const float scale = split ? split_scale((const uint32_t *)h_flag + 4, dist) : 0.f;
+    const float scale =
+        split ? split_scale((const uint32_t *)h_flag + 4, dist, B == 1) : 0.f;
     nv.next("ncvis.batched.knn");
     NCVIS_CUDA(cudaMemsetAsync(knn_i, 0xff, sizeof(int32_t) * nk, s));
     int C = kp.C();  // candidates per point

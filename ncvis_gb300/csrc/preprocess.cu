@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(256) split_rows(
 
 }  // namespace
 
-float split_scale(const uint32_t norms[3], int dist) {
+float split_scale(const uint32_t norms[3], int dist, bool one_problem) {
     // Unit rows (and rows of zeros).
     if (dist == kCosine || dist == kCorrelation) return 0x1p14f;
     if (norms[0] == 0u) return 1.f;
@@ -198,6 +198,12 @@ float split_scale(const uint32_t norms[3], int dist) {
     std::memcpy(&low, &low_bits, 4);
     // Squared norms must keep their own precision in FP32.
     if (low < 0x1p-100f || top > 0x1p100f) return 0.f;
+    // Distances 1 - <q, c> are rounded to 2^-24, and equal ones go by index.  Where a
+    // row's products all lie within 2^-14 many distances are equal though their
+    // products are not, and the CUDA cores' search ranks by the distance: 20,000 x 64
+    // at products of 2^-18 and 1,000 x 16 at 2^-20 held other neighbours from the tensor
+    // cores, none at 2^-16.  A problem of a batch may hold the smallest norms only.
+    if (dist == kInnerProduct && (one_problem ? std::sqrt(low * top) : low) < 0x1p-14f) return 0.f;
     const int e = std::ilogb(std::sqrt(top)) + 1;  // norms < 2^e (1 + rounding)
     const float scale = std::ldexp(1.f, 14 - e);
     return std::sqrt(low) * scale >= 2.f ? scale : 0.f;

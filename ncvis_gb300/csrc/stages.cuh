@@ -156,8 +156,9 @@ void launch_knn_select_tc(const __nv_bfloat16 *Xb, const float *sqnorm, int64_t 
 // split_scale: the s for the rows' norms (the words of launch_preprocess), 0
 // where no s serves them all: hi + lo holds s x to one unit in FP32's last
 // place only while |s x| >= 2^-3, so every row's norm must stay within 2^13 of
-// the largest (and that be finite).
-float split_scale(const uint32_t norms[3], int dist);
+// the largest (and that be finite).  0 too for inner products so small that the
+// distances' rounding decides (one_problem: the norms are one problem's).
+float split_scale(const uint32_t norms[3], int dist, bool one_problem = true);
 KnnTcPlan plan_knn_split(int D, int R, int dist);
 bool knn_split_supported(int64_t N, int D, int R, int dist);
 void launch_split_rows(const float *Xp, const float *sqnorm, int64_t N, int D, float scale,
