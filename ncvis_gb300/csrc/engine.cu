@@ -256,12 +256,14 @@ static KnnF32Plan plan_knn_fp32(size_t N, size_t D, int k, int rerank_factor, in
 
 // Runs the search into cand (plan.cand_bytes) with block (plan.block_bytes) as
 // scratch; norms: the words of launch_preprocess, on the host.  Returns the number
-// of candidates per row.
+// of candidates per row; plan.split becomes whether the tensor cores ran, whose
+// timeout flag is the caller's to read.
 static int run_knn_fp32(const float *Xp, const float *sqn, size_t N, size_t D, int dist,
-                        const KnnF32Plan &plan, const uint32_t *norms, int32_t *cand, char *block,
+                        KnnF32Plan &plan, const uint32_t *norms, int32_t *cand, char *block,
                         int *timeout_flag, cudaStream_t s) {
     const float scale = plan.split ? split_scale(norms, dist) : 0.f;
-    if (scale == 0.f) {
+    plan.split = scale != 0.f;
+    if (!plan.split) {
         launch_knn_select_f32(Xp, sqn, (int64_t)N, (int)D, dist, plan.simt, cand, s);
         return plan.simt.C();
     }
