@@ -591,8 +591,9 @@ size_t knn_order_workspace_bytes(int64_t N, int D, const KnnTcPlan &tp, const Kn
     // sort_by_cell: counts, cursors, starts, permutation, sorted rows.
     b += 2 * a(sizeof(int) * C) + a(sizeof(int64_t) * (C + 1)) + a(sizeof(int32_t) * n);
     b += 2 * a(2 * n * ldb);
-    // the sweep's work list: a query tile, or a CTA's piece of one of the last, is
-    // at most two items.
+    // the sweep's work list: a whole query tile is at most two items; one in n pieces
+    // has n - 1 seeds and at most n + 1 ranges (one piece wraps around), and the last
+    // tiles are in at most ctas pieces more than there are of them.
     b += a(sizeof(int64_t) * (ctas + 1)) + a(sizeof(TcItem) * 2 * (tiles + ctas));
     return b;
 }

@@ -20,7 +20,6 @@
 // findKNN stores them.
 #include <algorithm>
 #include <cfloat>
-#include <type_traits>
 
 #include "common.cuh"
 #include "stages.cuh"

@@ -391,7 +391,12 @@ __device__ __forceinline__ void flush_queue(float (&ls)[R], int32_t (&li)[R], fl
 // 131,072 x 100 3,800 and 3,600.  Sweeps over kFillMaxRows rows or more (TcWork::fill)
 // go without: its loop beside theirs costs them more than the filling gives (whole
 // calls without and with it: 150,000 x 100 5.98 and 5.92 ms, 150,000 x 32 4.90 and
-// 5.08, 250,000 x 64 11.4 and 12.0, 500,000 x 64 38.0 and 41.5).
+// 5.08, 250,000 x 64 11.4 and 12.0, 500,000 x 64 38.0 and 41.5).  That rule is for the
+// sweeps of one problem's rows (launch_sweep_work, the ordered sweep); the lists of the
+// inverted file and of batched problems take short sweeps each and always fill, and so
+// does squared L2 without folded norms (127 and 128 columns), which has no other form
+// (before the filling and now: inverted file of 1,000,000 x 100 33.9 and 21.2 ms, squared
+// L2 of 100,000 x 127 6.20 and 4.79, 300,000 x 127 44.2 and 43.0).
 constexpr int kPending = 16;
 
 // Orders entries a and b by score, equal scores by index (the order they are met
@@ -1157,6 +1162,7 @@ void launch_merge_lists(int64_t N, const TcSweep &w, const TcLists &lists, int R
                         const int32_t *order, int32_t *cand_i, cudaStream_t s) {
     if (lists.count == 0) return;
     require(R == 32 || R == 64, "knn: lists of 32 or 64 candidates", kInternal);
+    require(!order || keep <= R, "knn: more candidates than seeded lists hold", kInternal);
     const int warps = 4;
     const size_t smem = sizeof(float) * warps * lists.count * R;  // at most 8 lists: 8 KB
     const unsigned grid = (unsigned)ceil_div(N - lists.row0, warps);

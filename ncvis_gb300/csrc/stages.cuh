@@ -94,7 +94,9 @@ struct alignas(16) TcItem {
 // The lists of the rows whose query tiles several items share (`count` > 0): rows
 // (in the launch's numbering) from row0 on have a list per slot, R candidates and
 // their scores at [((row - row0) * count + slot) * R], best first; -1 marks an
-// empty entry, with the largest score.
+// empty entry, with the largest score or, after a kTcSeed item, the seed's bound:
+// empty entries of one list may then come before another's candidates, but never
+// among the R best of them all, which is how many may be kept (launch_merge_lists).
 struct TcLists {
     int32_t *idx = nullptr;
     float *score = nullptr;
@@ -141,7 +143,7 @@ struct TcRun {
 };
 // The best `keep` candidates of every split row's lists (by score, then by list)
 // into cand_i[row * keep], -1 behind them where there are fewer; rows are
-// order[row] when `order` is given.
+// order[row] when `order` is given (the ordered sweep, which seeds its lists: keep <= R).
 void launch_merge_lists(int64_t N, const TcSweep &w, const TcLists &lists, int R, int keep,
                         const int32_t *order, int32_t *cand_i, cudaStream_t s);
 void launch_knn_select_tc(const __nv_bfloat16 *Xb, const float *sqnorm, int64_t N,

@@ -220,14 +220,13 @@ __global__ void __launch_bounds__(T, 1) merge_rows_thread(
 // the ids are distinct) and gathers the distances in parallel; lane 0 runs
 // the sort and the deduplication (sequential: the tie order is
 // libstdc++'s); the warp writes the kept entries.  A row of more than C
-// items goes to `next`, or, in the last tier, to the global scratch.
+// items is merged on the global scratch.
 template <int C, int W>
 __global__ void __launch_bounds__(32 * W, 1) merge_rows_warp(
     int k, const int32_t *__restrict__ inds, const float *__restrict__ dists,
     const int64_t *__restrict__ in_off, int32_t *__restrict__ in_key, SortItem *__restrict__ g_items,
     int32_t *__restrict__ out_col, float *__restrict__ out_val, int32_t *__restrict__ kept,
-    const int32_t *__restrict__ rows, const int32_t *__restrict__ n_rows, int32_t *__restrict__ next,
-    int32_t *__restrict__ n_next) {
+    const int32_t *__restrict__ rows, const int32_t *__restrict__ n_rows) {
     extern __shared__ __align__(16) SortItem sm_items[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     SortItem *items = sm_items + (size_t)warp * C;
@@ -241,13 +240,9 @@ __global__ void __launch_bounds__(32 * W, 1) merge_rows_warp(
         const int L = k + nin;
         const int64_t base = i * k + ib;  // row-aligned output offset
         if (L > C) {
-            if (lane == 0) {
-                if (next)
-                    next[atomicAdd(n_next, 1)] = (int32_t)i;
-                else
-                    kept[i] = merge_global(i, k, inds, dists, in_off, in_key, g_items, out_col,
-                                           out_val);
-            }
+            if (lane == 0)
+                kept[i] = merge_global(i, k, inds, dists, in_off, in_key, g_items, out_col,
+                                       out_val);
             continue;
         }
         const int32_t *ink = in_key + ib;
@@ -787,8 +782,7 @@ void launch_merge_big(int k, const int32_t *inds, const float *dists, const int6
 template <int C, int W>
 void launch_merge_warp(int k, const int32_t *inds, const float *dists, const int64_t *in_off,
                        int32_t *in_key, SortItem *g_items, int32_t *out_col, float *out_val,
-                       int32_t *kept, const int32_t *rows, const int32_t *n_rows, int32_t *next,
-                       int32_t *n_next, cudaStream_t s) {
+                       int32_t *kept, const int32_t *rows, const int32_t *n_rows, cudaStream_t s) {
     const size_t smem = (sizeof(SortItem) + sizeof(int32_t)) * C * W;
     // Set on every launch: the attribute is per device, and a cached flag
     // would race between host threads running different engines.
@@ -797,7 +791,7 @@ void launch_merge_warp(int k, const int32_t *inds, const float *dists, const int
     // A grid of resident blocks that reads the list's length on the device.
     const int64_t grid = (int64_t)num_sms() * blocks_per_sm(smem, 32 * W);
     NCVIS_LAUNCH((merge_rows_warp<C, W>), grid, 32 * W, smem, s, k, inds, dists, in_off, in_key,
-                 g_items, out_col, out_val, kept, rows, n_rows, next, n_next);
+                 g_items, out_col, out_val, kept, rows, n_rows);
 }
 
 // The kept entries from their row-aligned places to the CSR, kRowLanes lanes a row,
@@ -946,8 +940,7 @@ int64_t run_symmetrize(int64_t N, int k, const int32_t *inds, const float *dists
     launch_merge_big<kCap2, kWarps2>(k, inds, dists, w.in_off, w.in_key, w.out_col, w.out_val,
                                      w.kept, w.tier1, w.n_tier + 2, w.tier3, w.n_tier + 3, s);
     launch_merge_warp<kCap3, kWarps3>(k, inds, dists, w.in_off, w.in_key, w.items, w.out_col,
-                                      w.out_val, w.kept, w.tier3, w.n_tier + 3, nullptr, nullptr,
-                                      s);
+                                      w.out_val, w.kept, w.tier3, w.n_tier + 3, s);
     launch_exclusive_scan_i32_to_i64(w.kept, row_ptr, N, w.scan, s);
     NCVIS_LAUNCH(compact_rows, ceil_div((size_t)N * kRowLanes, 256), 256, 0, s, N, k, w.in_off, w.kept, row_ptr,
                  w.out_col, w.out_val, cols, vals, src);
