@@ -30,6 +30,7 @@
 #include <cfloat>
 #include <cmath>
 
+#include "chain_blocks.h"
 #include "common.cuh"
 #include "rng.cuh"
 #include "stages.cuh"
@@ -1052,7 +1053,7 @@ int sgd_default_chains(int64_t E, int64_t N, int d) {
 }
 
 size_t sgd_workspace_bytes(int chains) {
-    // Blocks of kThreads chains, or up to two of fewer per SM (run_sgd_hogwild).
+    // Blocks of kThreads chains, or up to two of fewer per SM (chain_block_threads).
     const int64_t most = std::max<int64_t>(chains, (int64_t)num_sms() * 2048);
     return sizeof(double) * ((most + kThreads - 1) / kThreads + 1);
 }
@@ -1061,12 +1062,7 @@ void run_sgd_hogwild(const SgdArgs &g, int epoch_begin, int epoch_end, const siz
                      int chains, void *workspace, cudaStream_t s) {
     require(g.N >= 2 && g.N < (int64_t(1) << 31), "optimize: N must be in [2, 2^31)");
     if (chains <= 0) chains = sgd_default_chains(g.E, g.N, g.d);
-    // Few chains are spread over all SMs: a sample's row gather and its reduction
-    // each take an SM's load unit a cycle a lane, so that 5,000 chains in blocks of
-    // 256 waited for 20 SMs (547 us an epoch of 20 noise samples at 10,000 points;
-    // 474 in blocks of 32).
-    const int sms = num_sms();
-    const int threads = std::max(32, std::min(kThreads, chains / sms / 32 * 32));
+    const int threads = chain_block_threads(chains, num_sms(), kThreads);
     const int blocks = (int)ceil_div(chains, threads);
     const int64_t total_chains = chains;
     const int64_t chunk = ((g.E + total_chains - 1) / total_chains + 3) & ~(int64_t)3;
