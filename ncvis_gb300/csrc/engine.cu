@@ -491,15 +491,14 @@ void ncvis_engine::fit(const float *X, size_t N, size_t D, float *Y, bool host) 
     const size_t o_vals = L.take(sizeof(float) * 2 * nk);
     const size_t o_src = L.take(sizeof(int32_t) * 2 * nk);
     const size_t o_Q = L.take(sizeof(float) * 4);
-    const size_t o_init = L.take(init_workspace_bytes((int64_t)N, d));
     const size_t o_sgd = L.take(sgd_workspace_bytes(chains));
     const size_t o_stream = replay ? L.take(sizeof(int32_t) * std::max<size_t>(o.replay_len, 1)) : 0;
     const size_t ord_bytes = knn_order_workspace_bytes((int64_t)N, (int)D, tp, op);
     const size_t o_ord = ord_bytes ? L.take(ord_bytes) : 0;
     KnnBf16Sweep bs(N, tp, op, bf16 && !ivf);
     // Last: the candidates, and the symmetrization's workspace, which the
-    // search's part rows, lists and work list share (they are read for the last
-    // time before it).  Where memory, or the caller's limit, has no room for those
+    // search's part rows, lists and work list (read for the last time before it)
+    // and the initial embedding's workspace (written after it) share.  Where memory, or the caller's limit, has no room for those
     // the FP32 search takes the CUDA cores and the BF16 one whole query tiles.
     const size_t o_ci = L.total;
     auto cand_bytes = [&] {
@@ -508,7 +507,8 @@ void ncvis_engine::fit(const float *X, size_t N, size_t D, float *Y, bool host) 
     auto total_bytes = [&] {
         return o_ci + cand_bytes() +
                align256(std::max({symmetrize_workspace_bytes((int64_t)N, k), fp.block_bytes(),
-                                  bf16 && !ivf ? bs.bytes : 0}));
+                                  bf16 && !ivf ? bs.bytes : 0,
+                                  init_workspace_bytes((int64_t)N, d)}));
     };
     auto take_less = [&] {
         fp.split = false;
@@ -595,7 +595,7 @@ void ncvis_engine::fit(const float *X, size_t N, size_t D, float *Y, bool host) 
     nv.next("ncvis.init");
     const float init_alpha = (float)(1. / k);
     run_init_embedding((int64_t)N, d, row_ptr, cols, (uint64_t)p.random_seed, p.n_init_epochs,
-                       init_alpha, dY, base + o_init, s, o.init_sequential_stats != 0);
+                       init_alpha, dY, base + o_sym, s, o.init_sequential_stats != 0);
     NCVIS_CUDA(cudaEventRecord(ev.ev[6], s));
     nv.next("ncvis.optimize");
 
@@ -751,7 +751,6 @@ void ncvis_engine::fit_batched(const float *dX, size_t D, const int64_t *offsets
     const size_t o_cols = L.take(sizeof(int32_t) * 2 * nk);
     const size_t o_vals = L.take(sizeof(float) * 2 * nk);
     const size_t o_src = L.take(sizeof(int32_t) * 2 * nk);
-    const size_t o_init = L.take(init_batched_workspace_bytes(total, h_ti[B], (int)B, d));
     const size_t o_off = L.take(sizeof(int64_t) * (B + 1));
     const size_t o_tq = L.take(sizeof(int64_t) * (B + 1));
     const size_t o_ti = L.take(sizeof(int64_t) * (B + 1));
@@ -770,7 +769,7 @@ void ncvis_engine::fit_batched(const float *dX, size_t D, const int64_t *offsets
     const size_t o_Xcp = fold ? L.take(sizeof(__nv_bfloat16) * total_pad * tp.ldb) : 0;
     const size_t o_sqp = bf16 ? L.take(sizeof(float) * total_pad) : 0;
     // The work list, the candidates and the symmetrization's workspace, which
-    // the FP32 search's part rows share, as in fit().
+    // the FP32 search's part rows and the initial embedding share, as in fit().
     const size_t o_pad = L.total;
     auto pad_bytes = [&] { return bf16 || split ? align256(sizeof(int64_t) * (B + 1)) : 0; };
     auto wb_bytes = [&] { return bf16 || split ? align256(sizeof(int64_t) * (tw.ctas + 1)) : 0; };
@@ -785,7 +784,8 @@ void ncvis_engine::fit_batched(const float *dX, size_t D, const int64_t *offsets
         const size_t rows =
             split ? sizeof(__half) * (sp.fold ? 3 : 2) * (size_t)total_pad * sp.ldb : 0;
         return o_pad + pad_bytes() + wb_bytes() + wi_bytes() + cand_bytes() +
-               align256(std::max(symmetrize_workspace_bytes(total, k), rows));
+               align256(std::max({symmetrize_workspace_bytes(total, k), rows,
+                                  init_batched_workspace_bytes(total, h_ti[B], (int)B, d)}));
     };
     if (split && o.arena_limit && total_bytes() > o.arena_limit) split = false;
     char *base = nullptr;
@@ -931,7 +931,7 @@ void ncvis_engine::fit_batched(const float *dX, size_t D, const int64_t *offsets
     nv.next("ncvis.batched.init");
     const float init_alpha = (float)(1. / k);
     run_init_embedding_batched(total, d, d_off, d_ti, (int)B, h_ti[B], d_seed, row_ptr, cols,
-                               p.n_init_epochs, init_alpha, dY, base + o_init, s);
+                               p.n_init_epochs, init_alpha, dY, base + o_sym, s);
     NCVIS_CUDA(cudaEventRecord(ev.ev[6], s));
     nv.next("ncvis.batched.optimize");
 
