@@ -15,6 +15,7 @@
 // An epoch is three launches: the sums and the mean, the deviation, and the
 // standardisation; a statistic is finished by the last block of its launch.
 #include <algorithm>
+#include <type_traits>
 
 #include "common.cuh"
 #include "rng.cuh"
@@ -113,15 +114,22 @@ __device__ __forceinline__ BlockRows block_rows(const RowBlocks &w) {
     return r;
 }
 
+// The sums that finish_stat finds not finite stay as they are.
+struct KeepSum {};
+
 // stat[c] of one problem from its blocks' FP64 sums, by the last of them to
 // arrive: kMean the sum / n, else sqrt(sum / n), in FP32 as the reference does.
 // Every block leaves its sums in part; the last one adds them up in the order of
 // the blocks, so the result does not depend on who is last.  sum: in thread
-// c < d the block's sum of dimension c.
-template <bool kMean>
+// c < d the block's sum of dimension c.  again(c), unless it is KeepSum: the
+// thread's share of dimension c's sum over all of the problem's rows in FP64, which
+// the last block takes where the sum is not finite: sums held as two FP32 numbers
+// (Sum2) turn into NaN once a term or a partial sum is infinite, and an infinite sum
+// of squares has to stay one (an infinite mean and NaN both leave nothing but NaN).
+template <bool kMean, class Again>
 __device__ __forceinline__ void finish_stat(int d, double sum, double *__restrict__ part,
                                             int *__restrict__ done, const BlockRows &b,
-                                            float *__restrict__ stat) {
+                                            float *__restrict__ stat, Again again) {
     __shared__ double red[kThreads / 32];
     __shared__ bool last;
     if (threadIdx.x < d) {
@@ -134,10 +142,8 @@ __device__ __forceinline__ void finish_stat(int d, double sum, double *__restric
     if (!last) return;
     __threadfence();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int c = 0; c < d; ++c) {
-        double s = 0.0;
-        for (int64_t t = threadIdx.x; t < b.blocks; t += kThreads)
-            s += __ldcg(part + (b.first + t) * d + c);
+    // Thread 0 gets the block's sum.
+    auto over_block = [&](double s) {
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
         if (lane == 0) red[warp] = s;
@@ -145,6 +151,18 @@ __device__ __forceinline__ void finish_stat(int d, double sum, double *__restric
         if (threadIdx.x == 0) {
             s = 0.0;
             for (int w = 0; w < kThreads / 32; ++w) s += red[w];
+        }
+        return s;
+    };
+    for (int c = 0; c < d; ++c) {
+        double s = 0.0;
+        for (int64_t t = threadIdx.x; t < b.blocks; t += kThreads)
+            s += __ldcg(part + (b.first + t) * d + c);
+        s = over_block(s);
+        if constexpr (!std::is_same_v<Again, KeepSum>) {
+            if (__syncthreads_or(threadIdx.x == 0 && !isfinite(s))) s = over_block(again(c));
+        }
+        if (threadIdx.x == 0) {
             const float v = __fdiv_rn((float)s, (float)b.n);
             stat[b.problem * d + c] = kMean ? v : sqrtf(v);
         }
@@ -170,15 +188,10 @@ struct Sum2 {
 };
 
 // Thread c < D gets the block's sum of sum[c]: over the warps' lanes, then over
-// the warps in FP64.  Where a value or a sum left FP32's range (which turns the two
-// numbers into NaN), the block sums its values, value(i) for rows i of [begin, end),
-// in FP64 instead: an infinite sum stays one.
-template <int D, class Value>
-__device__ __forceinline__ double block_sum(Sum2 (&sum)[D], int64_t begin, int64_t end,
-                                            Value value) {
+// the warps in FP64.
+template <int D>
+__device__ __forceinline__ double block_sum(Sum2 (&sum)[D]) {
     __shared__ double red[D][kThreads / 32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    bool out_of_range = false;
 #pragma unroll
     for (int c = 0; c < D; ++c) {
 #pragma unroll
@@ -187,39 +200,14 @@ __device__ __forceinline__ double block_sum(Sum2 (&sum)[D], int64_t begin, int64
             const float l = __shfl_xor_sync(0xffffffffu, sum[c].lo, o);
             sum[c].add(h, l);
         }
-        out_of_range |= !isfinite(sum[c].hi);
-        if (lane == 0) red[c][warp] = (double)sum[c].hi + (double)sum[c].lo;
+        if ((threadIdx.x & 31) == 0)
+            red[c][threadIdx.x >> 5] = (double)sum[c].hi + (double)sum[c].lo;
     }
-    if (__syncthreads_or(out_of_range)) {
-        double exact[D];
-#pragma unroll
-        for (int c = 0; c < D; ++c) exact[c] = 0.0;
-        for (int64_t i = begin + threadIdx.x; i < end; i += kThreads) {
-            const RowVec<D> v = value(i);
-#pragma unroll
-            for (int c = 0; c < D; ++c) exact[c] += (double)v.v[c];
-        }
-#pragma unroll
-        for (int c = 0; c < D; ++c) {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) exact[c] += __shfl_xor_sync(0xffffffffu, exact[c], o);
-            if (lane == 0) red[c][warp] = exact[c];
-        }
-        __syncthreads();
-    }
+    __syncthreads();
     double s = 0.0;
     if (threadIdx.x < D)
         for (int w = 0; w < kThreads / 32; ++w) s += red[threadIdx.x][w];
     return s;
-}
-
-// Row i as this block wrote it (not through the read-only path).
-template <int D>
-__device__ __forceinline__ RowVec<D> written_row(const float *Y, int64_t i) {
-    RowVec<D> r;
-#pragma unroll
-    for (int c = 0; c < D; ++c) r.v[c] = __ldcg(Y + i * kPitch<D> + c);
-    return r;
 }
 
 // One init epoch's neighbour sums for d <= 4 and their means, one thread per row:
@@ -269,9 +257,7 @@ __global__ void __launch_bounds__(kThreads) spmm_mean(
 #pragma unroll
         for (int c = 0; c < D; ++c) sum[c].hi = acc.v[c];
     }
-    const double s = block_sum<D>(sum, b.row, b.end,
-                                  [&](int64_t r) { return written_row<D>(Ynew, r); });
-    finish_stat<true>(D, s, part, done, b, mean);
+    finish_stat<true>(D, block_sum<D>(sum), part, done, b, mean, KeepSum());
 }
 
 // The same for few rows, where the longest row is what an epoch waits for: a row's
@@ -410,9 +396,7 @@ __global__ void __launch_bounds__(kThreads) spmm_mean_share(
         const RowVec<D> acc = long_row_sum<D>(lp, (int)(row_ptr[li + 1] - lp), cols, alpha, Yold);
         if (lane == 0) finish(li, acc);
     }
-    const double s = block_sum<D>(sum, b.row, b.end,
-                                  [&](int64_t r) { return written_row<D>(Ynew, r); });
-    finish_stat<true>(D, s, part, done, b, mean);
+    finish_stat<true>(D, block_sum<D>(sum), part, done, b, mean, KeepSum());
 }
 
 // sigma from the rows and their mean: (y - mean)^2 rounded to FP32 as the
@@ -429,21 +413,28 @@ __global__ void __launch_bounds__(kThreads) centred_sigma(RowBlocks blocks,
     float m[D];
 #pragma unroll
     for (int c = 0; c < D; ++c) m[c] = mean[b.problem * D + c];
-    auto term = [&](int64_t i) {
-        RowVec<D> t = load_row<D>(Y, i);
+    for (int64_t i = b.row + threadIdx.x; i < b.end; i += kThreads) {
+        const RowVec<D> y = load_row<D>(Y, i);
 #pragma unroll
         for (int c = 0; c < D; ++c) {
-            const float dev = __fsub_rn(t.v[c], m[c]);
-            t.v[c] = __fmul_rn(dev, dev);
+            const float dev = __fsub_rn(y.v[c], m[c]);
+            sum[c].add(__fmul_rn(dev, dev), 0.f);
         }
-        return t;
-    };
-    for (int64_t i = b.row + threadIdx.x; i < b.end; i += kThreads) {
-        const RowVec<D> t = term(i);
-#pragma unroll
-        for (int c = 0; c < D; ++c) sum[c].add(t.v[c], 0.f);
     }
-    finish_stat<false>(D, block_sum<D>(sum, b.row, b.end, term), part, done, b, sigma);
+    auto again = [&](int c) {
+        const float centre = mean[b.problem * D + c];
+        const int64_t row0 = blocks.off ? blocks.off[b.problem] : 0;
+        double s = 0.0;
+        if (isfinite(centre))
+            for (int64_t i = threadIdx.x; i < b.n; i += kThreads) {
+                const float dev = __fsub_rn(__ldg(Y + (row0 + i) * kPitch<D> + c), centre);
+                s += (double)__fmul_rn(dev, dev);
+            }
+        else
+            s = (double)centre * (double)centre;
+        return s;
+    };
+    finish_stat<false>(D, block_sum<D>(sum), part, done, b, sigma, again);
 }
 
 // The two for any d, one thread per row and dimension: neighbouring threads read
@@ -478,7 +469,7 @@ __global__ void __launch_bounds__(kThreads) spmm_mean_any(
             sum += (double)acc;
         }
     }
-    finish_stat<true>(d, block_sum_any(d, sum), part, done, b, mean);
+    finish_stat<true>(d, block_sum_any(d, sum), part, done, b, mean, KeepSum());
 }
 
 __global__ void __launch_bounds__(kThreads) centred_sigma_any(RowBlocks blocks, int d,
@@ -497,7 +488,7 @@ __global__ void __launch_bounds__(kThreads) centred_sigma_any(RowBlocks blocks, 
             sum += (double)__fmul_rn(dev, dev);
         }
     }
-    finish_stat<false>(d, block_sum_any(d, sum), part, done, b, sigma);
+    finish_stat<false>(d, block_sum_any(d, sum), part, done, b, sigma, KeepSum());
 }
 
 // The reference's one-thread statistics (src/ncvis.cpp:226-254 on one
