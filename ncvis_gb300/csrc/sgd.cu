@@ -1062,7 +1062,7 @@ void run_sgd_hogwild(const SgdArgs &g, int epoch_begin, int epoch_end, const siz
                      int chains, void *workspace, cudaStream_t s) {
     require(g.N >= 2 && g.N < (int64_t(1) << 31), "optimize: N must be in [2, 2^31)");
     if (chains <= 0) chains = sgd_default_chains(g.E, g.N, g.d);
-    const int threads = chain_block_threads(chains, num_sms(), kThreads);
+    const int threads = chain_block_threads(chains, g.d, num_sms(), kThreads);
     const int blocks = (int)ceil_div(chains, threads);
     const int64_t total_chains = chains;
     const int64_t chunk = ((g.E + total_chains - 1) / total_chains + 3) & ~(int64_t)3;

@@ -1,4 +1,4 @@
-"""The unstaged optimizer's block sizes leave no SM with more chains than full blocks
+"""The unstaged optimizer's block sizes leave no SM with far more chains than full blocks
 do (tests/harness/chain_blocks_check.cpp); the loop is src/ncvis.cpp:275-352."""
 import os
 import subprocess
@@ -6,7 +6,7 @@ import subprocess
 from conftest import ROOT
 
 
-def test_no_sm_has_more_chains_than_full_blocks_give_it(tmp_path):
+def test_no_sm_has_far_more_chains_than_full_blocks_give_it(tmp_path):
     exe = str(tmp_path / "chain_blocks_check")
     r = subprocess.run(["g++", "-std=c++17", "-O2", "-I", os.path.join(ROOT, "ncvis_gb300", "csrc"),
                         os.path.join(ROOT, "tests", "harness", "chain_blocks_check.cpp"), "-o", exe],
