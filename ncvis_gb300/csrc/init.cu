@@ -15,7 +15,7 @@
 // An epoch is three launches: the sums and the mean, the deviation, and the
 // standardisation; a statistic is finished by the last block of its launch.
 #include <algorithm>
-#include <type_traits>
+#include <cfloat>
 
 #include "common.cuh"
 #include "rng.cuh"
@@ -114,22 +114,15 @@ __device__ __forceinline__ BlockRows block_rows(const RowBlocks &w) {
     return r;
 }
 
-// The sums that finish_stat finds not finite stay as they are.
-struct KeepSum {};
-
 // stat[c] of one problem from its blocks' FP64 sums, by the last of them to
 // arrive: kMean the sum / n, else sqrt(sum / n), in FP32 as the reference does.
 // Every block leaves its sums in part; the last one adds them up in the order of
 // the blocks, so the result does not depend on who is last.  sum: in thread
-// c < d the block's sum of dimension c.  again(c), unless it is KeepSum: the
-// thread's share of dimension c's sum over all of the problem's rows in FP64, which
-// the last block takes where the sum is not finite: sums held as two FP32 numbers
-// (Sum2) turn into NaN once a term or a partial sum is infinite, and an infinite sum
-// of squares has to stay one (an infinite mean and NaN both leave nothing but NaN).
-template <bool kMean, class Again>
+// c < d the block's sum of dimension c.
+template <bool kMean>
 __device__ __forceinline__ void finish_stat(int d, double sum, double *__restrict__ part,
                                             int *__restrict__ done, const BlockRows &b,
-                                            float *__restrict__ stat, Again again) {
+                                            float *__restrict__ stat) {
     __shared__ double red[kThreads / 32];
     __shared__ bool last;
     if (threadIdx.x < d) {
@@ -142,8 +135,10 @@ __device__ __forceinline__ void finish_stat(int d, double sum, double *__restric
     if (!last) return;
     __threadfence();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    // Thread 0 gets the block's sum.
-    auto over_block = [&](double s) {
+    for (int c = 0; c < d; ++c) {
+        double s = 0.0;
+        for (int64_t t = threadIdx.x; t < b.blocks; t += kThreads)
+            s += __ldcg(part + (b.first + t) * d + c);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
         if (lane == 0) red[warp] = s;
@@ -151,18 +146,6 @@ __device__ __forceinline__ void finish_stat(int d, double sum, double *__restric
         if (threadIdx.x == 0) {
             s = 0.0;
             for (int w = 0; w < kThreads / 32; ++w) s += red[w];
-        }
-        return s;
-    };
-    for (int c = 0; c < d; ++c) {
-        double s = 0.0;
-        for (int64_t t = threadIdx.x; t < b.blocks; t += kThreads)
-            s += __ldcg(part + (b.first + t) * d + c);
-        s = over_block(s);
-        if constexpr (!std::is_same_v<Again, KeepSum>) {
-            if (__syncthreads_or(threadIdx.x == 0 && !isfinite(s))) s = over_block(again(c));
-        }
-        if (threadIdx.x == 0) {
             const float v = __fdiv_rn((float)s, (float)b.n);
             stat[b.problem * d + c] = kMean ? v : sqrtf(v);
         }
@@ -175,6 +158,10 @@ __device__ __forceinline__ void finish_stat(int d, double sum, double *__restric
 // statistics' FP64 sums up to a warp's are formed in it, because an FP64 add of a
 // warp takes 16 cycles of an SM here, which with the conversions was 13 of the
 // deviation pass's 20 us at 500,001 x 3.
+// kSquares: where the sum leaves FP32's range it is infinite, as an FP64 one is by the
+// time it is rounded, not the NaN that the parts' differences make (a sum of values
+// that leaves it makes the mean infinite or NaN, and either every row NaN).
+template <bool kSquares>
 struct Sum2 {
     float hi = 0.f, lo = 0.f;
     __device__ __forceinline__ void add(float h, float l) {
@@ -182,15 +169,16 @@ struct Sum2 {
         const float t = __fsub_rn(s, hi);
         const float e = __fadd_rn(__fsub_rn(hi, __fsub_rn(s, t)), __fsub_rn(h, t));
         const float r = __fadd_rn(e, __fadd_rn(lo, l));
-        hi = __fadd_rn(s, r);
-        lo = __fsub_rn(r, __fsub_rn(hi, s));
+        const bool keep = kSquares && !(s <= FLT_MAX);
+        hi = keep ? s : __fadd_rn(s, r);
+        lo = keep ? 0.f : __fsub_rn(r, __fsub_rn(hi, s));
     }
 };
 
 // Thread c < D gets the block's sum of sum[c]: over the warps' lanes, then over
 // the warps in FP64.
-template <int D>
-__device__ __forceinline__ double block_sum(Sum2 (&sum)[D]) {
+template <int D, bool kSquares>
+__device__ __forceinline__ double block_sum(Sum2<kSquares> (&sum)[D]) {
     __shared__ double red[D][kThreads / 32];
 #pragma unroll
     for (int c = 0; c < D; ++c) {
@@ -250,14 +238,14 @@ __global__ void __launch_bounds__(kThreads) spmm_mean(
     double *__restrict__ part, int *__restrict__ done, float *__restrict__ mean) {
     const BlockRows b = block_rows(blocks);
     const int64_t i = b.row + threadIdx.x;
-    Sum2 sum[D];
+    Sum2<false> sum[D];
     if (i < b.end) {
         const RowVec<D> acc = row_sum<D>(row_ptr[i], row_ptr[i + 1], cols, alpha, Yold);
         store_row<D>(Ynew, i, acc);
 #pragma unroll
         for (int c = 0; c < D; ++c) sum[c].hi = acc.v[c];
     }
-    finish_stat<true>(D, block_sum<D>(sum), part, done, b, mean, KeepSum());
+    finish_stat<true>(D, block_sum(sum), part, done, b, mean);
 }
 
 // The same for few rows, where the longest row is what an epoch waits for: a row's
@@ -345,7 +333,7 @@ __global__ void __launch_bounds__(kThreads) spmm_mean_share(
     __shared__ int n_long[kWarps];
     const BlockRows b = block_rows(blocks);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    Sum2 sum[D];
+    Sum2<false> sum[D];
     auto finish = [&](int64_t i, const RowVec<D> &acc) {
         store_row<D>(Ynew, i, acc);
 #pragma unroll
@@ -396,7 +384,7 @@ __global__ void __launch_bounds__(kThreads) spmm_mean_share(
         const RowVec<D> acc = long_row_sum<D>(lp, (int)(row_ptr[li + 1] - lp), cols, alpha, Yold);
         if (lane == 0) finish(li, acc);
     }
-    finish_stat<true>(D, block_sum<D>(sum), part, done, b, mean, KeepSum());
+    finish_stat<true>(D, block_sum(sum), part, done, b, mean);
 }
 
 // sigma from the rows and their mean: (y - mean)^2 rounded to FP32 as the
@@ -409,7 +397,7 @@ __global__ void __launch_bounds__(kThreads) centred_sigma(RowBlocks blocks,
                                                           int *__restrict__ done,
                                                           float *__restrict__ sigma) {
     const BlockRows b = block_rows(blocks);
-    Sum2 sum[D];
+    Sum2<true> sum[D];
     float m[D];
 #pragma unroll
     for (int c = 0; c < D; ++c) m[c] = mean[b.problem * D + c];
@@ -421,20 +409,7 @@ __global__ void __launch_bounds__(kThreads) centred_sigma(RowBlocks blocks,
             sum[c].add(__fmul_rn(dev, dev), 0.f);
         }
     }
-    auto again = [&](int c) {
-        const float centre = mean[b.problem * D + c];
-        const int64_t row0 = blocks.off ? blocks.off[b.problem] : 0;
-        double s = 0.0;
-        if (isfinite(centre))
-            for (int64_t i = threadIdx.x; i < b.n; i += kThreads) {
-                const float dev = __fsub_rn(__ldg(Y + (row0 + i) * kPitch<D> + c), centre);
-                s += (double)__fmul_rn(dev, dev);
-            }
-        else
-            s = (double)centre * (double)centre;
-        return s;
-    };
-    finish_stat<false>(D, block_sum<D>(sum), part, done, b, sigma, again);
+    finish_stat<false>(D, block_sum(sum), part, done, b, sigma);
 }
 
 // The two for any d, one thread per row and dimension: neighbouring threads read
@@ -469,7 +444,7 @@ __global__ void __launch_bounds__(kThreads) spmm_mean_any(
             sum += (double)acc;
         }
     }
-    finish_stat<true>(d, block_sum_any(d, sum), part, done, b, mean, KeepSum());
+    finish_stat<true>(d, block_sum_any(d, sum), part, done, b, mean);
 }
 
 __global__ void __launch_bounds__(kThreads) centred_sigma_any(RowBlocks blocks, int d,
@@ -488,7 +463,7 @@ __global__ void __launch_bounds__(kThreads) centred_sigma_any(RowBlocks blocks, 
             sum += (double)__fmul_rn(dev, dev);
         }
     }
-    finish_stat<false>(d, block_sum_any(d, sum), part, done, b, sigma, KeepSum());
+    finish_stat<false>(d, block_sum_any(d, sum), part, done, b, sigma);
 }
 
 // The reference's one-thread statistics (src/ncvis.cpp:226-254 on one
