@@ -28,8 +28,10 @@ Fn driver_entry(const char *name) {
 
 std::mutex g_mu;
 // By device and context id; ids are not used again, so the entry of a context that
-// was destroyed, whose pool went with it, is never met.
-std::map<std::pair<int, unsigned long long>, cudaMemPool_t> g_pools;
+// was destroyed, whose pool went with it, is never met.  Never destroyed: an engine
+// may outlive the library's static objects.
+using Pools = std::map<std::pair<int, unsigned long long>, cudaMemPool_t>;
+Pools &g_pools = *new Pools;
 
 }  // namespace
 
