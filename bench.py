@@ -37,9 +37,9 @@ sys.path.insert(0, ROOT)
 N_FULL, D_FULL, K_NN, D_EMB, EPOCHS, INIT_EPOCHS = 1_024_000, 100, 15, 2, 50, 20
 ONE_THREAD_N = 32_768  # points of the one-thread CPU figure
 RECALL_QUERIES = 10_000  # recall@15 sample against FP64 exact search
-# DRAM bytes (read + write) of one full-size BF16 kNN-selection launch, from a
-# one-pass ncu capture (dram__bytes_read.sum + dram__bytes_write.sum).
-KNN_TRAFFIC_BYTES = 250.94e9
+# DRAM bytes (read + write) of one full-size BF16 kNN-selection launch: a constant, from a
+# one-pass ncu capture of this kernel (dram__bytes_read.sum + dram__bytes_write.sum).
+KNN_TRAFFIC_BYTES = 139.34e9
 
 
 def parse():
@@ -505,7 +505,7 @@ def run_ours(args):
     roof.update({"kernel": "knn candidate selection (knn_select_tc)", "achieved": achieved,
                  "peak": peak, "frac": achieved / peak,
                  "traffic": KNN_TRAFFIC_BYTES if (n == N_FULL and args.knn == "bf16") else None,
-                 "traffic_unit": "DRAM bytes per launch (ncu)",
+                 "traffic_unit": "DRAM bytes per launch (from an ncu capture, not of this run)",
                  "kernel_ms": sweep_ms, "cell_ordering_ms": order_ms,
                  "frac_of_knn_stage": flops / (knn_ms / 1000.0) / 1e12 / peak,
                  "algorithmic": f"2*N^2*D = {flops:.3e} FLOP per launch (D=100 unpadded)"})

@@ -112,7 +112,8 @@ typedef struct ncvis_options {
     size_t arena_limit;     /* largest device arena (the fit's device buffers) the engine may
                                hold, in bytes (0: no limit); a fit that needs more fails as an
                                allocation failure (NCVIS_CUDA_ERROR) */
-    int init_sequential_stats; /* init_embedding's mean and std: 0 from FP64 partial sums;
+    int init_sequential_stats; /* init_embedding's mean and std: 0 from FP64 partial sums
+                               (up to a warp's in two FP32 numbers, about 48 bits);
                                nonzero as the reference's one thread sums them (see
                                ncvis_init_embedding_device) */
     int knn_order_cells;    /* k-means cells that order the rows before the exact BF16 search
