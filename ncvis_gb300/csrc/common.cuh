@@ -48,8 +48,8 @@ unsigned long long current_context_id();
 // 0.44 ms a call (1,000 x 32 neighbours, 800,000 x 15 symmetrization).  This one
 // keeps at most kPoolKeeps bytes between calls; they go back when an engine that has
 // fitted on the device is destroyed, when an allocation finds no room and on request
-// (ncvis_release_workspace).  CUDA orders
-// reuse between streams and threads; each context has a pool of its own.
+// (ncvis_release_workspace).  CUDA orders reuse between streams and threads; each
+// context has a pool of its own.
 constexpr size_t kPoolKeeps = size_t(1) << 30;
 cudaMemPool_t workspace_pool();
 // Gives back what the pool of device `dev` keeps unused.
